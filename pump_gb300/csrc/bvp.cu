@@ -7,8 +7,10 @@
 // hoisted value is computed by exactly the same operations the expression
 // performs, so every rounding is unchanged and only repeated work is
 // removed.  The finite-difference bisection (2pBVP.cu:71-95) is replicated
-// step for step.  Cost evaluation is binary64-bound (the expression promotes
-// through pow(double)), so these kernels are limited by the FP64 pipe.
+// step for step (bisect.cuh).  The expression is binary64 (it promotes
+// through pow(double)); almost every value it gives is certified from
+// binary32 arithmetic instead (ffcost.cuh), so the kernels are bound by
+// instruction issue.
 //
 // The precision-mode minimiser (closed form, binary64 refinement) is in
 // bvp_precise.cu, compiled with multiply-add contraction.
@@ -17,8 +19,9 @@
 #include <type_traits>
 
 #include "common.cuh"
-#include "ffcost.cuh"
 #include "ctx.h"
+#include "bisect.cuh"
+#include "ffcost.cuh"
 #include "pathpoint.cuh"
 #include "tune.h"
 
@@ -41,12 +44,6 @@ __device__ __forceinline__ double f2d(float f) {
   return __longlong_as_double((long long)(sign | ((unsigned long long)(e + (1023u - 127u)) << 52) |
                                           ((unsigned long long)(u & 0x7FFFFFu) << 29)));
 }
-
-// The bisection's stopping test compares a binary32 |dcval| with the
-// binary64 constant 0.0001 (2pBVP.cu:86).  binary32 0.0001f is below 0.0001
-// and the next binary32 above it, so (double)x > 0.0001 exactly when
-// x > 0.0001f (NaN false either way): the test runs in binary32.
-constexpr float kDcvalTol = 0.0001f;
 
 struct PairCoef {
   double s7;                                     // first seven (tau-free) terms
@@ -128,176 +125,53 @@ __device__ __forceinline__ float cost_eval(const PairCoef &c, float tau) {
   return (float)((1.0 / t3) * s);
 }
 
-// ------------------------------------------- the cost off the binary64 pipe
-// (ffcost.cuh: cost_ff, PairFF)
-__device__ __forceinline__ float cost_fast(const PairCoef &c, const PairFF &f, float tau) {
-  bool ok;
-  const float v = cost_ff(f, tau, &ok);
-  return ok ? v : cost_eval(c, tau);
-}
-
-// dcost, 2pBVP.cu:109-115
-__device__ __forceinline__ float dcost_eval(const PairCoef &c, const PairFF &f, float tau) {
-  const float dtau = (float)0.000001;
-  return (cost_fast(c, f, tau + dtau / 2) - cost_fast(c, f, tau - dtau / 2)) / dtau;
-}
-
-// toptBisection, 2pBVP.cu:71-95.  The reference's halving loop (:78-80) is
-// unbounded; here it stops after 160 halvings (tl < 1e-50 has underflowed to
-// zero long before), exactly as the oracle does.
-__device__ float topt_bisection(const PairCoef &c, const PairFF &f, float tmax) {
-  float tu = tmax;
-  if (dcost_eval(c, f, tmax) < 0) return tmax;
-  float tl = (float)0.01;
-  int halvings = 0;
-  while (dcost_eval(c, f, tl) > 0 && halvings < 160) {
-    tl = tl / 2;
-    ++halvings;
+// The reference's cost of the pair (x0, x1) at tau, every operation in its
+// own type: what the certified evaluations fall back to.  Out of line, so that
+// its registers do not count against the pair kernel's occupancy.
+struct ParityCost {
+  struct States {
+    float x0[kDim], x1[kDim];
+  };
+  static __device__ __noinline__ float eval(const States s, float tau) {
+    return cost_eval(make_coef(s.x0, s.x1), tau);
   }
-  float topt = 0;
-  float dcval = 1;
-  int itr = 0;
-  while (fabsf(dcval) > kDcvalTol && itr < 50) {
-    ++itr;
-    topt = (tu + tl) / 2;
-    dcval = dcost_eval(c, f, topt);
-    if (dcval > 0)
-      tu = topt;
-    else
-      tl = topt;
+  static __device__ __forceinline__ float cost(const float *x0, const float *x1, float tau) {
+    States s;
+#pragma unroll
+    for (int d = 0; d < kDim; ++d) {
+      s.x0[d] = x0[d];
+      s.x1[d] = x1[d];
+    }
+    return eval(s, tau);
   }
-  return topt;
-}
+};
 
 // --------------------------------------------------------------- kernels
-// Persistent parity kernel.  The reference's bisection runs a different
-// number of steps per pair (tmax test, halving loop, up to 50 bisection
-// steps, then the final cost), so one thread per pair leaves most lanes of a
-// warp idle while the slowest pair finishes.  Here every lane runs a small
-// state machine over the same sequence of evaluations toptBisection performs
-// for its pair, and each warp iteration evaluates exactly two costs in every
-// lane (the two sides of dcost, or the final cost and a spare).  A lane whose
-// pair is done stores it and takes the next pair of the warp's chunk of
-// kParityChunk consecutive pairs (16 per lane on average, so lanes idle only
-// while a chunk's last pairs finish).  Per pair, the evaluated expressions and
-// their order are unchanged.
-//
-// A lane whose evaluation the float-float bound does not certify waits
-// (keeping its state and the certified side of the pair) until
-// kFallbackLanes lanes of its warp wait, or until no lane of the warp can
-// go on: then the waiting lanes run the binary64 evaluation together.  The
-// binary64 instructions cost a warp the same for one lane as for 32, so this
-// spends them on several lanes at once.
-// Launch bounds (128, 6): 80 registers, 6 blocks per SM (9.9 ms at N = 4000,
-// 10.1 with 96 registers and 5 blocks).
-constexpr int kParityChunk = 512;
-constexpr int kFallbackLanes = 8;
-constexpr int kRefillLanes = 8;
-
-__global__ void __launch_bounds__(128, 6) bvp_pairs_parity_persistent(
-    const float *__restrict__ samples, int N, float tmax, float *__restrict__ copts,
-    float *__restrict__ topts) {
-  const long long npairs = (long long)N * (N - 1);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  const float h = (float)0.000001 / 2;  // dtau / 2 of dcost
-  const float dtau = (float)0.000001;
-  const long long warp_id = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  long long chunk_next = warp_id * kParityChunk;
-  const long long chunk_end = chunk_next + kParityChunk < npairs ? chunk_next + kParityChunk : npairs;
-  // lane state
-  long long idx = -1;
-  int phase = 0, halvings = 0, itr = 0;
-  float tu = 0, tl = 0, topt = 0, dcval = 0;
-  float x0[kDim], x1[kDim];
-  PairFF pf{};
-  // the step's evaluation points and values; pending: a value waits for the
-  // binary64 evaluation (ok_a / ok_b: that side is certified already)
-  float ta = 0, tb = 0, ca = 0, cb = 0;
-  bool pending = false, ok_a = true, ok_b = true;
-  while (true) {
-    // lanes without a pair take the next pairs of the warp's chunk, once
-    // kRefillLanes of them wait (or no lane has a pair): the pair set-up
-    // then runs for several lanes at once (N = 4000: 7.38 ms refilling each
-    // lane at once, 6.40 ms with 4 lanes, 6.10 ms with 8, 6.59 ms with 16)
-    const unsigned need = __ballot_sync(0xffffffffu, idx < 0);
-    if (need && chunk_next < chunk_end && (__popc(need) >= kRefillLanes || need == 0xffffffffu)) {
-      const int avail = (int)(chunk_end - chunk_next);
-      const int rank = __popc(need & lt);
-      const bool mine = (need >> lane) & 1u;
-      if (mine && rank < avail) {
-        idx = chunk_next + rank;
-        const int i = (int)(idx / (N - 1));
-        const int r = (int)(idx - (long long)i * (N - 1));
-        const int j = r + (r >= i);
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) {
-          x0[d] = __ldg(&samples[i * kDim + d]);
-          x1[d] = __ldg(&samples[j * kDim + d]);
-        }
-        pf = make_pair_ff(x0, x1);
-        phase = 0;
-        tu = tmax;
-      }
-      chunk_next += __popc(need) < avail ? __popc(need) : avail;
-    }
-    const unsigned active = __ballot_sync(0xffffffffu, idx >= 0);
-    if (active == 0u) break;  // nothing left
-    if (idx >= 0 && !pending) {
-      // the two evaluation points of this step
-      if (phase == 0) { ta = tmax + h; tb = tmax - h; }
-      else if (phase == 1) { ta = tl + h; tb = tl - h; }
-      else if (phase == 2) { ++itr; topt = (tu + tl) / 2; ta = topt + h; tb = topt - h; }
-      else { ta = topt; tb = topt; }
-      ca = cost_ff(pf, ta, &ok_a);
-      cb = cost_ff(pf, tb, &ok_b);
-      pending = !(ok_a && ok_b);
-    }
-    const unsigned waiting = __ballot_sync(0xffffffffu, pending);
-    if (waiting && (__popc(waiting) >= kFallbackLanes || waiting == active)) {
-      if (pending) {
-        const PairCoef c = make_coef(x0, x1);
-        if (!ok_a) ca = cost_eval(c, ta);
-        if (!ok_b) cb = cost_eval(c, tb);
-        pending = false;
-      }
-    }
-    if (idx < 0 || pending) continue;
-    const float d = (ca - cb) / dtau;
-    if (phase == 0) {
-      if (d < 0) { topt = tmax; phase = 3; }
-      else { tl = (float)0.01; halvings = 0; phase = 1; }
-    } else if (phase == 1) {
-      if (d > 0 && halvings < 160) { tl = tl / 2; ++halvings; }
-      else { topt = 0; dcval = 1; itr = 0; phase = 2; }
-    } else if (phase == 2) {
-      dcval = d;
-      if (dcval > 0) tu = topt; else tl = topt;
-      if (!(fabsf(dcval) > kDcvalTol && itr < 50)) phase = 3;
-    } else {
-      topts[idx] = topt;
-      copts[idx] = ca;
-      idx = -1;
-    }
-  }
+// All pairs: each warp walks `chunk` consecutive pairs (bisect.cuh).  Bound by
+// instruction issue.  N = 4000 (16 M pairs): 6.11 ms with two float-float costs
+// per finite difference, 3.64 ms with the differences' signs from cost_delta
+// where it settles them, 1.93 ms in two stages with their step limits (about
+// 110 warp instructions a pair; 31 KB of queue a block, 80 registers, 6 blocks
+// an SM).
+__global__ void __launch_bounds__(kBisectThreads, 6) bvp_pairs_parity_persistent(AllPairs src,
+                                                                                 int chunk) {
+  __shared__ BisectQueue s_queue[kBisectWarps];
+  const long long left = (long long)src.N * (src.N - 1);
+  const int warp = threadIdx.x >> 5;
+  const long long first = (blockIdx.x * (long long)kBisectWarps + warp) * chunk;
+  if (first >= left) return;
+  bisect_warp<ParityCost, kBisectRefill>(src, s_queue[warp], first,
+                                        left - first < chunk ? (int)(left - first) : chunk);
 }
 
-__global__ void bvp_batch_kernel(const BvpJobs jb) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= jb.n * jb.jobs) return;
-  const int j = k >= jb.n ? 1 : 0;
-  k -= j * jb.n;
-  float x0[kDim], x1[kDim];
-#pragma unroll
-  for (int d = 0; d < kDim; ++d) {
-    x0[d] = jb.x0[k * kDim + d];
-    x1[d] = jb.x1[(jb.x1_same ? 0 : k) * kDim + d];
-  }
-  const PairCoef c = make_coef(x0, x1);
-  const PairFF f = make_pair_ff(x0, x1);
-  const float tp = topt_bisection(c, f, jb.tmax[j]);
-  if (jb.topt[j]) jb.topt[j][k] = tp;
-  if (jb.cost[j]) jb.cost[j][k] = cost_fast(c, f, tp);
+// Explicit pairs, 32 per warp.
+__global__ void __launch_bounds__(128) bvp_batch_kernel(const JobPairs src) {
+  const long long total = (long long)src.jb.n * src.jb.jobs;
+  __shared__ BisectQueue s_queue[kBisectWarps];
+  const int warp = threadIdx.x >> 5;
+  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * 32;
+  if (first >= total) return;
+  bisect_warp<ParityCost, 32>(src, s_queue[warp], first, total - first < 32 ? (int)(total - first) : 32);
 }
 
 // One thread per edge: findDiscretizedPath, 2pBVP.cu:53-69.  The edge's end
@@ -747,34 +621,45 @@ pump_status_t bvp_jobs_launch(const BvpJobs &jb, int mode, cudaStream_t stream) 
   if (mode == PUMP_BVP_PARITY_GPU) return bvp_jobs_refgpu_launch(jb, stream);
   const long long total = (long long)jb.n * jb.jobs;
   const int threads = total < 152LL * 128 ? 32 : 128;
-  bvp_batch_kernel<<<grid_for(total, threads), threads, 0, stream>>>(jb);
+  bvp_batch_kernel<<<grid_for(total, threads), threads, 0, stream>>>(JobPairs{jb});
   return launch_status("bvp_batch");
 }
 
 namespace {
-// Each edge's optimal time in the host arithmetic (tmax 5), one thread per
-// edge (the lane-refill kernel of all pairs took 1.15 ms on the N = 4000
-// query's 799,800 edges, this one about 0.9 ms).
-__global__ void edge_topts_parity_kernel(const float *__restrict__ samples, const int *__restrict__ src,
-                                         const int *__restrict__ dst, long long E,
-                                         float *__restrict__ topt) {
-  const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  float x0[kDim], x1[kDim];
-  const int a = src[e], b = dst[e];
+// Each edge's optimal time in the host arithmetic (tmax 5).
+struct EdgePairs {
+  static constexpr bool kWantCost = false;
+  const float *__restrict__ samples;
+  const int *__restrict__ src, *__restrict__ dst;
+  float *__restrict__ topt;
+  __device__ __forceinline__ void load(long long e, float *x0, float *x1) const {
+    const int a = __ldg(&src[e]), b = __ldg(&dst[e]);
 #pragma unroll
-  for (int d = 0; d < kDim; ++d) {
-    x0[d] = __ldg(&samples[a * kDim + d]);
-    x1[d] = __ldg(&samples[b * kDim + d]);
+    for (int d = 0; d < kDim; ++d) {
+      x0[d] = __ldg(&samples[a * kDim + d]);
+      x1[d] = __ldg(&samples[b * kDim + d]);
+    }
   }
-  topt[e] = topt_bisection(make_coef(x0, x1), make_pair_ff(x0, x1), 5.0f);
+  __device__ __forceinline__ float tmax(long long) const { return 5.0f; }
+  __device__ __forceinline__ void store(long long e, float t, float) const { topt[e] = t; }
+};
+__global__ void __launch_bounds__(kBisectThreads, 6) edge_topts_parity_kernel(EdgePairs src,
+                                                                              long long E, int chunk) {
+  __shared__ BisectQueue s_queue[kBisectWarps];
+  const int warp = threadIdx.x >> 5;
+  const long long first = (blockIdx.x * (long long)kBisectWarps + warp) * chunk;
+  if (first >= E) return;
+  bisect_warp<ParityCost, kBisectRefill>(src, s_queue[warp], first,
+                                         E - first < chunk ? (int)(E - first) : chunk);
 }
 }  // namespace
 
 pump_status_t edge_topts_parity_async(const float *d_samples, const int *d_src, const int *d_dst,
                                       long long E, float *d_topt, cudaStream_t stream) {
   if (E <= 0) return PUMP_OK;
-  edge_topts_parity_kernel<<<grid_for(E, 128), 128, 0, stream>>>(d_samples, d_src, d_dst, E, d_topt);
+  const int chunk = bisect_chunk(E);
+  edge_topts_parity_kernel<<<grid_for(E, kBisectWarps * chunk), kBisectThreads, 0, stream>>>(
+      EdgePairs{d_samples, d_src, d_dst, d_topt}, E, chunk);
   return launch_status("edge_topts_parity");
 }
 
@@ -820,14 +705,12 @@ extern "C" pump_status_t pump_bvp_pairs(const float *d_samples, int N, float tma
   if (N < 2 || !d_samples || !d_copts || !d_topts || !(tmax > 0))
     return set_error(PUMP_ERR_BAD_INPUT, "pump_bvp_pairs: bad arguments (N=%d)", N);
   const long long npairs = (long long)N * (N - 1);
-  const int threads = 128;
-  long long blocks = (npairs + threads - 1) / threads;
-  if (blocks > 2147483647LL) blocks = 2147483647LL;
   if (mode == PUMP_BVP_PARITY) {
-    const long long nblk = (npairs + 4LL * kParityChunk - 1) / (4LL * kParityChunk);  // 4 warps
+    const int chunk = bisect_chunk(npairs);
+    const long long per = (long long)kBisectWarps * chunk, nblk = (npairs + per - 1) / per;
     if (nblk > 2147483647LL) return set_error(PUMP_ERR_CAPACITY, "pump_bvp_pairs: N=%d", N);
-    bvp_pairs_parity_persistent<<<(unsigned)nblk, 128, 0, (cudaStream_t)stream>>>(
-        d_samples, N, tmax, d_copts, d_topts);
+    bvp_pairs_parity_persistent<<<(unsigned)nblk, kBisectThreads, 0, (cudaStream_t)stream>>>(
+        AllPairs{d_samples, N, tmax, d_copts, d_topts}, chunk);
   } else if (mode == PUMP_BVP_PRECISION) {
     PUMP_TRY(bvp_pairs_precision_launch(d_samples, N, tmax, d_copts, d_topts, (cudaStream_t)stream));
   } else if (mode == PUMP_BVP_PARITY_GPU) {

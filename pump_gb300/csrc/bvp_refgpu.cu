@@ -19,15 +19,17 @@
 // A GPU test compares all N(N-1) pairs at N = 1000 and 4000 with the
 // reference's fillCoptsTopts run on the GB300 (SHA-256 of both arrays).
 //
-// The kernel walks the pairs as bvp.cu's parity kernel does (a per-lane
-// state machine over the bisection's evaluations, lanes refilled from the
-// warp's chunk of pairs), which changes the order of work, not any pair's
-// arithmetic.  Cost: 0.59 s for the 16 M pairs of N = 4000 (the reference's
-// kernel 0.62 s); CUDA's pow for tau (three calls per evaluation) dominates.
+// The kernel walks the pairs as the parity kernel does (bisect.cuh), which
+// changes the order of work, not any pair's arithmetic: almost every
+// comparison and cost is certified from binary32 arithmetic (ffcost.cuh).
+// What is left first tries a binary64 evaluation with its own bound, and only
+// then CUDA's pow: one evaluation of the expression with pow takes tens of
+// microseconds, as long as a warp's other work on a chunk of pairs.
 #include <math.h>
 
 #include "common.cuh"
 #include "ctx.h"
+#include "bisect.cuh"
 #include "ffcost.cuh"
 
 namespace pump {
@@ -62,176 +64,76 @@ __device__ __forceinline__ float cost_dev(float tau, const float *a, const float
   return c;
 }
 
-// dcost, 2pBVP.cu:109-115
-__device__ __forceinline__ float dcost_dev(float tau, const float *a, const float *b, const CoordPow &p) {
-  float dtau = 0.000001;
-  float d = (cost_dev(tau + dtau / 2, a, b, p) - cost_dev(tau - dtau / 2, a, b, p)) / dtau;
-  return d;
-}
-
-// toptBisection, 2pBVP.cu:71-95; the halving loop, unbounded in the
-// reference, stops after 160 halvings (as in bvp.cu and the oracle)
-__device__ float topt_dev(const float *a, const float *b, const CoordPow &p, float tmax) {
-  float tu = tmax;
-  if (dcost_dev(tmax, a, b, p) < 0) return tmax;
-  float tl = 0.01;
-  int halvings = 0;
-  while (dcost_dev(tl, a, b, p) > 0 && halvings < 160) {
-    tl = tl / 2;
-    ++halvings;
+// The reference kernel's cost of the pair at tau, out of line (the registers
+// of the binary64 powers do not count against the pair kernel's occupancy).
+//
+// Its binary64 value lies within 2^-46.9 of the terms' magnitudes (over t^3)
+// of the exact sum of its rounded binary32 terms (ffcost.cuh); the same sum
+// with correctly rounded powers, here, within 2^-47 of them.  When every
+// value within 2^-45 of them of the latter converts to the same binary32,
+// that is the result; otherwise the expression is evaluated with pow, as the
+// reference kernel does.
+struct RefGpuCost {
+  struct States {
+    float a[kDim], b[kDim];
+  };
+  static __device__ __noinline__ float eval(const States st, float tau) {
+    const PairFF f = make_pair_ff(st.a, st.b);
+    const float a29 = __fmul_rn(f.a29, f.b29 + f.c29 * tau);
+    const float a30 = __fmul_rn(f.a30, f.b30 + f.c30 * tau);
+    const double t = tau, t2 = t * t, t3 = t2 * t;
+    const float *x = st.a, *y = st.b;
+    const double s7 = 12 * (p2f(x[0]) + p2f(x[2]) + p2f(x[1]) + p2f(y[0]) + p2f(y[2]) + p2f(y[1])) -
+                      (double)(__fmul_rn(24 * x[1], y[1]));
+    const double d2 = 4 * (p2f(x[4]) + p2f(x[3]) + p2f(x[5]) + p2f(y[4]) + p2f(y[3]) + p2f(y[5])) +
+                      ((double)__fmul_rn(4 * x[4], y[4]) + (double)__fmul_rn(4 * x[3], y[3]) +
+                       (double)__fmul_rn(4 * x[5], y[5]));
+    const double d3 = (double)f.d3.hi + (double)f.d3.lo;
+    const double d4 = 1.0 + (double)kGRef * (double)kGRef;
+    const double k = ((double)__fmul_rn(f.k8, tau) + (double)__fmul_rn(f.k9, tau)) -
+                     ((double)__fmul_rn(f.k10, tau) + (double)__fmul_rn(f.k11, tau)) -
+                     ((double)__fmul_rn(f.k12, tau) + (double)__fmul_rn(f.k13, tau)) -
+                     ((double)__fmul_rn(f.k14, tau) + (double)__fmul_rn(f.k15, tau));
+    const double v = ((s7 + k) + ((double)a29 + (double)a30) + ((d4 * t + d3) * t + d2) * t2) / t3;
+    const float mag = f.abs_s7 + f.abs_k * tau + fabsf(a29) + fabsf(a30) +
+                      ((((float)d4) * tau + f.abs_d3) * tau + f.abs_d2) * tau * tau;
+    const double B = (double)mag * 0x1p-45 / t3 + fabs(v) * 0x1p-50;
+    const float lo = (float)(v - B), hi = (float)(v + B);
+    if (tau >= 1e-4f && tau <= 1e4f && lo == hi && fabsf(lo) > 1e-30f && fabsf(lo) < 1e30f) return lo;
+    return cost_dev(tau, st.a, st.b, coord_pow(st.a, st.b));
   }
-  float topt = 0;
-  float dcval = 1;
-  int maxItrs = 50;
-  int itr = 0;
-  while (fabsf(dcval) > 0.0001 && itr < maxItrs && ++itr) {
-    topt = (tu + tl) / 2;
-    dcval = dcost_dev(topt, a, b, p);
-    if (dcval > 0)
-      tu = topt;
-    else
-      tl = topt;
+  static __device__ __forceinline__ float cost(const float *x0, const float *x1, float tau) {
+    States st;
+#pragma unroll
+    for (int d = 0; d < kDim; ++d) {
+      st.a[d] = x0[d];
+      st.b[d] = x1[d];
+    }
+    return eval(st, tau);
   }
-  return topt;
-}
-
-// The reference expression's costs at ta and tb (each when wanted); out of
-// line, so that the registers of the binary64 powers do not count against
-// the pair kernel's occupancy (80-96 registers instead of 106: 10.57 ms ->
-// 10.04 ms at N = 4000 with 5 blocks of 128 per SM, 10.27 ms with 6).
-struct PairStates {
-  float a[kDim], b[kDim];
 };
-struct CostPair {
-  float ca, cb;
-};
-__device__ __noinline__ CostPair refgpu_costs(const PairStates st, float ta, float tb, bool want_a,
-                                              bool want_b) {
-  const CoordPow p = coord_pow(st.a, st.b);
-  CostPair r{0.0f, 0.0f};
-  if (want_a) r.ca = cost_dev(ta, st.a, st.b, p);
-  if (want_b) r.cb = cost_dev(tb, st.a, st.b, p);
-  return r;
+
+// N = 1000 (1 M pairs): 1.75-2.1 ms with two float-float costs per finite
+// difference and pow for what they do not certify (one wave, its warps held by
+// the pow evaluations), 0.24 ms now.
+__global__ void __launch_bounds__(kBisectThreads, 5) bvp_pairs_refgpu_kernel(AllPairs src, int chunk) {
+  __shared__ BisectQueue s_queue[kBisectWarps];
+  const long long left = (long long)src.N * (src.N - 1);
+  const int warp = threadIdx.x >> 5;
+  const long long first = (blockIdx.x * (long long)kBisectWarps + warp) * chunk;
+  if (first >= left) return;
+  bisect_warp<RefGpuCost, kBisectRefill>(src, s_queue[warp], first,
+                                        left - first < chunk ? (int)(left - first) : chunk);
 }
 
-// All ordered pairs: per lane, the evaluations of toptBisection as a state
-// machine (phase 0: the tmax test, 1: halving, 2: bisection, 3: the final
-// cost), two cost evaluations per step; a lane whose pair is done takes the
-// next pair of its warp's chunk of kChunk pairs.  Each evaluation is first
-// certified in float-float (cost_ff, ffcost.cuh); a lane whose value is not
-// certified waits until kFallback lanes of its warp wait (or no lane can go
-// on), and they evaluate the reference's expression (CUDA's pow included)
-// together.
-constexpr int kChunk = 512;
-constexpr int kFallback = 8;
-constexpr int kRefill = 8;
-
-__global__ void __launch_bounds__(128, 5) bvp_pairs_refgpu_kernel(const float *__restrict__ samples,
-                                                               int N, float tmax,
-                                                               float *__restrict__ copts,
-                                                               float *__restrict__ topts) {
-  const long long npairs = (long long)N * (N - 1);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  float dtau = 0.000001;
-  const float h = dtau / 2;
-  const long long warp_id = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-  long long chunk_next = warp_id * kChunk;
-  const long long chunk_end = chunk_next + kChunk < npairs ? chunk_next + kChunk : npairs;
-  long long idx = -1;
-  int phase = 0, halvings = 0, itr = 0;
-  float tu = 0, tl = 0, topt = 0, dcval = 0;
-  float a[kDim], b[kDim];
-  PairFF pf{};
-  float ta = 0, tb = 0, ca = 0, cb = 0;
-  bool pending = false, ok_a = true, ok_b = true;
-  while (true) {
-    // (refilled once kRefill lanes wait, or none has a pair, as in the parity
-    // kernel)
-    const unsigned need = __ballot_sync(0xffffffffu, idx < 0);
-    if (need && chunk_next < chunk_end && (__popc(need) >= kRefill || need == 0xffffffffu)) {
-      const int avail = (int)(chunk_end - chunk_next);
-      const int rank = __popc(need & lt);
-      if (((need >> lane) & 1u) && rank < avail) {
-        idx = chunk_next + rank;
-        const int i = (int)(idx / (N - 1));
-        const int r = (int)(idx - (long long)i * (N - 1));
-        const int j = r + (r >= i);
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) {
-          a[d] = __ldg(&samples[i * kDim + d]);
-          b[d] = __ldg(&samples[j * kDim + d]);
-        }
-        pf = make_pair_ff(a, b);
-        phase = 0;
-        tu = tmax;
-      }
-      chunk_next += __popc(need) < avail ? __popc(need) : avail;
-    }
-    const unsigned active = __ballot_sync(0xffffffffu, idx >= 0);
-    if (active == 0u) break;
-    if (idx >= 0 && !pending) {
-      if (phase == 0) { ta = tmax + h; tb = tmax - h; }
-      else if (phase == 1) { ta = tl + h; tb = tl - h; }
-      else if (phase == 2) { ++itr; topt = (tu + tl) / 2; ta = topt + h; tb = topt - h; }
-      else { ta = topt; tb = topt; }
-      ca = cost_ff(pf, ta, &ok_a);
-      cb = cost_ff(pf, tb, &ok_b);
-      pending = !(ok_a && ok_b);
-    }
-    const unsigned waiting = __ballot_sync(0xffffffffu, pending);
-    if (waiting && (__popc(waiting) >= kFallback || waiting == active)) {
-      if (pending) {
-        PairStates st;
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) {
-          st.a[d] = a[d];
-          st.b[d] = b[d];
-        }
-        const CostPair r = refgpu_costs(st, ta, tb, !ok_a, !ok_b);
-        if (!ok_a) ca = r.ca;
-        if (!ok_b) cb = r.cb;
-        pending = false;
-      }
-    }
-    if (idx < 0 || pending) continue;
-    const float d = (ca - cb) / dtau;
-    if (phase == 0) {
-      if (d < 0) { topt = tmax; phase = 3; }
-      else { tl = (float)0.01; halvings = 0; phase = 1; }
-    } else if (phase == 1) {
-      if (d > 0 && halvings < 160) { tl = tl / 2; ++halvings; }
-      else { topt = 0; dcval = 1; itr = 0; phase = 2; }
-    } else if (phase == 2) {
-      dcval = d;
-      if (dcval > 0) tu = topt; else tl = topt;
-      // (double)|dcval| > 0.0001 exactly when |dcval| > 0.0001f: binary32
-      // 0.0001f is below 0.0001 and the next binary32 above it
-      if (!(fabsf(dcval) > 0.0001f && itr < 50)) phase = 3;
-    } else {
-      topts[idx] = topt;
-      copts[idx] = ca;
-      idx = -1;
-    }
-  }
-}
-
-// Explicit pairs (the BvpJobs layout of ctx.h), one thread per (job, pair).
-__global__ void bvp_batch_refgpu_kernel(const BvpJobs jb) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= jb.n * jb.jobs) return;
-  const int j = k >= jb.n ? 1 : 0;
-  k -= j * jb.n;
-  float a[kDim], b[kDim];
-#pragma unroll
-  for (int d = 0; d < kDim; ++d) {
-    a[d] = jb.x0[k * kDim + d];
-    b[d] = jb.x1[(jb.x1_same ? 0 : k) * kDim + d];
-  }
-  const CoordPow p = coord_pow(a, b);
-  const float tp = topt_dev(a, b, p, jb.tmax[j]);
-  if (jb.topt[j]) jb.topt[j][k] = tp;
-  if (jb.cost[j]) jb.cost[j][k] = cost_dev(tp, a, b, p);
+// Explicit pairs (the BvpJobs layout of ctx.h), 32 per warp.
+__global__ void __launch_bounds__(128) bvp_batch_refgpu_kernel(const JobPairs src) {
+  const long long total = (long long)src.jb.n * src.jb.jobs;
+  __shared__ BisectQueue s_queue[kBisectWarps];
+  const int warp = threadIdx.x >> 5;
+  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * 32;
+  if (first >= total) return;
+  bisect_warp<RefGpuCost, 32>(src, s_queue[warp], first, total - first < 32 ? (int)(total - first) : 32);
 }
 
 }  // namespace
@@ -239,9 +141,11 @@ __global__ void bvp_batch_refgpu_kernel(const BvpJobs jb) {
 pump_status_t bvp_pairs_refgpu_launch(const float *d_samples, int N, float tmax, float *d_copts,
                                       float *d_topts, cudaStream_t stream) {
   const long long npairs = (long long)N * (N - 1);
-  const long long nblk = (npairs + 4LL * kChunk - 1) / (4LL * kChunk);  // 4 warps per block
+  const int chunk = bisect_chunk(npairs);
+  const long long per = (long long)kBisectWarps * chunk, nblk = (npairs + per - 1) / per;
   if (nblk > 2147483647LL) return set_error(PUMP_ERR_CAPACITY, "pump_bvp_pairs: N=%d", N);
-  bvp_pairs_refgpu_kernel<<<(unsigned)nblk, 128, 0, stream>>>(d_samples, N, tmax, d_copts, d_topts);
+  bvp_pairs_refgpu_kernel<<<(unsigned)nblk, kBisectThreads, 0, stream>>>(
+      AllPairs{d_samples, N, tmax, d_copts, d_topts}, chunk);
   return launch_status("bvp_pairs_refgpu");
 }
 
@@ -249,7 +153,7 @@ pump_status_t bvp_jobs_refgpu_launch(const BvpJobs &jb, cudaStream_t stream) {
   if (jb.n <= 0) return PUMP_OK;
   const long long total = (long long)jb.n * jb.jobs;
   const int threads = total < 152LL * 128 ? 32 : 128;
-  bvp_batch_refgpu_kernel<<<grid_for(total, threads), threads, 0, stream>>>(jb);
+  bvp_batch_refgpu_kernel<<<grid_for(total, threads), threads, 0, stream>>>(JobPairs{jb});
   return launch_status("bvp_batch_refgpu");
 }
 

@@ -80,6 +80,38 @@ def test_bvp_pairs_parity_random(gpu, pumplib, oracle):
     assert same_bits(t, rt) and same_bits(c, rc)
 
 
+@pytest.mark.parametrize("tmax", [5.0, 0.005, 60.0])
+@pytest.mark.parametrize("kind", ["plain", "near", "nearer", "x10", "x1e-3", "shift", "rest", "same", "special"])
+def test_bvp_pairs_parity_certified_steps(kind, tmax, gpu, pumplib, oracle):
+    """The bisection's steps taken without evaluating the costs, over states
+    where the certificates fail or leave their range: nearly equal and equal
+    states, other scales, a far origin, NaN and infinite coordinates, brackets
+    at both ends of the range.  Bit for bit; 37 samples: 1332 pairs, not a
+    multiple of a warp's or a block's share."""
+    torch, _ = gpu
+    rng = np.random.default_rng(17)
+    s = np.concatenate([rng.uniform(0, 1, (37, 3)), rng.uniform(-1, 1, (37, 3))], 1)
+    if kind in ("near", "nearer"):
+        s = s[0] + (s - s[0]) * (1e-2 if kind == "near" else 1e-4)
+    if kind == "x10":
+        s = s * 10
+    if kind == "x1e-3":
+        s = s * 1e-3
+    if kind == "shift":
+        s[:, :3] += 100
+    if kind == "rest":
+        s[:, 3:] = 0
+    if kind == "same":
+        s = s[rng.integers(0, 4, 37)]
+    s = s.astype(np.float32)
+    if kind == "special":
+        s[3, 2], s[5, 4], s[9, 1], s[11, 5] = np.nan, np.inf, 3e38, 1e-40
+    c, t = run_bvp_pairs(torch, pumplib, s, tmax=tmax)
+    rc, rt = oracle.bvp_pairs(s, tmax)
+    nan = np.isnan(rc)
+    assert np.array_equal(np.isnan(c), nan) and same_bits(t, rt) and same_bits(c[~nan], rc[~nan])
+
+
 def test_bvp_batch_parity(gpu, pumplib, oracle):
     torch, _ = gpu
     L = pumplib.load()
