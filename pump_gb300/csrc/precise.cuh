@@ -8,16 +8,16 @@
 //   A0 = 12|p1-p0|^2, A1 = -12 (p1-p0).(v0+v1), A2 = 4(|v0|^2+v0.v1+|v1|^2),
 //   A3 = 2g(v0z-v1z), A4 = 1+g^2,
 // so c'(t) = 0 is the quartic Q(t) = A4 t^4 - A2 t^2 - 2 A1 t - 3 A0 = 0.
-// The coefficients are assembled exactly enough in float-float (pairs of
-// binary32, ~46-bit significands) on the FP32 pipe; the roots of Q are
-// bracketed in binary32 (pieces split at the inflection point and the real
-// roots of Q'); each candidate minimum is refined with one Newton step whose
-// residual Q(x) is evaluated in binary64 (the FP64 pipe, ~1/64 of the FP32
-// rate on this GPU, does only Q(x) and the cost); the candidates (and tmax)
-// are compared by their binary64 cost.  Translation units including this header are compiled
-// with multiply-add contraction (the mode is not bound to the reference's
-// roundings): the binary64 Horner evaluations issue as DFMA, half the
-// FP64-pipe instructions of separate multiply and add.
+// The coefficients are assembled in float-float (pairs of binary32, ~46-bit
+// significands).  For almost every pair the root, one Newton step and the cost
+// follow in binary32 and float-float with a bound on their error, and the
+// rounded results are certain (precise_min).  The other pairs take the general
+// way: the roots of Q are bracketed in binary32 (pieces split at the
+// inflection point and the real roots of Q'); each candidate minimum is
+// refined with one Newton step whose residual Q(x) is evaluated in binary64;
+// the candidates (and tmax) are compared by their binary64 cost.  Translation
+// units including this header are compiled with multiply-add contraction (the
+// mode is not bound to the reference's roundings).
 #pragma once
 #include <math.h>
 
@@ -214,39 +214,65 @@ __device__ __forceinline__ int minima_f32(const QuarticF &q, float tmax, float *
 
 // Coefficients of one pair: A0 = 12|D|^2, A1 = -12 D.S, A2 = 4(|v0|^2 +
 // v0.v1 + |v1|^2), A3 = 2g(v0z - v1z) with D = p1 - p0, S = v0 + v1, in
-// float-float (differences and products exact, sums to ~2^-46), then the
-// binary32 copies (the high parts) for bracketing and binary64 values (hi +
-// lo, one addition each) for the refinement and the cost.
-struct PairQuartic {
-  QuarticF f;
-  Quartic q;
+// float-float (differences and products exact, sums to ~2^-44 of their terms'
+// magnitudes), and |D|.|S| summed by magnitude.
+struct PairCoefs {
+  FF dd, ds, A2s, A3;  // |D|^2, D.S, A2 / 4, A3
+  float abs_ds;        // sum of |D_d S_d|
 };
-
-__device__ __forceinline__ PairQuartic make_pair_quartic(const SampleF &a, const SampleF &b) {
+// x y added to the float-float sum s: the product exact to u^2, its high part
+// by TwoSum, the errors in binary32.
+__device__ __forceinline__ void ff_accum(FF x, FF y, FF *s) {
+  const FF p = two_prod(x.h, y.h);
+  const float pl = fmaf(x.h, y.l, fmaf(x.l, y.h, p.l));
+  const FF t = two_sum(s->h, p.h);
+  s->h = t.h;
+  s->l = s->l + (t.l + pl);
+}
+__device__ __forceinline__ PairCoefs make_pair_coefs(const SampleF &a, const SampleF &b) {
+  PairCoefs r;
   FF D[3], S[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     D[d] = two_sum(b.p[d], -a.p[d]);
     S[d] = two_sum(a.v[d], b.v[d]);
   }
-  const FF dd = ff_add(ff_add(ff_mul(D[0], D[0]), ff_mul(D[1], D[1])), ff_mul(D[2], D[2]));
-  const FF ds = ff_add(ff_add(ff_mul(D[0], S[0]), ff_mul(D[1], S[1])), ff_mul(D[2], S[2]));
-  const FF v01 = ff_add(ff_add(two_prod(a.v[0], b.v[0]), two_prod(a.v[1], b.v[1])),
-                        two_prod(a.v[2], b.v[2]));
-  const FF A0 = ff_mulf(dd, 12.0f), A0x3 = ff_mulf(dd, 36.0f);
-  const FF A1 = ff_mulf(ds, -12.0f), A1x2 = ff_mulf(ds, -24.0f);
-  const FF A2s = ff_add(ff_add(a.vv, v01), b.vv);
-  const FF A3 = ff_mulf(two_sum(a.v[2], -b.v[2]), 2.0f * PUMP_G);
+  FF dd = {0.0f, 0.0f}, ds = {0.0f, 0.0f}, vv = a.vv;
+  r.abs_ds = 0.0f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    ff_accum(D[d], D[d], &dd);
+    ff_accum(D[d], S[d], &ds);
+    ff_accum({a.v[d], 0.0f}, {b.v[d], 0.0f}, &vv);
+    r.abs_ds = fmaf(fabsf(D[d].h), fabsf(S[d].h), r.abs_ds);
+  }
+  r.dd = fast_two_sum(dd.h, dd.l);
+  r.ds = two_sum(ds.h, ds.l);
+  r.A2s = ff_add({vv.h, vv.l}, b.vv);
+  r.A3 = ff_mulf(two_sum(a.v[2], -b.v[2]), 2.0f * PUMP_G);
+  return r;
+}
+
+// The binary32 copies (the high parts) for bracketing and the binary64 values
+// (hi + lo, one addition each) for the refinement and the cost.
+struct PairQuartic {
+  QuarticF f;
+  Quartic q;
+};
+
+__device__ __forceinline__ PairQuartic make_pair_quartic(const PairCoefs &c) {
+  const FF A0 = ff_mulf(c.dd, 12.0f), A0x3 = ff_mulf(c.dd, 36.0f);
+  const FF A1 = ff_mulf(c.ds, -12.0f), A1x2 = ff_mulf(c.ds, -24.0f);
   const double g = (double)PUMP_G;
   PairQuartic r;
   r.f.A0 = A0.h;
   r.f.A1 = A1.h;
-  r.f.A2 = 4.0f * A2s.h;
+  r.f.A2 = 4.0f * c.A2s.h;
   r.f.A4 = fmaf(PUMP_G, PUMP_G, 1.0f);
   r.q.A0 = ff2d(A0);
   r.q.A1 = ff2d(A1);
-  r.q.A2 = 4.0 * ff2d(A2s);
-  r.q.A3 = ff2d(A3);
+  r.q.A2 = 4.0 * ff2d(c.A2s);
+  r.q.A3 = ff2d(c.A3);
   r.q.A4 = 1.0 + g * g;
   r.q.A0x3 = ff2d(A0x3);
   r.q.A1x2 = ff2d(A1x2);
@@ -265,43 +291,151 @@ __device__ __forceinline__ double refine(const PairQuartic &pq, float x) {
   return ok ? fma(-f, f2d_exact(r), xd) : xd;
 }
 
-// Global minimiser of the cost on (0, tmax]: candidates from the binary32
-// analysis, each refined by one Newton step (quadratic convergence takes a
-// ~1e-6 relative root to ~1e-12) and compared by their binary64 cost.  In
-// the common case of one candidate the binary64 work is the same
-// straight-line sequence for every pair, so the FP64 pipe runs with full
-// warps.
-// Global minimiser on (0, tmax] in binary64 (*t) and its binary64 cost (*c).
-__device__ __forceinline__ void precise_tau(const SampleF &a, const SampleF &b, float tmax,
-                                            double *t_out, double *c_out) {
-  const PairQuartic pq = make_pair_quartic(a, b);
+// Global minimiser of the cost on (0, tmax] and its cost, any pair: candidates
+// from the binary32 analysis, each refined by one Newton step in binary64
+// (quadratic convergence takes a ~1e-6 relative root to ~1e-12) and compared
+// by their binary64 cost.  Out of line: one pair in thousands needs it
+// (precise_min).
+struct Minimum64 {
+  double t, c;
+};
+__device__ __noinline__ Minimum64 precise_general(const PairCoefs pc, float tmax) {
+  const PairQuartic pq = make_pair_quartic(pc);
   float cand[2] = {0.0f, 0.0f};
   bool tmax_cand = false;
   const int nc = minima_f32(pq.f, tmax, &cand[0], &cand[1], &tmax_cand);
-  // primary candidate, evaluated by every lane with the same instructions
   const bool primary_root = nc > 0;
   const double tm = f2d_exact(tmax);
   const double xr = refine(pq, primary_root ? cand[0] : tmax);
-  double best_t = primary_root ? xr : tm;
-  double best_c = pq.q.cost(best_t);
-  // rare: a second interior minimum, or the cost still falling at tmax
+  Minimum64 m;
+  m.t = primary_root ? xr : tm;
+  m.c = pq.q.cost(m.t);
   if (nc > 1) {
     const double t2 = refine(pq, cand[1]);
     const double c2 = pq.q.cost(t2);
-    if (c2 < best_c) { best_c = c2; best_t = t2; }
+    if (c2 < m.c) { m.c = c2; m.t = t2; }
   }
   if (primary_root && tmax_cand) {
     const double c3 = pq.q.cost(tm);
-    if (c3 < best_c) { best_c = c3; best_t = tm; }
+    if (c3 < m.c) { m.c = c3; m.t = tm; }
   }
-  *t_out = best_t;
-  *c_out = best_c;
+  return m;
 }
 
-// The same for a pair given only in binary32.
-__device__ __forceinline__ void precise_tau(const float *x0, const float *x1, float tmax,
-                                            double *t_out, double *c_out) {
-  precise_tau(to_sample_f(x0), to_sample_f(x1), tmax, t_out, c_out);
+// Whether every value within `bound` of h + l rounds to h in binary32.
+__device__ __forceinline__ bool rounds_to(float h, float l, float bound) {
+  const float ah = fabsf(h);
+  const unsigned u = __float_as_uint(ah), e = u >> 23;
+  const float room = 0.5f * fminf(__uint_as_float(u + 1u) - ah, ah - __uint_as_float(u - 1u)) - fabsf(l);
+  return e >= 2u && e <= 253u && bound < 0.99f * room;
+}
+__device__ __forceinline__ float rcp_f32(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sqrt_f32(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// The optimal time and cost, correctly rounded binary32 values (t, c) with
+// the rest of the time in dt (t + dt: about 2^-44 relative).
+//
+// In almost every pair Q has one positive root, which is then the cost's only
+// minimum (c' = Q / t^4).  With tc = sqrt(A2 / (6 A4)), the inflection point of
+// Q, that is certain when A1 >= 0 (one sign change); when A1 < 0 and Q' has no
+// zero on t > 0 (|A1| >= 2/3 A2 tc: Q increases); and when Q < 0 up to tc (A4
+// tc^4 + 2 |A1| tc < 3 A0), since Q is convex beyond (the last two tested with
+// 1e-3 margins).  The root comes from two closed-form steps (the biquadratic
+// without the linear term, then with that term frozen at its root) and three
+// Halley steps in binary32: of 2 M random pairs, all are within 1e-4 before
+// the third step, which leaves its cube.  Any positive root that the steps
+// converge to is the root.
+//
+// Then one Newton step with the residual Q(x) in float-float gives dx, and the
+// cost at the root is c(x) + c'(x) dx / 2 (c' vanishes at the root; third
+// order), c(x) in float-float.  Errors, u = 2^-24, as multiples of the terms'
+// magnitudes: the coefficients at most 36 u^2, 1/x 6 u^2 a factor, each product
+// 6 u^2 and sum 8 u^2: under 140 u^2 for the cost, 100 u^2 for Q.  The bounds
+// take 2^-40 (256 u^2).  Where a bound reaches a rounding boundary (about 1e-4
+// of pairs) and wherever a condition fails, precise_general decides.
+//
+// Why float-float: the binary64 pipe runs at 1/64 of the binary32 rate here,
+// so the 18 binary64 instructions a pair that the refinement and the cost used
+// to take bounded the pair kernel at 0.54 ms for N = 4000, and their
+// conversions and the bracketing filled the rest of the issue slots.
+struct PreciseMin {
+  float t, dt, c;
+};
+__device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const SampleF &sb, float tmax) {
+  const PairCoefs pc = make_pair_coefs(sa, sb);
+  constexpr double kA4d = 1.0 + (double)PUMP_G * (double)PUMP_G;
+  constexpr float kA4 = (float)kA4d, kA4l = (float)(kA4d - (double)kA4), kR4 = (float)(1.0 / kA4d);
+  // Q / A4 = t^4 - a t^2 - b t - c
+  const float a = pc.A2s.h * (4.0f * kR4), b = pc.ds.h * (-24.0f * kR4), c = pc.dd.h * (36.0f * kR4);
+  const float tc = sqrt_f32(a * (1.0f / 6.0f));
+  const float tc2 = tc * tc;
+  const bool unique = b >= 0.0f || -b >= 1.334f * a * tc || tc * fmaf(tc2, tc, -b) < 0.999f * c;
+  const float aa = a * a;
+  const float t0 = sqrt_f32(0.5f * (a + sqrt_f32(fmaf(4.0f, c, aa))));
+  const float t1 = 0.5f * (a + sqrt_f32(fmaxf(fmaf(4.0f, fmaf(b, t0, c), aa), c)));
+  float x = sqrt_f32(t1), step = 0.0f;
+#pragma unroll
+  for (int it = 0; it < 3; ++it) {
+    const float x2 = x * x;
+    const float q = fmaf(fmaf(x2 - a, x, -b), x, -c);
+    const float dq = fmaf(fmaf(4.0f, x2, -2.0f * a), x, -b);
+    const float r = rcp_f32(dq);
+    const float s = q * r;
+    // Halley: s / (1 - s q'' / (2 q')), the quotient by its own estimate
+    step = s * rcp_f32(fmaf(-s * r, fmaf(6.0f, x2, -a), 1.0f));
+    x = x - step;
+  }
+  bool ok = unique && fabsf(step) <= 2e-3f * x && x >= 1e-6f && x <= 1e6f;
+  const bool beyond = x > tmax * 1.00001f;  // the cost still falls at tmax
+  x = fminf(x, tmax);
+  // Q(x), the Newton step and its error
+  const FF x2 = two_prod(x, x);
+  const FF A2 = {4.0f * pc.A2s.h, 4.0f * pc.A2s.l};
+  FF q = ff_mul({kA4, kA4l}, x2);
+  const float dq = fmaf(fmaf(4.0f, q.h, -2.0f * A2.h), x, 24.0f * pc.ds.h);
+  const float ddq = fmaf(12.0f, q.h, 2.0f * A2.h) * 1.01f;  // (over its magnitude)
+  const float mq = fmaf(fmaf(q.h + 3.0f * A2.h, x, 24.0f * pc.abs_ds), x, 36.0f * pc.dd.h);
+  q = ff_mulf(ff_add(q, {-A2.h, -A2.l}), x);
+  q = ff_mulf(ff_add(q, ff_mulf(pc.ds, 24.0f)), x);
+  q = ff_add(q, ff_mulf(pc.dd, -36.0f));
+  const float r = rcp_f32(x);
+  const float rq = rcp_f32(dq);
+  float dx = -(q.h * rq);
+  if (x >= tmax) dx = beyond ? 0.0f : fminf(dx, 0.0f);
+  const float bt = beyond ? 0.0f
+                          : fabsf(rq) * fmaf(fabsf(dx), fmaf(mq * r, 0x1p-18f, fabsf(dx) * ddq), mq * 0x1p-40f);
+  ok = ok && fabsf(dx) <= 0x1p-18f * x && (beyond || dq > 0.0f);
+  // c(x) = A3 + A4 x + r (A2 + r (A1 + r A0)), 1/x in float-float
+  const FF rr = {r, r * fmaf(-x, r, 1.0f)};
+  FF v = ff_add(ff_mul(ff_mulf(pc.dd, 12.0f), rr), ff_mulf(pc.ds, -12.0f));
+  v = ff_add(ff_mul(v, rr), A2);
+  v = ff_add(ff_mul(v, rr), pc.A3);
+  v = ff_add(v, ff_mulf({kA4, kA4l}, x));
+  const float r2 = r * r;
+  const float mc = fmaf(r, fmaf(r, fmaf(r, 12.0f * pc.dd.h, 12.0f * pc.abs_ds), 3.0f * A2.h),
+                        fmaf(kA4, x, fabsf(pc.A3.h)));
+  v = fast_two_sum(v.h, fmaf(q.h * r2 * r2, beyond ? 0.0f : 0.5f * dx, v.l));
+  PreciseMin m;
+  const FF t = fast_two_sum(x, dx);
+  m.t = t.h;
+  m.dt = t.l;
+  m.c = v.h;
+  ok = ok && rounds_to(t.h, t.l, bt) && rounds_to(v.h, v.l, mc * 0x1p-40f);
+  if (!ok) {
+    const Minimum64 g = precise_general(pc, tmax);
+    m.t = d2f_rn(g.t);
+    m.dt = (float)(g.t - (double)m.t);
+    m.c = d2f_rn(g.c);
+  }
+  return m;
 }
 
 }  // namespace

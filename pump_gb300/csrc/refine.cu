@@ -2,7 +2,7 @@
 // its adjoint with respect to the intermediate nodes, and a gradient descent
 // over many paths whose loop is captured into a CUDA graph (include/pump.h
 // states the objective).  One CTA per path:
-//   1. segments: the binary64 optimal time tau_i (precise.cuh), the cost, the
+//   1. segments: the optimal time tau_i (precise.cuh), the cost, the
 //      cost's partial derivatives and dtau/dx by the implicit function theorem;
 //   2. segment start times (warp scan of tau);
 //   3. waypoints: one warp per segment, its waypoints in order, lanes over the
@@ -13,7 +13,8 @@
 //   4. start-time adjoints to earlier taus (suffix scan), taus to nodes.
 // Every sum runs in a fixed order (no floating-point atomics), so results
 // are the same from run to run.
-// Binary64 only for the optimal time; everything else binary32.  This
+// The optimal time and the cost are correctly rounded (float-float, binary64
+// where that is not certain); everything else is binary32.  This
 // translation unit is compiled with multiply-add contraction.
 #include <math.h>
 #include <string.h>
@@ -113,11 +114,10 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
       x0[d] = x[i * 6 + d];
       x1[d] = x[i * 6 + 6 + d];
     }
-    double td, cd;
-    precise_tau(x0, x1, a.tmax, &td, &cd);
-    const float t = (float)td;
+    const PreciseMin pm = precise_min(to_sample_f(x0), to_sample_f(x1), a.tmax);
+    const float t = pm.t;
     s_tau[i] = t;
-    csum += (float)cd;
+    csum += pm.c;
     if (Grad) {
       // dA/dx of A0 = 12|D|^2, A1 = -12 D.S, A2 = 4(v0.v0 + v0.v1 + v1.v1),
       // A3 = 2g(v0z - v1z) with D = p1 - p0, S = v0 + v1
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
       A2 *= 4.0f;
       const float r1 = 1.0f / t, r2 = r1 * r1, r3 = r2 * r1, r4 = r2 * r2, r5 = r4 * r1;
       const float Ft = 12.0f * A0 * r5 + 6.0f * A1 * r4 + 2.0f * A2 * r3;  // c''(tau)
-      const bool clamped = td >= (double)a.tmax;
+      const bool clamped = t > a.tmax || (t == a.tmax && pm.dt >= 0.0f);
       const float g2 = 2.0f * PUMP_G;
 #pragma unroll
       for (int m = 0; m < 12; ++m) {

@@ -821,6 +821,37 @@ def test_bvp_pairs_precision_vs_long_double(gpu, pumplib, oracle, goldens):
     assert far_t <= 2, stats
 
 
+@pytest.mark.parametrize("tmax", [5.0, 0.4])
+@pytest.mark.parametrize("kind", ["plain", "near", "x10", "x1e-3", "rest"])
+def test_bvp_pairs_precision_certified_and_general(kind, tmax, gpu, pumplib, oracle):
+    """Both ways to the optimum, the certified one and the general one (nearly
+    equal states have several stationary points or miss a bound), with the
+    minimum inside the bracket and at tmax: the correctly rounded cost and time
+    of the binary64 minimiser, so at most 1 ulp from its binary32 rounding (2
+    for the time, whose binary64 value moves by more than the cost's)."""
+    torch, _ = gpu
+    rng = np.random.default_rng(23)
+    N = 45
+    s = np.concatenate([rng.uniform(0, 1, (N, 3)), rng.uniform(-1, 1, (N, 3))], 1)
+    if kind == "near":
+        s = s[0] + (s - s[0]) * 1e-2
+    if kind == "x10":
+        s = s * 10
+    if kind == "x1e-3":
+        s = s * 1e-3
+    if kind == "rest":
+        s[:, 3:] = 0
+    s = s.astype(np.float32)
+    c, t = run_bvp_pairs(torch, pumplib, s, mode=pumplib.PUMP_BVP_PRECISION, tmax=tmax)
+    i, j = np.nonzero(~np.eye(N, dtype=bool))
+    t64, c64 = oracle.bvp_binary64(s[i], s[j], tmax)
+
+    def ulps(a, b):
+        return np.abs(a.view(np.int32).astype(np.int64) - b.astype(np.float32).view(np.int32))
+    assert ulps(c, c64).max() <= 1
+    assert ulps(t, t64).max() <= 2
+
+
 def test_mc_cp_binary32_vs_binary64(gpu, pumplib, oracle):
     """The binary32 Monte Carlo CP (collision tests as the reference's, in
     binary32) against the same estimate with every test in binary64: hit
