@@ -186,8 +186,6 @@ pump_status_t roadmap_pairs_edges(Ctx *ctx, const float *d_samples, int N, float
                                   bool cooperative = true);
 pump_status_t frontier_compact_device(Ctx *ctx, const uint8_t *d_flags, int N, int *d_active,
                                       int *d_count, int **d_error_out, cudaStream_t stream);
-pump_status_t particle_rowmax_async(const float *d_table, int P, int T, float *d_rowmax,
-                                    cudaStream_t stream);
 pump_status_t particle_tables_async(uint64_t seed, int P, int T, float *d_tmajor, float *d_pmajor,
                                     cudaStream_t stream);
 pump_status_t bvp_pairs_precision_launch(const float *d_samples, int N, float tmax, float *d_copts,
@@ -288,8 +286,7 @@ pump_status_t candidate_paths_async(const CandidateBufs &cb, int n_paths, int n_
 pump_status_t mc_cp_hits_async(const float *d_paths, const int *d_offset, const int *d_len,
                                int n_paths, const float *d_offsets_t, int Pmc, int T_rows,
                                float offset_mult, const float *d_obstacles, int numObs,
-                               int *d_hits, cudaStream_t stream, const float *d_rowmax,
-                               const int *copy_src = nullptr, int *copy_dst = nullptr,
+                               int *d_hits, cudaStream_t stream, const int *copy_src = nullptr, int *copy_dst = nullptr,
                                int copy_words = 0, unsigned int *done = nullptr,
                                unsigned int seq = 0);
 // Halton samples of a query (sampler.cu:20-41), N x 6, then (goal_row) the

@@ -24,6 +24,10 @@
 //
 // Monte Carlo CP.  Thread per (particle, path) over many paths per launch;
 // obstacles staged in shared memory; the same segment test as freeEdges.
+#include <math.h>
+
+#include <type_traits>
+
 #include "collide.cuh"
 #include "search.h"
 
@@ -638,86 +642,129 @@ inline const void *hsmc_loop_kernel_for(int P) {
 // collisionProbability.cu:39-92.  A particle collides when any of the
 // segments t = 0 .. T-3 of its perturbed path hits a box; the reference walks
 // the segments in order and stops at the first hit, which gives the same
-// answer as testing all of them.  Block = 32 particles (the lanes) x
-// kMcWarps warps; warp w tests segments t = w, w + kMcWarps, ...; the
-// per-particle OR over warps is taken in shared memory and the block adds
-// its popcount to hits[k].  Grid (ceil(Pmc / 32), paths).
-// MC CP of path k (blockIdx.y): 32 particles per block (one per lane), the
-// kMcWarps warps splitting the path's segments (16: a smoothing batch of a
-// few paths is a few hundred blocks, so the segments are split finely to
-// shorten each warp's chain).  With rowmax (the largest |offset|
-// per table row and axis), each block first marks, per segment, the boxes
-// that some particle's segment could touch: the path segment's bounding box
-// widened by fl(rowmax * |offset_mult|) on both ends.  A particle's position
-// fl(path + fl(offset * offset_mult)) lies inside that box by the
-// monotonicity of rounding, so a box disjoint from it is broadphase-disjoint
-// from every particle's segment and the reference's test of it passes; only
-// the marked boxes are tested, in index order.  Without rowmax (or with more
-// than kMcFilterObs boxes, or a NaN state) every box is tested.
-constexpr int kMcFilterObs = 128;
+// answer as testing all of them.
+//
+// Block = 32 K particles (K per lane) of one path x kMcWarps warps, which
+// split the path's segments into consecutive runs (a run carries a segment's
+// end over as the next one's start).  Per segment the warp takes the bounding
+// box of its particles' segments (the ones that have not collided) by warp
+// reductions, tests the boxes against it one per lane, and only those that it
+// is not broadphase-disjoint from are tested per particle: a box disjoint
+// from the common bounding box is disjoint from every particle's, whose
+// reference test then passes.  With a NaN coordinate every box is kept.  (One
+// particle per lane and every box tested by every particle: 268 us for 64
+// paths x 2048 particles and 40 boxes.)  Bound by instruction issue for large
+// calls, by one warp's chain of segments for small ones; hence K: particles
+// per lane share the reductions and box tests of a large call (K = 4), and a
+// small call spreads over the SMs (K = 1).
 constexpr int kMcWarps = 16;
 
+__device__ __forceinline__ float warp_min_f32(float x) {
+  float y;
+  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float warp_max_f32(float x) {
+  float y;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Grid (ceil(Pmc / (32 K)), paths).
+template <int K>
 __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
     const float *__restrict__ paths, const int *__restrict__ offset, const int *__restrict__ len,
     const float *__restrict__ offsets_t, int Pmc, int T_rows, float offset_mult,
     const float *__restrict__ obs, int numObs, int k0, int *__restrict__ hits,
-    const float *__restrict__ rowmax, const int *copy_src, int *copy_dst, int copy_words,
-    unsigned int *done, unsigned int seq) {
+    const int *copy_src, int *copy_dst, int copy_words, unsigned int *done, unsigned int seq) {
   extern __shared__ float4 s_obs4[];
   float *s_obs = reinterpret_cast<float *>(s_obs4);
-  uint32_t *s_mask = reinterpret_cast<uint32_t *>(s_obs + ((numObs * 12 + 3) & ~3));
-  __shared__ unsigned int s_hit[kMcWarps];
+  __shared__ unsigned int s_hit[K][kMcWarps];
   stage_obstacles(obs, numObs, s_obs);
-  const int k = k0 + blockIdx.y;
+  const int path_k = k0 + blockIdx.y;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = blockIdx.x * 32 + lane;
-  const int T = len[k];
-  const float *path = paths + (long long)offset[k] * kDim;
-  const bool filter = rowmax != nullptr && numObs <= kMcFilterObs && T <= T_rows;
-  if (filter) {
-    const float om = fabsf(offset_mult);
-    for (int t = threadIdx.x; t < T - 2; t += blockDim.x) {
-      float lo[3], hi[3];
-      bool nan = false;
+  const int p0 = blockIdx.x * (32 * K) + lane;
+  const int T = len[path_k];
+  const float *path = paths + (long long)offset[path_k] * kDim;
+  const int segs = T <= T_rows ? T - 2 : 0;
+  const int per = segs > 0 ? (segs + kMcWarps - 1) / kMcWarps : 0;
+  const int t0 = warp * per, t1 = t0 + per < segs ? t0 + per : segs;
+  unsigned int todo = 0u;  // bit k: particle p0 + 32 k exists and has not collided
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float m0 = rowmax[t * 3 + d] * om, m1 = rowmax[(t + 1) * 3 + d] * om;
-        const float a = path[t * kDim + d], b = path[(t + 1) * kDim + d];
-        nan = nan || a != a || b != b;
-        lo[d] = fminf(a - m0, b - m1);
-        hi[d] = fmaxf(a + m0, b + m1);
-      }
-      uint32_t m[kMcFilterObs / 32] = {0u, 0u, 0u, 0u};
-      for (int o = 0; o < numObs; ++o)
-        if (nan || !broadphase_valid(lo, hi, &s_obs[o * 12])) m[o >> 5] |= 1u << (o & 31);
+  for (int k = 0; k < K; ++k)
+    if (p0 + 32 * k < Pmc) todo |= 1u << k;
+  unsigned int coll = 0u;
+  float v[K][3], w[K][3];
+  auto load = [&](int t, float (&x)[K][3]) {
 #pragma unroll
-      for (int q = 0; q < kMcFilterObs / 32; ++q) s_mask[t * (kMcFilterObs / 32) + q] = m[q];
+    for (int k = 0; k < K; ++k) {
+      const int p = p0 + 32 * k < Pmc ? p0 + 32 * k : Pmc - 1;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        x[k][d] = path[t * kDim + d] + __ldg(&offsets_t[((long long)t * Pmc + p) * 3 + d]) * offset_mult;
     }
-    __syncthreads();
-  }
-  bool coll = false;
-  if (p < Pmc && T <= T_rows) {
-    const int words = (numObs + 31) / 32;
-    for (int t = warp; t < T - 2 && !coll; t += kMcWarps) {
-      float v[3], w[3];
+  };
+  if (t0 < t1) load(t0, v);
+  for (int t = t0; t < t1; ++t) {
+    if (!__any_sync(0xffffffffu, todo != 0u)) break;
+    load(t + 1, w);
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool nan = false;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        v[d] = path[t * kDim + d] + __ldg(&offsets_t[((long long)t * Pmc + p) * 3 + d]) * offset_mult;
-        w[d] = path[(t + 1) * kDim + d] +
-               __ldg(&offsets_t[((long long)(t + 1) * Pmc + p) * 3 + d]) * offset_mult;
-      }
-      coll = filter ? !segment_valid_masked(v, w, &s_mask[t * (kMcFilterObs / 32)], words, s_obs)
-                    : !segment_valid(v, w, numObs, s_obs);
+    for (int k = 0; k < K; ++k)
+      if ((todo >> k) & 1u)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          nan = nan || v[k][d] != v[k][d] || w[k][d] != w[k][d];
+          lo[d] = fminf(lo[d], fminf(v[k][d], w[k][d]));
+          hi[d] = fmaxf(hi[d], fmaxf(v[k][d], w[k][d]));
+        }
+    nan = __any_sync(0xffffffffu, nan);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = warp_min_f32(lo[d]);
+      hi[d] = warp_max_f32(hi[d]);
     }
+    for (int c0 = 0; c0 < numObs; c0 += 32) {
+      bool keep = false;
+      if (c0 + lane < numObs) {
+        const float4 *bx = s_obs4 + (c0 + lane) * 3;
+        const float4 a = bx[0], b = bx[1], c = bx[2];  // lo = a.xyz, hi = (b.z, b.w, c.x)
+        keep = nan || !((hi[0] <= a.x) | (b.z <= lo[0]) | (hi[1] <= a.y) | (b.w <= lo[1]) |
+                        (hi[2] <= a.z) | (c.x <= lo[2]));
+      }
+      unsigned int boxes = __ballot_sync(0xffffffffu, keep);
+      while (boxes) {
+        const float *ob = &s_obs[(c0 + __ffs(boxes) - 1) * 12];
+        boxes &= boxes - 1u;
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (((todo >> k) & 1u) && segment_box_hit(v[k], w[k], ob)) {
+            coll |= 1u << k;
+            todo &= ~(1u << k);
+          }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[k][d] = w[k][d];
   }
-  const unsigned int bal = __ballot_sync(0xffffffffu, coll);
-  if (lane == 0) s_hit[warp] = bal;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const unsigned int bal = __ballot_sync(0xffffffffu, (coll >> k) & 1u);
+    if (lane == 0) s_hit[k][warp] = bal;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int any = 0;
-    for (int q = 0; q < kMcWarps; ++q) any |= s_hit[q];
-    const int total = __popc(any);
-    if (total) atomicAdd(&hits[k], total);
+  if (warp == 0) {
+    int total = 0;
+    if (lane < K) {
+      unsigned int any = 0;
+      for (int q = 0; q < kMcWarps; ++q) any |= s_hit[lane][q];
+      total = __popc(any);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0 && total) atomicAdd(&hits[path_k], total);
   }
   if (copy_dst) {
     // the last block to finish copies the caller's results (hit counts
@@ -742,30 +789,6 @@ __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
   }
 }
 
-// Largest |offset| per row and axis of the time-major table (T rows of P
-// particles), for the MC CP box filter.
-__global__ void particle_rowmax_kernel(const float *__restrict__ table, int P,
-                                       float *__restrict__ rowmax) {
-  const int t = blockIdx.x;
-  float m[3] = {0.0f, 0.0f, 0.0f};
-  for (int p = threadIdx.x; p < P; p += blockDim.x)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) m[d] = fmaxf(m[d], fabsf(table[((long long)t * P + p) * 3 + d]));
-  __shared__ float s_m[3][32];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    float v = m[d];
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) s_m[d][threadIdx.x >> 5] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    float v = 0.0f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = fmaxf(v, s_m[threadIdx.x][w]);
-    rowmax[t * 3 + threadIdx.x] = v;
-  }
-}
-
 __global__ void mc_cp_finish_kernel(const int *__restrict__ hits, const int *__restrict__ len,
                                     int n, int Pmc, int T_rows, float *__restrict__ cp,
                                     int *__restrict__ error) {
@@ -777,52 +800,45 @@ __global__ void mc_cp_finish_kernel(const int *__restrict__ hits, const int *__r
 
 }  // namespace
 
-pump_status_t particle_rowmax_async(const float *d_table, int P, int T, float *d_rowmax,
-                                    cudaStream_t stream) {
-  particle_rowmax_kernel<<<T, 256, 0, stream>>>(d_table, P, d_rowmax);
-  return launch_status("particle_rowmax");
-}
-
 pump_status_t mc_cp_hits_async(const float *d_paths, const int *d_offset, const int *d_len,
                                int n_paths, const float *d_offsets_t, int Pmc, int T_rows,
                                float offset_mult, const float *d_obstacles, int numObs,
-                               int *d_hits, cudaStream_t stream, const float *d_rowmax,
-                               const int *copy_src, int *copy_dst, int copy_words,
-                               unsigned int *done, unsigned int seq) {
+                               int *d_hits, cudaStream_t stream, const int *copy_src,
+                               int *copy_dst, int copy_words, unsigned int *done,
+                               unsigned int seq) {
   if (n_paths <= 0) return PUMP_OK;
   if (copy_dst && n_paths > 65535)
     return set_error(PUMP_ERR_BAD_INPUT, "mc_cp: copy-out with %d paths", n_paths);
-  if (numObs > kMcFilterObs) d_rowmax = nullptr;
-  size_t smem = sizeof(float) * (size_t)((numObs * 12 + 3) & ~3);
-  if (d_rowmax) smem += sizeof(uint32_t) * (kMcFilterObs / 32) * (size_t)T_rows;
-  if (smem > 200 * 1024) {
-    if (!d_rowmax) return set_error(PUMP_ERR_CAPACITY, "mc_cp: %d obstacles", numObs);
-    d_rowmax = nullptr;  // masks for this many rows do not fit: test every box
-    smem = sizeof(float) * (size_t)((numObs * 12 + 3) & ~3);
-    if (smem > 200 * 1024) return set_error(PUMP_ERR_CAPACITY, "mc_cp: %d obstacles", numObs);
-  }
-  PUMP_TRY(smem_attr((const void *)mc_cp_kernel, smem));
-  for (int k0 = 0; k0 < n_paths; k0 += 65535) {
-    const int nk = n_paths - k0 < 65535 ? n_paths - k0 : 65535;
-    dim3 grid(grid_for(Pmc, 32), (unsigned)nk);
-    mc_cp_kernel<<<grid, 32 * kMcWarps, smem, stream>>>(d_paths, d_offset, d_len, d_offsets_t, Pmc, T_rows,
-                                              offset_mult, d_obstacles, numObs, k0, d_hits,
-                                              d_rowmax, copy_src, copy_dst, copy_words, done,
-                                              seq);
-    PUMP_TRY(launch_status("mc_cp_kernel"));
-  }
-  return PUMP_OK;
+  const size_t smem = sizeof(float) * (size_t)((numObs * 12 + 3) & ~3);
+  if (smem > 200 * 1024) return set_error(PUMP_ERR_CAPACITY, "mc_cp: %d obstacles", numObs);
+  auto go = [&](auto per_lane) -> pump_status_t {
+    constexpr int K = decltype(per_lane)::value;
+    PUMP_TRY(smem_attr((const void *)mc_cp_kernel<K>, smem));
+    for (int k0 = 0; k0 < n_paths; k0 += 65535) {
+      const int nk = n_paths - k0 < 65535 ? n_paths - k0 : 65535;
+      dim3 grid(grid_for(Pmc, 32 * K), (unsigned)nk);
+      mc_cp_kernel<K><<<grid, 32 * kMcWarps, smem, stream>>>(
+          d_paths, d_offset, d_len, d_offsets_t, Pmc, T_rows, offset_mult, d_obstacles, numObs, k0,
+          d_hits, copy_src, copy_dst, copy_words, done, seq);
+      PUMP_TRY(launch_status("mc_cp_kernel"));
+    }
+    return PUMP_OK;
+  };
+  // particles per lane: four once that still leaves every SM two blocks
+  const long long blocks = (long long)n_paths * grid_for(Pmc, 32);
+  if (blocks >= 8LL * kNumSMs) return go(std::integral_constant<int, 4>{});
+  return go(std::integral_constant<int, 1>{});
 }
 
 pump_status_t mc_cp_async(const float *d_paths, const int *d_offset, const int *d_len, int n_paths,
                           const float *d_offsets_t, int Pmc, int T_rows, float offset_mult,
                           const float *d_obstacles, int numObs, int *d_hits, float *d_cp,
-                          int *d_error, cudaStream_t stream, const float *d_rowmax) {
+                          int *d_error, cudaStream_t stream) {
   if (n_paths <= 0) return PUMP_OK;
   PUMP_CUDA_TRY(cudaMemsetAsync(d_hits, 0, sizeof(int) * n_paths, stream));
   PUMP_TRY(mc_cp_hits_async(d_paths, d_offset, d_len, n_paths, d_offsets_t, Pmc, T_rows,
-                            offset_mult, d_obstacles, numObs, d_hits, stream, d_rowmax, nullptr,
-                            nullptr, 0, nullptr, 0u));
+                            offset_mult, d_obstacles, numObs, d_hits, stream, nullptr, nullptr, 0,
+                            nullptr, 0u));
   mc_cp_finish_kernel<<<grid_for(n_paths, 128), 128, 0, stream>>>(d_hits, d_len, n_paths, Pmc,
                                                                   T_rows, d_cp, d_error);
   return launch_status("mc_cp_finish_kernel");
@@ -1070,5 +1086,5 @@ extern "C" pump_status_t pump_mc_cp(const float *d_paths, const int *d_offset, c
       (n_paths > 0 && (!d_paths || !d_offset || !d_len || !d_offsets_t || !d_hits || !d_cp)))
     return set_error(PUMP_ERR_BAD_INPUT, "pump_mc_cp: bad arguments");
   return mc_cp_async(d_paths, d_offset, d_len, n_paths, d_offsets_t, Pmc, T_rows, offset_mult,
-                     d_obstacles, numObs, d_hits, d_cp, d_error, (cudaStream_t)stream, nullptr);
+                     d_obstacles, numObs, d_hits, d_cp, d_error, (cudaStream_t)stream);
 }

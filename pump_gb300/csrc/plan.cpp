@@ -52,7 +52,7 @@ pump_status_t hsmc_boxes_async(int num_new, int W, const int *d_edge, const int 
 pump_status_t mc_cp_async(const float *d_paths, const int *d_offset, const int *d_len, int n_paths,
                           const float *d_offsets_t, int Pmc, int T_rows, float offset_mult,
                           const float *d_obstacles, int numObs, int *d_hits, float *d_cp,
-                          int *d_error, cudaStream_t stream, const float *d_rowmax);
+                          int *d_error, cudaStream_t stream);
 
 namespace {
 
@@ -358,7 +358,6 @@ class Planner {
     return pb_.bvp_mode == PUMP_BVP_PARITY_GPU ? d_toptH_.p : d_toptE_.p;
   }
   const float *d_table_ = nullptr;   // context-cached particle table
-  const float *d_rowmax_ = nullptr;  // its largest |offset| per row and axis
   const float *obs_p_ = nullptr;    // device obstacles used by the MC CP
   DevBuf<uint8_t> d_free_s_, d_free_e_;
   DevBuf<int> d_open_cnt_;  // per node: expandable edges, -1 until checked
@@ -615,7 +614,6 @@ pump_status_t Planner::online() {
                      "%d boxes or %d waypoints x %d half-spaces exceed the HSMC shared-memory stage",
                      nobs_, W_, maxHS_);
   PUMP_TRY(ctx_->particle_table(pb_.seed, pb_.num_mc, pb_.table_rows, &d_table_, s_));
-  d_rowmax_ = d_table_ + 3 * (size_t)pb_.num_mc * pb_.table_rows;
   return PUMP_OK;
 }
 
@@ -1151,7 +1149,7 @@ pump_status_t Planner::eval_launch(CandSet &c, const std::vector<std::vector<flo
   if (with_cp)
     PUMP_TRY(mc_cp_hits_async(c.states.p, d_ints + 2 * n, cb.len, n, d_table_, pb_.num_mc,
                               pb_.table_rows, pb_.offset_mult, obs_p_, nobs_, cb.hits, s_,
-                              d_rowmax_, copy_out ? c.out.p : nullptr,
+                              copy_out ? c.out.p : nullptr,
                               copy_out ? reinterpret_cast<int *>(hout) : nullptr,
                               (int)head_words, cb.done, c.seq));
   if (!copy_out)
@@ -1404,10 +1402,6 @@ pump_status_t Planner::evaluate_paths(const std::vector<std::vector<float>> &xs,
   d_table_ = d_table;
   obs_p_ = d_obs;
   nobs_ = nobs;
-  DevBuf<float> d_rowmax;
-  PUMP_TRY(d_rowmax.alloc(3 * (size_t)pb_.table_rows));
-  PUMP_TRY(particle_rowmax_async(d_table, pb_.num_mc, pb_.table_rows, d_rowmax.p, s_));
-  d_rowmax_ = d_rowmax.p;
   std::vector<int> ln;
   std::vector<float> cs, cps;
   PUMP_TRY(eval_candidates(xs, dt_, pb_.table_rows, true, true, ln, cs, cps));

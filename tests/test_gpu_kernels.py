@@ -770,6 +770,42 @@ def test_mc_cp(gpu, pumplib, oracle, goldens):
             assert np.float32(host(cps)[k]) == np.float32(cp)
 
 
+@pytest.mark.parametrize("n_paths", [3, 60])
+@pytest.mark.parametrize("Pmc,boxes", [(1000, 0), (1000, 33), (2048, 32), (31, 130), (1, 5)])
+def test_mc_cp_box_filter(Pmc, boxes, n_paths, gpu, pumplib, oracle):
+    """The warp's common bounding box against boxes in groups of 32 (one group
+    and one box over it), particle counts with ragged warps and blocks, one
+    and four particles per lane (few and many paths), path lengths around the
+    16 warps' shares, and a NaN state."""
+    from pump_gb300 import workloads
+    torch, _ = gpu
+    L = pumplib.load()
+    T = 60
+    obs = workloads.random_boxes(boxes, 5) if boxes else np.zeros((0, 12), np.float32)
+    tm, pm = oracle.particle_tables(77, Pmc, T)
+    rng = np.random.default_rng(3)
+    lens = np.array([[2, 3, 17, 18, 19, 33, 35, 50, 60, 61][k % 10] for k in range(n_paths)], np.int32)
+    paths = []
+    for k, n in enumerate(lens):
+        a, b = rng.uniform(0, 1, 3), rng.uniform(0, 1, 3)
+        x = np.zeros((n, 6), np.float32)
+        x[:, :3] = a + (b - a) * np.linspace(0, 1, n)[:, None] + rng.normal(0, 0.01, (n, 3))
+        if k == 4:
+            x[n // 2, 1] = np.nan
+        paths.append(x)
+    offs = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int32)
+    hits, cps = empty(torch, n_paths, torch.int32), empty(torch, n_paths, torch.float32)
+    d_p, d_o, d_l = dev(torch, np.concatenate(paths)), dev(torch, offs), dev(torch, lens)
+    d_tm, d_obs = dev(torch, tm), dev(torch, obs if boxes else np.zeros((1, 12), np.float32))
+    for om in (np.float32(0.05), np.float32(0.5)):
+        pumplib.check(L.pump_mc_cp(ptr(d_p), ptr(d_o), ptr(d_l), n_paths, ptr(d_tm), Pmc, T, float(om),
+                                   ptr(d_obs), boxes, ptr(hits), ptr(cps), 0, stream(torch)))
+        torch.cuda.synchronize()
+        for k, x in enumerate(paths):
+            h = oracle.mccp(x, len(x), pm, om, obs)[0] if len(x) <= T else 0
+            assert int(host(hits)[k]) == h, (k, len(x))
+
+
 @pytest.mark.parametrize("N,density", [(0, 0.5), (1, 1.0), (4095, 0.3), (4096, 1.0), (100_000, 0.01),
                                        (1_000_000, 0.5), (777_777, 0.0)])
 def test_frontier_compact(N, density, gpu, pumplib):
