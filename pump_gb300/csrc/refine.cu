@@ -5,11 +5,11 @@
 //   1. segments: the optimal time tau_i (precise.cuh), the cost, the
 //      cost's partial derivatives and dtau/dx by the implicit function theorem;
 //   2. segment start times (warp scan of tau);
-//   3. waypoints: one warp per segment, its waypoints in order, lanes over the
-//      boxes (staged in shared memory); the bound's partial derivatives with
+//   3. waypoints: one warp per segment, lanes over its waypoints and boxes
+//      (staged in shared memory); the bound's partial derivatives with
 //      respect to each waypoint's position, velocity and noise scale are
-//      warp-reduced and pushed back to the segment's two nodes, its tau and
-//      its start time;
+//      pushed back to the segment's two nodes, its tau and its start time, and
+//      warp-reduced once per segment;
 //   4. start-time adjoints to earlier taus (suffix scan), taus to nodes.
 // Every sum runs in a fixed order (no floating-point atomics), so results
 // are the same from run to run.
@@ -31,6 +31,9 @@ constexpr int kRefThreads = 256;
 constexpr int kRefWarps = kRefThreads / 32;
 constexpr float kEpsV = 1e-12f;  // added to v.v (a waypoint at rest)
 constexpr float kEpsD = 1e-12f;  // added to a.a under the square root
+// From this many noise scales on, erfcf(z / sqrt 2) / 2 (2e-48) and
+// expf(-z^2 / 2) (5e-47) are below half of binary32's smallest value.
+constexpr float kZeroZ = 14.6f;
 
 enum Mode { kPlain = 0, kStep = 1, kAccept = 2 };
 
@@ -70,7 +73,7 @@ struct Basis {
 };
 
 template <bool Grad, int M>
-__global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a, Work w) {
+__global__ void __launch_bounds__(kRefThreads, Grad ? 3 : 4) refine_kernel(pump_refine_args a, Work w) {
   extern __shared__ float s_obs[];  // per box: lo[0..2], hi[0..2]
   __shared__ float s_tau[kMaxSeg], s_T0[kMaxSeg], s_taubar[kMaxSeg], s_Tbar[kMaxSeg];
   __shared__ float s_dtau[kMaxSeg * 12];  // dtau_i / d(x_i, x_{i+1})
@@ -184,8 +187,20 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
   }
   __syncthreads();
 
-  // 3. waypoints: warp per segment, its W waypoints in order, lanes over boxes
+  // 3. waypoints: warp per segment, its lanes split evenly over the waypoints
+  // (32 at a time; W = 8: four lanes each), each lane with its waypoint's state
+  // and every slots-th box.  A box kZeroZ or more noise scales away adds
+  // exactly zero to every sum (its tail probability and its density underflow
+  // in binary32), so only the others evaluate them; each lane adds its parts
+  // of the segment's adjoints, reduced once per segment.  Bound by instruction
+  // issue.  1024 paths, 40 boxes, noise 2e-3: 226 us with the lanes over the
+  // boxes of one waypoint at a time, every tail and density evaluated and
+  // seven reductions per waypoint; 74 us with the lanes over the (waypoint,
+  // box) pairs, the waypoints' states from shuffles; 56 us so.
   const float om = a.offset_mult, sf2 = a.sigma_floor * a.sigma_floor;
+  const int nobs = a.num_obstacles;
+  const int slots = a.W < 32 ? 32 / a.W : 1;
+  const int my_k = lane / slots, my_slot = lane - my_k * slots;
   float bsum = 0.0f;
   for (int i = warp; i < nseg; i += kRefWarps) {
     float x0[6], x1[6];
@@ -199,7 +214,10 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
 #pragma unroll
     for (int m = 0; m < 12; ++m) acc[m] = 0.0f;
     float tb_acc = 0.0f, Tb_acc = 0.0f;
-    for (int k = 0; k < a.W; ++k) {
+    bool any = false;
+    for (int k0 = 0; k0 < a.W; k0 += 32) {
+      const int k = k0 + my_k;
+      if (k >= a.W) continue;
       const float s = (float)k / (float)a.W;
       const Basis B(s);
       float p[3], v[3];
@@ -221,29 +239,29 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
       }
       const float S = om * sqrtf(V + sf2), invS = 1.0f / S;
       const float vv = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + kEpsV, ivv = 1.0f / vv;
-      float gp[3] = {0.0f, 0.0f, 0.0f}, gv[3] = {0.0f, 0.0f, 0.0f}, gS = 0.0f;
-      for (int o = lane; o < a.num_obstacles; o += 32) {
+      // distances squared from which z >= kZeroZ (1 % above); never outside the
+      // range where the square is a normal number (NaN and zero S included)
+      const float far2 = S > 1e-15f && S < 1e15f ? (1.01f * kZeroZ * kZeroZ) * (S * S) : INFINITY;
+      for (int o = my_slot; o < nobs; o += slots) {
         const float *bx = &s_obs[o * 6];
         float r[3];
-        bool inside[3];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const float lo = bx[d], hi = bx[3 + d];
-          r[d] = fminf(fmaxf(p[d], lo), hi) - p[d];
-          inside[d] = p[d] >= lo && p[d] <= hi;
-        }
+        for (int d = 0; d < 3; ++d) r[d] = fminf(fmaxf(p[d], bx[d]), bx[3 + d]) - p[d];
         const float beta = (r[0] * v[0] + r[1] * v[1] + r[2] * v[2]) * ivv;
         float av[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) av[d] = r[d] - beta * v[d];
-        const float dist = sqrtf(av[0] * av[0] + av[1] * av[1] + av[2] * av[2] + kEpsD);
+        const float dist2 = av[0] * av[0] + av[1] * av[1] + av[2] * av[2] + kEpsD;
+        if (dist2 >= far2 && dist2 < 1e30f) continue;
+        const float dist = sqrtf(dist2);
         const float z = dist * invS;
         bsum += 0.5f * erfcf(z * 0.70710678118654752f);
         if (Grad) {
+          any = true;
           const float zb = -0.39894228040143268f * expf(-0.5f * z * z);  // -phi(z)
-          gS -= zb * z * invS;
+          const float gS = -(zb * z * invS);
           const float sc = zb * invS / dist;
-          float abar[3];
+          float abar[3], gp[3], gv[3];
 #pragma unroll
           for (int d = 0; d < 3; ++d) abar[d] = sc * av[d];
           const float betabar = -(abar[0] * v[0] + abar[1] * v[1] + abar[2] * v[2]);
@@ -251,40 +269,42 @@ __global__ void __launch_bounds__(kRefThreads) refine_kernel(pump_refine_args a,
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             const float rbar = abar[d] + betabar * v[d] * ivv;
-            gv[d] += -beta * abar[d] + betabar * r[d] * ivv + 2.0f * vvbar * v[d];
-            if (!inside[d]) gp[d] -= rbar;
+            gv[d] = -beta * abar[d] + betabar * r[d] * ivv + 2.0f * vvbar * v[d];
+            const bool inside = p[d] >= bx[d] && p[d] <= bx[3 + d];
+            gp[d] = inside ? 0.0f : -rbar;
           }
-        }
-      }
-      if (Grad) {
-        // every lane ends with the same sums (xor butterfly)
+          // back to the segment's nodes, tau and start time
+          const float Tb = gS * om * om * 0.5f * invS * dVdT;  // dB/dS dS/dV dV/dT
+          const float gr = B.g0 * rt;
+          float tb = s * Tb;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          gp[d] = warp_sum(gp[d]) * lam;
-          gv[d] = warp_sum(gv[d]) * lam;
+          for (int d = 0; d < 3; ++d) {
+            acc[d] += B.h0 * gp[d] + gr * gv[d];
+            acc[6 + d] += B.h1 * gp[d] - gr * gv[d];
+            acc[3 + d] += t * B.h2 * gp[d] + B.g1 * gv[d];
+            acc[9 + d] += t * B.h3 * gp[d] + B.g2 * gv[d];
+            tb += (B.h2 * x0[3 + d] + B.h3 * x1[3 + d]) * gp[d];
+            tb -= B.g0 * (x0[d] - x1[d]) * rt * rt * gv[d];
+          }
+          tb_acc += tb;
+          Tb_acc += Tb;
         }
-        gS = warp_sum(gS) * lam;
-        const float Tb = gS * om * om * 0.5f * invS * dVdT;  // dB/dS dS/dV dV/dT
-        float tb = s * Tb;
-        const float gr = B.g0 * rt;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          acc[d] += B.h0 * gp[d] + gr * gv[d];
-          acc[6 + d] += B.h1 * gp[d] - gr * gv[d];
-          acc[3 + d] += t * B.h2 * gp[d] + B.g1 * gv[d];
-          acc[9 + d] += t * B.h3 * gp[d] + B.g2 * gv[d];
-          tb += (B.h2 * x0[3 + d] + B.h3 * x1[3 + d]) * gp[d];
-          tb -= B.g0 * (x0[d] - x1[d]) * rt * rt * gv[d];
-        }
-        tb_acc += tb;
-        Tb_acc += Tb;
       }
     }
-    if (Grad && lane == 0) {
+    __syncwarp();
+    if (Grad) {
+      if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-      for (int m = 0; m < 12; ++m) s_g[i * 12 + m] += acc[m];
-      s_taubar[i] = tb_acc;
-      s_Tbar[i] = Tb_acc;
+        for (int m = 0; m < 12; ++m) acc[m] = warp_sum(acc[m]) * lam;
+        tb_acc = warp_sum(tb_acc) * lam;
+        Tb_acc = warp_sum(Tb_acc) * lam;
+      }
+      if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < 12; ++m) s_g[i * 12 + m] += acc[m];
+        s_taubar[i] = tb_acc;
+        s_Tbar[i] = Tb_acc;
+      }
     }
   }
   bsum = warp_sum(bsum);

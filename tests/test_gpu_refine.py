@@ -108,6 +108,24 @@ def test_fwd_bwd_match_binary64(gpu, pumplib, oracle, om, seed):
         assert np.linalg.norm(gk - g64) <= REL_G * np.linalg.norm(g64) + cond[3]
 
 
+@pytest.mark.parametrize("W,boxes,om", [(1, 1, 0.3), (33, 31, 0.05), (64, 33, 0.3), (7, 40, 0.3), (5, 0, 0.3)])
+def test_pairs_over_lanes(gpu, pumplib, oracle, W, boxes, om):
+    """Waypoint counts past one warp's 32 and ones that do not divide it, box
+    counts that leave some of a waypoint's lanes idle; no box at all."""
+    torch, _ = gpu
+    case = Case(torch, pumplib, oracle, 6, 11, om, W=W, n_range=(3, 9))
+    case.obs = case.obs[:boxes]
+    case.args.num_obstacles = boxes
+    case.R = oracle.Refine(case.obs, om, W=W, tmax=case.tmax, T_rows=case.T_rows)
+    g, J = bwd(torch, pumplib, case)
+    for k in range(case.args.n_paths):
+        X, lam = case.path(k).astype(np.float64), float(case.lam[k])
+        J64, g64 = case.R.grad(X, lam)
+        cond = 4 * case.conditioning(X, lam)
+        assert abs(J[k] - J64) <= REL_J * abs(J64) + cond[0]
+        assert np.linalg.norm(case.path(k, g) - g64) <= REL_G * np.linalg.norm(g64) + cond[3]
+
+
 def test_clamped_segments(gpu, pumplib, oracle):
     torch, _ = gpu
     case = Case(torch, pumplib, oracle, 16, 7, 0.3, tmax=0.3, n_range=(5, 8))
