@@ -179,10 +179,66 @@ __global__ void __launch_bounds__(128) bvp_batch_kernel(const JobPairs src) {
 // edges (T x W x 6 floats, contiguous in disc) are assembled in shared
 // memory and stored as whole lines, so the kernel's DRAM traffic is the
 // waypoint records it writes.  The block size T (64, 128, 256) is picked by
-// the autotuner.
+// the autotuner.  The bit-exact arithmetics are bound by instruction issue
+// (the 799,800 edges of the N = 4000 query: 524 us with every uncertified
+// waypoint's six states in binary64 by its own lane, 125 us now).
 template <int T>
 size_t discretize_smem(int numDisc) {
   return sizeof(float) * (size_t)T * (numDisc + 1) * kDim;
+}
+
+// The interior waypoints of one thread's edge in the bit-exact arithmetics,
+// written to o (numDisc + 1 records): float-float states, the uncertified ones
+// queued for finish_path_queue.
+template <int Cap>
+__device__ __forceinline__ void edge_waypoints_ff(float tau, const float *x0, const float *x1,
+                                                  int numDisc, float *o, PathQueue<Cap> &queue) {
+  const float dt = tau / numDisc;
+  const PathFF pe = path_ff_edge(tau, x0, x1);
+  const float *s_end = o;  // records 0 and numDisc hold the end states
+  for (int i = 1; i < numDisc; ++i) {
+    float x[kDim];
+    unsigned bad = path_point_try(dt * i, tau, x0, x1, pe, x);
+#pragma unroll
+    for (int d = 0; d < kDim; ++d) o[i * kDim + d] = x[d];
+    while (bad) {
+      const int d = __ffs(bad) - 1;
+      bad &= bad - 1u;
+      if (!queue.push(threadIdx.x, i, d)) {
+        const float *s0 = s_end + (d < 3 ? d : d - 3);
+        o[i * kDim + d] = path_state_now(d, dt * i, tau, s0[0], s0[3], s0[numDisc * kDim],
+                                        s0[numDisc * kDim + 3]);
+      }
+    }
+  }
+}
+// The queued states of a block, 32 of a kind per warp; call after a barrier.
+// item(th, &tau, &numDisc, &x0, &x1, &o): thread th's edge.
+template <int Cap, class Item>
+__device__ __forceinline__ void finish_path_queue(const PathQueue<Cap> &queue, Item item) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  int task = 0;
+  auto run = [&](auto kind) {
+    constexpr int Kind = decltype(kind)::value;
+    const int n = queue.n[Kind] < Cap ? queue.n[Kind] : Cap;
+    for (int q0 = 0; q0 < n; q0 += 32, ++task) {
+      if (task % warps != warp || q0 + lane >= n) continue;
+      const unsigned ent = queue.e[Kind][q0 + lane];
+      const int th = (int)(ent >> 20), i = (int)((ent >> 2) & 0x3ffffu), a = (int)(ent & 3u);
+      float tau;
+      int numDisc;
+      const float *x0, *x1;
+      float *o;
+      item(th, &tau, &numDisc, &x0, &x1, &o);
+      const float dt = tau / numDisc;
+      o[i * kDim + a + (Kind == kPathXY || Kind == kPathZ ? 0 : 3)] = path_state64<Kind>(
+          dt * i, tau, __ldg(x0 + a), __ldg(x0 + a + 3), __ldg(x1 + a), __ldg(x1 + a + 3));
+    }
+  };
+  run(std::integral_constant<int, kPathXY>{});
+  run(std::integral_constant<int, kPathVXY>{});
+  run(std::integral_constant<int, kPathZ>{});
+  run(std::integral_constant<int, kPathVZ>{});
 }
 
 template <int Mode, int T>
@@ -191,9 +247,14 @@ __global__ void __launch_bounds__(T) discretize_kernel(
     const float *__restrict__ toptE, long long E, int numDisc, float *__restrict__ disc) {
   extern __shared__ float4 s_dyn4[];
   float *s_out = reinterpret_cast<float *>(s_dyn4);
+  __shared__ PathQueue<Mode != PUMP_BVP_PRECISION ? T : 1> s_queue;
   const int W = numDisc + 1;
   const long long e0 = blockIdx.x * (long long)T;
   const int nv = (int)(E - e0 < T ? E - e0 : T);
+  if (Mode != PUMP_BVP_PRECISION) {
+    s_queue.clear();
+    __syncthreads();
+  }
   if (threadIdx.x < nv) {
     const long long e = e0 + threadIdx.x;
     const int a = src[e], b = dst[e];
@@ -213,30 +274,7 @@ __global__ void __launch_bounds__(T) discretize_kernel(
     const float tau = topt;
     const float dt = tau / numDisc;
     if (Mode != PUMP_BVP_PRECISION) {
-      // float-float waypoints; the uncertified ones (a few in a hundred) in
-      // binary64 afterwards, each lane taking its next one per round, so a
-      // warp runs the binary64 evaluation about once instead of once per
-      // waypoint index where some lane needs it
-      const PathFF pe = path_ff_edge(tau, x0, x1);
-      unsigned int redo = 0u;  // waypoints i < 32 left for binary64
-      for (int i = 1; i < numDisc; ++i) {
-        if (!path_point_try(dt * i, tau, x0, x1, pe, x)) {
-          if (i < 32) {
-            redo |= 1u << i;
-            continue;
-          }
-          path_point(dt * i, tau, x0, x1, x);
-        }
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) o[i * kDim + d] = x[d];
-      }
-      while (redo) {
-        const int i = __ffs(redo) - 1;
-        redo &= redo - 1u;
-        path_point(dt * i, tau, x0, x1, x);
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) o[i * kDim + d] = x[d];
-      }
+      edge_waypoints_ff(tau, x0, x1, numDisc, o, s_queue);
     } else {
       for (int i = 1; i < numDisc; ++i) {
         path_point_f32(dt * i, tau, x0, x1, x);
@@ -246,6 +284,16 @@ __global__ void __launch_bounds__(T) discretize_kernel(
     }
   }
   __syncthreads();
+  if (Mode != PUMP_BVP_PRECISION) {
+    finish_path_queue(s_queue, [&](int th, float *tau, int *nd, const float **x0, const float **x1, float **o) {
+      *tau = toptE[e0 + th];
+      *nd = numDisc;
+      *x0 = samples + src[e0 + th] * kDim;
+      *x1 = samples + dst[e0 + th] * kDim;
+      *o = s_out + th * W * kDim;
+    });
+    __syncthreads();
+  }
   block_store(disc + e0 * W * kDim, s_out, nv * W * kDim);
 }
 
@@ -381,6 +429,8 @@ __global__ void __launch_bounds__(T) discretize_off_kernel(
     float *__restrict__ disc, int *error) {
   extern __shared__ float4 s_dyn4[];
   float *s_out = reinterpret_cast<float *>(s_dyn4);
+  __shared__ PathQueue<Mode != PUMP_BVP_PRECISION ? T : 1> s_queue;
+  if (Mode != PUMP_BVP_PRECISION) s_queue.clear();  // (a barrier follows)
   const long long e0 = blockIdx.x * (long long)T;
   const int nv = (int)(E - e0 < T ? E - e0 : T);
   const long long base = off[e0];
@@ -408,30 +458,7 @@ __global__ void __launch_bounds__(T) discretize_off_kernel(
     const float tau = toptE[e];
     const float dt = tau / numDisc;
     if (Mode != PUMP_BVP_PRECISION) {
-      // float-float waypoints; the uncertified ones (a few in a hundred) in
-      // binary64 afterwards, each lane taking its next one per round, so a
-      // warp runs the binary64 evaluation about once instead of once per
-      // waypoint index where some lane needs it
-      const PathFF pe = path_ff_edge(tau, x0, x1);
-      unsigned int redo = 0u;  // waypoints i < 32 left for binary64
-      for (int i = 1; i < numDisc; ++i) {
-        if (!path_point_try(dt * i, tau, x0, x1, pe, x)) {
-          if (i < 32) {
-            redo |= 1u << i;
-            continue;
-          }
-          path_point(dt * i, tau, x0, x1, x);
-        }
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) o[i * kDim + d] = x[d];
-      }
-      while (redo) {
-        const int i = __ffs(redo) - 1;
-        redo &= redo - 1u;
-        path_point(dt * i, tau, x0, x1, x);
-#pragma unroll
-        for (int d = 0; d < kDim; ++d) o[i * kDim + d] = x[d];
-      }
+      edge_waypoints_ff(tau, x0, x1, numDisc, o, s_queue);
     } else {
       for (int i = 1; i < numDisc; ++i) {
         path_point_f32(dt * i, tau, x0, x1, x);
@@ -441,6 +468,16 @@ __global__ void __launch_bounds__(T) discretize_off_kernel(
     }
   }
   __syncthreads();
+  if (Mode != PUMP_BVP_PRECISION) {
+    finish_path_queue(s_queue, [&](int th, float *tau, int *nd, const float **x0, const float **x1, float **o) {
+      *tau = toptE[e0 + th];
+      *nd = (int)(off[e0 + th + 1] - off[e0 + th]) - 1;
+      *x0 = samples + src[e0 + th] * kDim;
+      *x1 = samples + dst[e0 + th] * kDim;
+      *o = s_out + (off[e0 + th] - base) * kDim;
+    });
+    __syncthreads();
+  }
   block_store(disc + base * kDim, s_out, (int)(off[e0 + nv] - base) * kDim);
 }
 

@@ -8,90 +8,107 @@
 #include "ffcost.cuh"
 
 namespace pump {
+namespace {
 
-// pathPoint, 2pBVP.cu:117-131, in the expression's own evaluation types.
-__device__ __forceinline__ void path_point(float t, float tau, const float *x0, const float *x1,
-                                           float *x) {
+// pathPoint, 2pBVP.cu:117-131, in the expression's own evaluation types, by
+// kind of state: the x and y positions, their velocities, the z position and
+// its velocity each have their own expression, over one axis's end states (p0,
+// v0) and (p1, v1).
+enum PathKind { kPathXY = 0, kPathVXY, kPathZ, kPathVZ, kPathKinds };
+template <int Kind>
+__device__ __forceinline__ float path_state64(float t, float tau, float p0, float v0, float p1, float v1) {
   const double t2 = p2f(t), t3 = p3f(t), u2 = p2f(tau), u3 = p3f(tau);
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int a = k, b = k + 3;
-    double r = (double)(t * x0[b] + x0[a]);
-    r = r + (t3 * (double)(2 * x0[a] - 2 * x1[a] + (x0[b] + x1[b]) * tau)) / u3;
-    r = r - (t2 * (double)(3 * x0[a] - 3 * x1[a] + (2 * x0[b] + x1[b]) * tau)) / u2;
-    x[k] = (float)r;
+  if (Kind == kPathXY) {
+    double r = (double)(t * v0 + p0);
+    r = r + (t3 * (double)(2 * p0 - 2 * p1 + (v0 + v1) * tau)) / u3;
+    r = r - (t2 * (double)(3 * p0 - 3 * p1 + (2 * v0 + v1) * tau)) / u2;
+    return (float)r;
   }
-  {
-    double r = (double)(t * x0[5]) * u3 + (double)x0[2] * u3;
-    double q1 = -3. * x0[2] + 3. * x1[2] - 2. * x0[5] * tau - 1. * x1[5] * tau;
-    r = r + (t2 * (double)tau) * q1;
-    double q2 = 2. * x0[2] - 2. * x1[2] + (double)((x0[5] + x1[5]) * tau);
-    r = r + t3 * q2;
-    x[2] = (float)(r / u3);
-  }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int a = k, b = k + 3;
-    float f1 = -(2 * t * (3 * x0[a] - 3 * x1[a] + x1[b] * tau));
+  if (Kind == kPathVXY) {
+    float f1 = -(2 * t * (3 * p0 - 3 * p1 + v1 * tau));
     double r = (double)f1 / u2;
-    r = r + (3 * t2 * (double)(2 * x0[a] - 2 * x1[a] + x1[b] * tau)) / u3;
+    r = r + (3 * t2 * (double)(2 * p0 - 2 * p1 + v1 * tau)) / u3;
     double inner = 3 * t2 - (double)(4 * t * tau) + u2;
-    r = r + ((double)x0[b] * inner) / u2;
-    x[3 + k] = (float)r;
+    r = r + ((double)v0 * inner) / u2;
+    return (float)r;
   }
-  {
-    double r = (double)x0[5] * u3;
-    double q1 = -6. * x0[2] + 6. * x1[2] - 4. * x0[5] * tau - 2. * x1[5] * tau;
-    r = r + (double)(t * tau) * q1;
-    double q2 = 6. * x0[2] - 6. * x1[2] + 3. * x0[5] * tau + 3. * x1[5] * tau;
-    r = r + t2 * q2;
-    x[5] = (float)(r / u3);
+  if (Kind == kPathZ) {
+    double r = (double)(t * v0) * u3 + (double)p0 * u3;
+    double q1 = -3. * p0 + 3. * p1 - 2. * v0 * tau - 1. * v1 * tau;
+    r = r + (t2 * (double)tau) * q1;
+    double q2 = 2. * p0 - 2. * p1 + (double)((v0 + v1) * tau);
+    r = r + t3 * q2;
+    return (float)(r / u3);
   }
+  double r = (double)v0 * u3;
+  double q1 = -6. * p0 + 6. * p1 - 4. * v0 * tau - 2. * v1 * tau;
+  r = r + (double)(t * tau) * q1;
+  double q2 = 6. * p0 - 6. * p1 + 3. * v0 * tau + 3. * v1 * tau;
+  r = r + t2 * q2;
+  return (float)(r / u3);
 }
 
-// path_point's binary32 results from float-float arithmetic (ffcost.cuh's
-// operations), certified as in cost_ff: each state is the sum of a few terms
-// (the position x0 + ... as A + t^3 X / tau^3 - t^2 Y / tau^2, with A, X and
-// Y the binary32 values path_point converts), evaluated exactly enough in
-// float-float; path_point's binary64 value differs from the exact sum of
-// those terms by its roundings (at most 16 of them, each within 2^-53 of a
-// partial result no larger than M, the sum of the terms' magnitudes, tau^3
-// and t^3 included: 2^-49 M), and the float-float value by at most about
-// 37 u^2 M = 2^-42.8 M (u = 2^-24; with the double-word error bounds of
-// Joldes, Muller and Popescu, 2017: 1.5 u^2 per product by a binary32,
-// 6 u^2 per product, 15 u^2 per quotient, 3 u^2 per sum, 25 to 28 u^2 for a
-// term, 9 u^2 for the three sums).
-// When the interval of half-width 2^-41 M around the float-float value lies
-// inside the binary32 rounding cell of its high part, that is path_point's
-// (float) conversion; otherwise (or for tau outside [2^-20, 2^20], values
-// outside [2^-40, 2^60] and non-finite values) path_point runs.  The
-// per-edge terms (path_ff_edge) are shared by the edge's waypoints.
+// State d (0 .. 5), out of line: evaluated in place, the compiler runs the
+// binary64 code ahead of the test that asks for it, which took six times the
+// rest of the waypoint kernel's time.
+__device__ __noinline__ float path_state_now(int d, float t, float tau, float p0, float v0, float p1,
+                                             float v1) {
+  if (d < 2) return path_state64<kPathXY>(t, tau, p0, v0, p1, v1);
+  if (d == 2) return path_state64<kPathZ>(t, tau, p0, v0, p1, v1);
+  if (d < 5) return path_state64<kPathVXY>(t, tau, p0, v0, p1, v1);
+  return path_state64<kPathVZ>(t, tau, p0, v0, p1, v1);
+}
+
+// The binary32 results of path_state64 from float-float arithmetic
+// (ffcost.cuh's operations), certified as in cost_ff: with r = t / tau each
+// state is the sum of a few terms (a position x0 + ... as A + X r^3 - Y r^2,
+// with A, X and Y the binary32 values the expression converts), evaluated
+// exactly enough in float-float.  The binary64 value differs from the exact sum
+// of those terms by its roundings (at most 16 of them, each within 2^-53 of a
+// partial result no larger than M, the sum of the terms' magnitudes, tau^3 and
+// t^3 included: 2^-49 M).  The float-float value: 1 / tau from a reciprocal
+// estimate and one residual to 7 u^2 (u = 2^-24), products by a binary32 value
+// 3 u^2 and by a float-float one 6 u^2, so r, r^2 and r^3 to 10, 26 and 42 u^2,
+// the edge's sums to 9 u^2 and the terms to at most 54 u^2; a sum of n terms
+// (their high parts by TwoSum, the errors and low parts in binary32) adds at
+// most 16 u^2: at most 70 u^2 M = 2^-41.9 M.  When the interval of half-width
+// 2^-41 M around the float-float value lies inside the binary32 rounding cell
+// of its high part, that is the expression's (float) conversion; otherwise (or
+// for tau outside [2^-20, 2^20], values outside [2^-40, 2^60] and non-finite
+// values) path_state64 gives it.  The per-edge terms (path_ff_edge) are shared
+// by the edge's waypoints.
 struct PathFF {
-  bool ok;                           // tau in range: the float-float path applies
-  FF u2, ru2, ru3;                   // tau^2 (exact), 1 / tau^2, 1 / tau^3
-  float X[2], Y[2], inner[2], Z[2];  // path_point's binary32 edge terms
-  FF q1, q2, q1v, q2v;               // its binary64 edge sums, exactly
-  float mq1, mq2, mq1v, mq2v;        // their terms' magnitudes
+  bool ok;                        // tau in range: the float-float values apply
+  FF rt, ru2;                     // 1 / tau, 1 / tau^2
+  float X[2], Y[2], inner[2];     // the expressions' binary32 edge terms
+  FF Z[2];                        // 3 Z / tau, Z the binary32 edge term
+  FF q1, q2, c1, c2;              // z's edge sums; its velocity's, over tau^3 and tau
+  float mq1, mq2, mc1, mc2;       // their terms' magnitudes
 };
 
-__device__ __forceinline__ FF ff_neg(FF x) { return {-x.hi, -x.lo}; }
+// Sum of a binary32 value and float-float terms.
+__device__ __forceinline__ FF ff_sum(float a, FF x, FF y) {
+  const FF s = ff_two_sum(a, x.hi);
+  const FF t = ff_two_sum(s.hi, y.hi);
+  return ff_fast_two_sum(t.hi, (s.lo + t.lo) + (x.lo + y.lo));
+}
 
 __device__ __forceinline__ PathFF path_ff_edge(float tau, const float *x0, const float *x1) {
   PathFF e;
   e.ok = tau >= 0x1p-20f && tau <= 0x1p20f;
-  e.u2 = ff_two_prod(tau, tau);
-  const FF u3 = ff_mul_f(e.u2, tau);
-  const FF one = {1.0f, 0.0f};
-  e.ru2 = ff_div(one, e.u2);
-  e.ru3 = ff_div(one, u3);
+  const float r = ff_rcp(tau);
+  e.rt = ff_fast_two_sum(r, r * fmaf(-tau, r, 1.0f));
+  e.ru2 = ff_mul(e.rt, e.rt);
+  const FF ru3 = ff_mul(e.ru2, e.rt);
+  const FF rt3 = ff_mul_f(e.rt, 3.0f);
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int a = k, b = k + 3;
-    // the same binary32 expressions as path_point
+    // the same binary32 expressions as path_state64
     e.X[k] = 2 * x0[a] - 2 * x1[a] + (x0[b] + x1[b]) * tau;
     e.Y[k] = 3 * x0[a] - 3 * x1[a] + (2 * x0[b] + x1[b]) * tau;
     e.inner[k] = 3 * x0[a] - 3 * x1[a] + x1[b] * tau;
-    e.Z[k] = 2 * x0[a] - 2 * x1[a] + x1[b] * tau;
+    e.Z[k] = ff_mul_f(rt3, 2 * x0[a] - 2 * x1[a] + x1[b] * tau);
   }
   // -3 x0z + 3 x1z - 2 x0vz tau - x1vz tau (each term exact in binary64)
   {
@@ -111,15 +128,15 @@ __device__ __forceinline__ PathFF path_ff_edge(float tau, const float *x0, const
   {
     const FF a = ff_two_prod(x0[2], -6.0f), b = ff_two_prod(x1[2], 6.0f);
     const FF c = ff_two_prod(4.0f * x0[5], -tau), d = ff_two_prod(2.0f * x1[5], -tau);
-    e.q1v = ff_add(ff_add(ff_add(a, b), c), d);
-    e.mq1v = fabsf(a.hi) + fabsf(b.hi) + fabsf(c.hi) + fabsf(d.hi);
+    e.c1 = ff_mul(ff_add(ff_add(ff_add(a, b), c), d), ru3);
+    e.mc1 = (fabsf(a.hi) + fabsf(b.hi) + fabsf(c.hi) + fabsf(d.hi)) * ru3.hi;
   }
   // 6 x0z - 6 x1z + 3 x0vz tau + 3 x1vz tau
   {
     const FF a = ff_two_prod(x0[2], 6.0f), b = ff_two_prod(x1[2], -6.0f);
     const FF c = ff_mul_f(ff_two_prod(x0[5], tau), 3.0f), d = ff_mul_f(ff_two_prod(x1[5], tau), 3.0f);
-    e.q2v = ff_add(ff_add(ff_add(a, b), c), d);
-    e.mq2v = fabsf(a.hi) + fabsf(b.hi) + fabsf(c.hi) + fabsf(d.hi);
+    e.c2 = ff_mul(ff_add(ff_add(ff_add(a, b), c), d), e.rt);
+    e.mc2 = (fabsf(a.hi) + fabsf(b.hi) + fabsf(c.hi) + fabsf(d.hi)) * e.rt.hi;
   }
   return e;
 }
@@ -141,74 +158,93 @@ __device__ __forceinline__ bool ff_certify(FF v, float M, float *out) {
   return a + B < up && B - a < down;
 }
 
-// x = path_point's values when every state is certified (true); false
-// leaves x unspecified.
-__device__ __forceinline__ bool path_point_try(float t, float tau, const float *x0,
-                                               const float *x1, const PathFF &e, float *x) {
-  bool ok = e.ok;
-  const FF t2 = ff_two_prod(t, t);
-  const FF t3 = ff_mul_f(t2, t);
-  float v[kDim];
+// The certified states of x; returns a bit per state that is not (its x is
+// then unspecified).
+__device__ __forceinline__ unsigned path_point_try(float t, float tau, const float *x0,
+                                                   const float *x1, const PathFF &e, float *x) {
+  const FF r = ff_mul_f(e.rt, t);
+  const FF r2 = ff_mul(r, r);
+  const FF r3 = ff_mul(r2, r);
+  unsigned bad = 0u;
+  // the velocities' 1 - (4 t tau) / tau^2 + 3 r^2, the binary32 product rounded
+  const FF r2x3 = ff_mul_f(r2, 3.0f);
+  const FF F = ff_mul_f(e.ru2, -(4 * t * tau));
+  const FF in = ff_sum(1.0f, F, r2x3);
+  const float min = 1.0f + (fabsf(F.hi) + r2x3.hi);
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     const int a = k, b = k + 3;
-    // position: A + t^3 X / tau^3 - t^2 Y / tau^2
+    // position: A + X r^3 - Y r^2
     const float A = t * x0[b] + x0[a];
-    const FF T1 = ff_mul(ff_mul_f(t3, e.X[k]), e.ru3);
-    const FF T2 = ff_mul(ff_mul_f(t2, e.Y[k]), e.ru2);
-    const FF V = ff_add(ff_add_f(T1, A), ff_neg(T2));
-    ok = ff_certify(V, fabsf(A) + fabsf(T1.hi) + fabsf(T2.hi), &v[k]) && ok;
-    // velocity: f1 / tau^2 + 3 t^2 Z / tau^3 + x0v (3 t^2 - F + tau^2) / tau^2
+    const FF T1 = ff_mul_f(r3, e.X[k]), T2 = ff_mul_f(r2, -e.Y[k]);
+    if (!ff_certify(ff_sum(A, T1, T2), fabsf(A) + fabsf(T1.hi) + fabsf(T2.hi), &x[k])) bad |= 1u << k;
+    // velocity: f1 / tau^2 + r^2 3 Z / tau + x0v (1 - F / tau^2 + 3 r^2)
     const float f1 = -(2 * t * e.inner[k]);
-    const float F = 4 * t * tau;
-    const FF t2x3 = ff_mul_f(t2, 3.0f);
     const FF S1 = ff_mul_f(e.ru2, f1);
-    const FF S2 = ff_mul(ff_mul_f(t2x3, e.Z[k]), e.ru3);
-    const FF in = ff_add(ff_add_f(t2x3, -F), e.u2);
-    const FF S3 = ff_mul(ff_mul_f(in, x0[b]), e.ru2);
-    const FF W = ff_add(ff_add(S1, S2), S3);
-    const float MW = fabsf(S1.hi) + fabsf(S2.hi) +
-                     fabsf(x0[b]) * ((t2x3.hi + fabsf(F)) + e.u2.hi) * e.ru2.hi;
-    ok = ff_certify(W, MW, &v[3 + k]) && ok;
+    const FF S2 = ff_mul(r2, e.Z[k]);
+    const FF S3 = ff_mul_f(in, x0[b]);
+    const FF s = ff_two_sum(S1.hi, S2.hi);
+    const FF u = ff_two_sum(s.hi, S3.hi);
+    const FF W = ff_fast_two_sum(u.hi, (s.lo + u.lo) + ((S1.lo + S2.lo) + S3.lo));
+    if (!ff_certify(W, fabsf(S1.hi) + fabsf(S2.hi) + fabsf(x0[b]) * min, &x[3 + k])) bad |= 1u << (3 + k);
   }
   {
-    // z: t x0vz + x0z + t^2 q1 / tau^2 + t^3 q2 / tau^3
+    // z: t x0vz + x0z + r^2 q1 + r^3 q2
     const float P = t * x0[5];
-    const FF T1 = ff_mul(ff_mul(t2, e.q1), e.ru2);
-    const FF T2 = ff_mul(ff_mul(t3, e.q2), e.ru3);
-    const FF V = ff_add(ff_add(ff_two_sum(P, x0[2]), T1), T2);
-    const float M = fabsf(P) + fabsf(x0[2]) + t2.hi * e.ru2.hi * e.mq1 + t3.hi * e.ru3.hi * e.mq2;
-    ok = ff_certify(V, M, &v[2]) && ok;
+    const FF T1 = ff_mul(r2, e.q1), T2 = ff_mul(r3, e.q2);
+    const FF A = ff_two_sum(P, x0[2]);
+    const FF s = ff_two_sum(A.hi, T1.hi);
+    const FF u = ff_two_sum(s.hi, T2.hi);
+    const FF V = ff_fast_two_sum(u.hi, ((A.lo + s.lo) + u.lo) + (T1.lo + T2.lo));
+    const float M = fabsf(P) + fabsf(x0[2]) + r2.hi * e.mq1 + fabsf(r3.hi) * e.mq2;
+    if (!ff_certify(V, M, &x[2])) bad |= 1u << 2;
   }
   {
-    // vz: x0vz + (t tau) q1v / tau^3 + t^2 q2v / tau^3
+    // vz: x0vz + (t tau) c1 + r^2 c2
     const float tt = t * tau;
-    const FF T1 = ff_mul(ff_mul_f(e.q1v, tt), e.ru3);
-    const FF T2 = ff_mul(ff_mul(t2, e.q2v), e.ru3);
-    const FF V = ff_add(ff_add_f(T1, x0[5]), T2);
-    const float M = fabsf(x0[5]) + (fabsf(tt) * e.mq1v + t2.hi * e.mq2v) * e.ru3.hi;
-    ok = ff_certify(V, M, &v[5]) && ok;
+    const FF T1 = ff_mul_f(e.c1, tt), T2 = ff_mul(r2, e.c2);
+    const float M = fabsf(x0[5]) + fabsf(tt) * e.mc1 + r2.hi * e.mc2;
+    if (!ff_certify(ff_sum(x0[5], T1, T2), M, &x[5])) bad |= 1u << 5;
   }
-#pragma unroll
-  for (int d = 0; d < kDim; ++d) x[d] = v[d];
-  return ok;
+  return e.ok ? bad : 0x3fu;
 }
 
-// path_point_try, else path_point; certified (when given): whether the
-// float-float values were used.
-__device__ __forceinline__ void path_point_ff(float t, float tau, const float *x0, const float *x1,
-                                              const PathFF &e, float *x,
-                                              bool *certified = nullptr) {
-  const bool ok = path_point_try(t, tau, x0, x1, e, x);
-  if (certified) *certified = ok;
-  if (!ok) path_point(t, tau, x0, x1, x);
-}
-
-// path_point through path_point_ff, the edge terms computed here.
+// pathPoint's values: certified, the remaining states in binary64.
 __device__ __forceinline__ void path_point_fast(float t, float tau, const float *x0,
                                                 const float *x1, float *x) {
-  path_point_ff(t, tau, x0, x1, path_ff_edge(tau, x0, x1), x);
+  const unsigned bad = path_point_try(t, tau, x0, x1, path_ff_edge(tau, x0, x1), x);
+  if (bad) {
+#pragma unroll
+    for (int d = 0; d < kDim; ++d) {
+      const int a = d < 3 ? d : d - 3;
+      if ((bad >> d) & 1u) x[d] = path_state_now(d, t, tau, x0[a], x0[a + 3], x1[a], x1[a + 3]);
+    }
+  }
 }
+
+// The waypoint kernels' queue of states left for binary64, shared by a block:
+// (thread, waypoint, axis) entries in one list per kind, so that a warp then
+// evaluates 32 of one kind at once (binary64 instructions occupy this GPU's
+// binary64 pipe for the same time for one lane as for 32; one state in about
+// 200 is left, and evaluating each lane's own as they came took most of the
+// kernel's time).  A full list returns false: the thread evaluates it itself.
+template <int Cap>
+struct PathQueue {
+  int n[kPathKinds];
+  unsigned e[kPathKinds][Cap];
+  __device__ __forceinline__ void clear() {
+    if (threadIdx.x < kPathKinds) n[threadIdx.x] = 0;
+  }
+  // state d (0 .. 5) of waypoint i of thread th's edge
+  __device__ __forceinline__ bool push(int th, int i, int d) {
+    const int axis = d < 3 ? d : d - 3;
+    const int kind = (axis == 2 ? kPathZ : kPathXY) + (d < 3 ? 0 : 1);
+    const int at = atomicAdd(&n[kind], 1);
+    if (at >= Cap) return false;
+    e[kind][at] = ((unsigned)th << 20) | ((unsigned)i << 2) | (unsigned)axis;
+    return true;
+  }
+};
 
 // The same trajectory as path_point (cubic position, quadratic velocity,
 // no gravity term) in binary32 Hermite form with s = t / tau; used by the
@@ -228,4 +264,5 @@ __device__ __forceinline__ void path_point_f32(float t, float tau, const float *
   }
 }
 
+}  // namespace
 }  // namespace pump

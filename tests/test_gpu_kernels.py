@@ -305,6 +305,41 @@ def test_waypoints_gpu_arithmetic_mode(gpu, pumplib, roadmap1000):
     assert same_bits(a[0], b[0]) and same_bits(a[1], b[1]) and same_bits(a[0], a[1])
 
 
+@pytest.mark.parametrize("numDisc", [1, 2, 8, 33])
+def test_waypoints_left_for_binary64(numDisc, gpu, pumplib, oracle):
+    """Waypoints whose states the float-float bounds leave for binary64: dyadic
+    times (many states fall on a rounding boundary), and times out of the
+    float-float range, whose every state overflows a block's lists.  Bit for
+    bit with the reference's expression, in both layouts; 150 edges leave a
+    ragged last block."""
+    torch, _ = gpu
+    L = pumplib.load()
+    rng = np.random.default_rng(29)
+    N, E = 40, 150
+    s = np.concatenate([rng.uniform(0, 1, (N, 3)), rng.uniform(-1, 1, (N, 3))], 1).astype(np.float32)
+    src, dst = rng.integers(0, N, E).astype(np.int32), rng.integers(0, N, E).astype(np.int32)
+    tau = np.array([1.0, 0.5, 0.371, 2.0 ** -21, 3e6, 0.25], np.float32)[np.arange(E) % 6]
+    tau[64:128] = np.float32(2.0 ** -21)
+    W = numDisc + 1
+    want = np.zeros((E, W, 6), np.float32)
+    x = np.zeros(6, np.float32)
+    for e in range(E):
+        dt = np.float32(tau[e] / np.float32(numDisc))
+        want[e, 0], want[e, numDisc] = s[src[e]], s[dst[e]]
+        for i in range(1, numDisc):
+            oracle.lib().orc_path_point(np.float32(dt * np.float32(i)), tau[e], s[src[e]], s[dst[e]], x)
+            want[e, i] = x
+    d = [dev(torch, a) for a in (s, src, dst, tau)]
+    out, out2 = empty(torch, E * W * 6, torch.float32), empty(torch, E * W * 6, torch.float32)
+    off = dev(torch, np.arange(E + 1, dtype=np.int64) * W)
+    pumplib.check(L.pump_discretize_edges(ptr(d[0]), ptr(d[1]), ptr(d[2]), ptr(d[3]), E, numDisc, 0, ptr(out),
+                                          stream(torch)))
+    pumplib.check(L.pump_discretize_edges_off(ptr(d[0]), ptr(d[1]), ptr(d[2]), ptr(d[3]), E, ptr(off), numDisc,
+                                              0, ptr(out2), stream(torch)))
+    torch.cuda.synchronize()
+    assert same_bits(host(out), want.reshape(-1)) and same_bits(host(out2), want.reshape(-1))
+
+
 def test_roadmap_edges_one_read(gpu, pumplib, roadmap1000):
     """rn and the edges from one read of the pair costs equal pump_select_kth +
     pump_build_edges (the oracle's sort and scan) bit for bit."""
