@@ -185,10 +185,13 @@ __global__ void position_variance_kernel(int T, double *__restrict__ var) {
 }
 
 // ------------------------------------------------------------------ HSMC
-// One warp per new path.  Lane l owns particles p = 32k + l (k < words), one
-// bit per particle in bits[k/32] bit (k%32), so offset loads of a k-step are
-// 32 consecutive particles (384 contiguous bytes) and word k of the packed
-// mask is a single __ballot_sync.  The warp first finds the edge's W x H
+// One warp per new path.  Lane l owns particles 128 c + 4 l + j (j < 4), one
+// bit each, so the offsets of a c-step are 128 consecutive particles, three
+// 16-byte loads a lane (12-byte records of 32 particles, three 4-byte loads:
+// 311 us for 12,000 paths x 1024 particles with about 38 active half-spaces a
+// path; 203 us so, with two half-spaces of a waypoint tested on each loaded
+// particle and the comparison's product folded into its bound).  Such
+// wavefronts are bound by instruction issue.  The warp first finds the edge's W x H
 // half-space slots that are active (the reference skips a half-space when
 // b >= 1000, PUMP.cu:642); with none active the new mask is the parent's and
 // only the hit count is computed.  Every active half-space is tested for
@@ -213,14 +216,23 @@ constexpr int kHsmcThreads = 128;
 constexpr int kHsmcWarps = kHsmcThreads / 32;
 // blocks of a launch that loops over a device-side path count
 constexpr int kHsmcPersistBlocks = kNumSMs * 8;
-// Paths per block chunk: a block's warps take the chunk's paths one at a
-// time from a shared-memory counter, so a warp whose paths are cheap (no
-// active half-space: the parent's masks copied) takes more of them while
-// another tests particles, instead of leaving its slot idle until the
-// block's slowest warp ends.
-// Two paths per warp: a mid-size wavefront (a few thousand paths) still
-// spreads over every warp of the launch.
-constexpr int kHsmcChunk = 2 * kHsmcWarps;
+// Paths per block chunk of a wavefront of n paths on `blocks` resident blocks:
+// a block's warps take the chunk's paths one at a time from a shared-memory
+// counter, so a warp whose paths are cheap (no active half-space: the parent's
+// masks copied) takes more of them while another tests particles.  One path
+// per warp while that fits the blocks (a small wavefront spreads over every
+// warp); then one chunk per block, up to 16 paths (no second, nearly empty
+// round: 12,000 paths in chunks of 8 were 1.23 rounds of 1,216 blocks); then
+// rounds of 16 or more.
+__host__ __device__ inline int hsmc_chunk(long long n, long long blocks) {
+  const long long rounds = n / (16 * blocks) > 1 ? n / (16 * blocks) : 1;
+  const long long c = (n + blocks * rounds - 1) / (blocks * rounds);
+  return c > kHsmcWarps ? (int)c : kHsmcWarps;
+}
+inline unsigned hsmc_blocks(long long n) {
+  const long long want = (n + kHsmcWarps - 1) / kHsmcWarps;
+  return (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks);
+}
 constexpr int kHsmcFilterObs = 128;
 
 
@@ -238,6 +250,23 @@ __host__ __device__ inline size_t hsmc_boxes_smem(int numObs, int W, int maxHS) 
   return sizeof(float) * hsmc_boxes_obs_floats(numObs) +
          (size_t)kHsmcWarps * (sizeof(float4) * hsmc_hs_stride(W, maxHS) + hsmc_cnt_stride(W) +
                                sizeof(int) * kHsmcFilterObs);
+}
+
+// The largest LHS with fl(LHS * om) < b (the products grow with LHS, so the
+// test is LHS <= *bound): from the quotient, moved to the neighbour that is on
+// the boundary.  False (the test needs the product) outside ordinary values or
+// if three steps do not reach it.
+__device__ __forceinline__ bool hsmc_lhs_bound(float b, float om, float *bound) {
+  if (!(b >= 1e-25f && b < 1e25f && om >= 1e-10f && om <= 1e10f)) return false;  // also NaN
+  unsigned u = __float_as_uint(b / om);
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (!(__uint_as_float(u) * om < b)) --u;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (__uint_as_float(u + 1u) * om < b) ++u;
+  *bound = __uint_as_float(u);
+  return __uint_as_float(u) * om < b && !(__uint_as_float(u + 1u) * om < b);
 }
 
 // New path w (the whole warp).  valid_in[prev] is read, valid_out[w] /
@@ -359,14 +388,13 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
     }
     __syncwarp();
   }
-  // which half-space slots are active (b < 1000 or NaN, as !(b >= 1000))
-  uint32_t act[kMaxHsSlots / 32];
-  int nact = 0;
-#pragma unroll
-  for (int c = 0; c < kMaxHsSlots / 32; ++c) {
+  // which half-space slots are active (b < 1000 or NaN, as !(b >= 1000)):
+  // lane c holds the mask of slots 32 c .. 32 c + 31
+  uint32_t act = 0u;
+  for (int c = 0; c * 32 < slots; ++c) {
     const int sidx = c * 32 + lane;
     bool a = false;
-    if (c * 32 < slots && sidx < slots) {
+    if (sidx < slots) {
       const int i = sidx / maxHS, s = sidx - i * maxHS;
       if (Boxes) {
         a = s < (int)hcnt[i] && !(hs[sidx].w >= 1000);
@@ -375,29 +403,102 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
         a = stored && !(__ldg(&p.bs[hsHead + sidx]) >= 1000);
       }
     }
-    act[c] = (c * 32 < slots) ? __ballot_sync(0xffffffffu, a) : 0u;
-    nact += __popc(act[c]);
+    const uint32_t bal = __ballot_sync(0xffffffffu, a);
+    if (lane == c) act = bal;
   }
   int overflow = 0;
-  if (nact > 0) {
-    // unpack: bits[q] bit b = particle 32 * (32 q + b) + lane
+  if (__any_sync(0xffffffffu, act != 0u)) {
+    // unpack: bit 4 c + j of bits[q] = particle 1024 q + 128 c + 4 lane + j,
+    // from word 32 q + 4 c + lane / 8 of the mask
     uint32_t bits[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       bits[q] = 0u;
-      for (int b = 0; b < 32; ++b) {
-        const int k = q * 32 + b;
-        if (k >= words) break;
-        const uint32_t wk = __shfl_sync(0xffffffffu, mine[q], b);
-        bits[q] |= ((wk >> lane) & 1u) << b;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if (q * 1024 + c * 128 >= P) break;
+        const uint32_t wk = __shfl_sync(0xffffffffu, mine[q], 4 * c + (lane >> 3));
+        bits[q] |= ((wk >> (4 * (lane & 7))) & 0xFu) << (4 * c);
       }
     }
     const float dtLocal = p.topts[edge] / (W - 1);
     const float t0 = p.times[prev];
+    const bool vec = (p.Pmc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.offsets_t) & 15) == 0;
+    // slot sidx: its half-space and its bound on the offset's projection
+    auto half_space = [&](int sidx, float (&h)[4]) {
+      if (Boxes) {
+        const float4 f = hs[sidx];
+        h[0] = f.x;
+        h[1] = f.y;
+        h[2] = f.z;
+        h[3] = f.w;
+      } else {
 #pragma unroll
-    for (int c = 0; c < kMaxHsSlots / 32; ++c) {
-      uint32_t m = act[c];
+        for (int d = 0; d < 3; ++d) h[d] = __ldg(&p.as[(hsHead + sidx) * 3 + d]);
+        h[3] = __ldg(&p.bs[hsHead + sidx]);
+      }
+    };
+    // The test of N half-spaces of one waypoint (table row `row`) on every
+    // particle: dead unless fl(LHS * offset_mult) < b.  Bounded: h[n][3] is the
+    // largest LHS that passes (hsmc_lhs_bound), which saves the product.  The
+    // tests of a particle already dead are computed and discarded, so the loads
+    // do not wait on the bits.
+    auto test = [&](const float *row, auto count, auto bounded, const float (&h)[2][4]) {
+      constexpr int N = decltype(count)::value;
+      constexpr bool Bounded = decltype(bounded)::value;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (q * 1024 >= P) break;
+        uint32_t bq = bits[q];
+        if (bq == 0u) continue;  // this lane's particles of the group are all dead
+#pragma unroll 2
+        for (int c = 0; c < 8; ++c) {
+          const int p0 = q * 1024 + c * 128 + 4 * lane;
+          if (p0 >= P) continue;
+          float o[4][3];
+          if (vec) {
+            const float4 *r4 = reinterpret_cast<const float4 *>(row + (long long)p0 * 3);
+            const float4 x = __ldg(r4), y = __ldg(r4 + 1), z = __ldg(r4 + 2);
+            o[0][0] = x.x; o[0][1] = x.y; o[0][2] = x.z;
+            o[1][0] = x.w; o[1][1] = y.x; o[1][2] = y.y;
+            o[2][0] = y.z; o[2][1] = y.w; o[2][2] = z.x;
+            o[3][0] = z.y; o[3][1] = z.z; o[3][2] = z.w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int pp = p0 + j < p.Pmc ? p0 + j : p.Pmc - 1;
+#pragma unroll
+              for (int d = 0; d < 3; ++d) o[j][d] = __ldg(&row[(long long)pp * 3 + d]);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            bool pass = true;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+              // (the reference's sum starts from 0, which changes no comparison)
+              const float LHS = o[j][0] * h[n][0] + o[j][1] * h[n][1] + o[j][2] * h[n][2];
+              pass = pass && (Bounded ? LHS <= h[n][3] : LHS * p.offset_mult < h[n][3]);
+            }
+            if (!pass) bq &= ~(1u << (4 * c + j));
+          }
+        }
+        bits[q] = bq;
+      }
+    };
+    for (int c = 0; c * 32 < slots; ++c) {
+      uint32_t m = __shfl_sync(0xffffffffu, act, c);
+      // lane l: the bound of slot 32 c + l
+      float lhs_bound = 0.0f;
+      bool exact = false;
+      if ((m >> lane) & 1u) {
+        const int sidx = c * 32 + lane;
+        const float b = Boxes ? hs[sidx].w : __ldg(&p.bs[hsHead + sidx]);
+        exact = hsmc_lhs_bound(b, p.offset_mult, &lhs_bound);
+      }
+      const uint32_t exact_mask = __ballot_sync(0xffffffffu, exact);
       while (m) {
+        // the waypoint's next one or two active slots
         const int sidx = c * 32 + __ffs(m) - 1;
         m &= m - 1;
         const int i = sidx / maxHS;
@@ -407,54 +508,49 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
           overflow = 1;
           dtIdx = dtIdx < 0 ? 0 : p.T_rows - 1;
         }
-        float a0, a1, a2, b;
-        if (Boxes) {
-          const float4 h = hs[sidx];
-          a0 = h.x;
-          a1 = h.y;
-          a2 = h.z;
-          b = h.w;
-        } else {
-          b = __ldg(&p.bs[hsHead + sidx]);
-          a0 = __ldg(&p.as[(hsHead + sidx) * 3 + 0]);
-          a1 = __ldg(&p.as[(hsHead + sidx) * 3 + 1]);
-          a2 = __ldg(&p.as[(hsHead + sidx) * 3 + 2]);
-        }
         const float *row = p.offsets_t + (long long)dtIdx * p.Pmc * 3;
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-          if (q * 32 >= words) break;
-          uint32_t bq = bits[q];
-          if (bq == 0u) continue;  // this lane's particles of the group are all dead
-          // the test of a particle already dead is computed and discarded,
-          // so the loads do not wait on the bits and many are in flight
-#pragma unroll 8
-          for (int bb = 0; bb < 32; ++bb) {
-            const int k = q * 32 + bb;
-            const int pp = 32 * k + lane;
-            if (k < words && pp < P) {
-              const float *off = row + (long long)pp * 3;
-              float LHS = 0;
-              LHS += __ldg(&off[0]) * a0;
-              LHS += __ldg(&off[1]) * a1;
-              LHS += __ldg(&off[2]) * a2;
-              if (!(LHS * p.offset_mult < b)) bq &= ~(1u << bb);
-            }
+        float h[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+        half_space(sidx, h[0]);
+        const int second = m ? c * 32 + __ffs(m) - 1 : slots;
+        const bool two = second < (i + 1) * maxHS;
+        if (two) {
+          half_space(second, h[1]);
+          m &= m - 1;
+        }
+        const float bound0 = __shfl_sync(0xffffffffu, lhs_bound, sidx & 31);
+        const float bound1 = __shfl_sync(0xffffffffu, lhs_bound, second & 31);
+        const uint32_t used = (1u << (sidx & 31)) | (two ? 1u << (second & 31) : 0u);
+        if ((exact_mask & used) == used) {
+          h[0][3] = bound0;
+          if (two) {
+            h[1][3] = bound1;
+            test(row, std::integral_constant<int, 2>{}, std::true_type{}, h);
+          } else {
+            test(row, std::integral_constant<int, 1>{}, std::true_type{}, h);
           }
-          bits[q] = bq;
+        } else {
+          test(row, std::integral_constant<int, 1>{}, std::false_type{}, h);
+          if (two) {
+#pragma unroll
+            for (int d = 0; d < 4; ++d) h[0][d] = h[1][d];
+            test(row, std::integral_constant<int, 1>{}, std::false_type{}, h);
+          }
         }
       }
     }
-    // repack: word k = ballot of bit k over lanes; lane (k & 31) keeps it
+    // repack: an octet's nibbles form word 4 c + lane / 8; lane j keeps word j
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       uint32_t keep = 0u;
-      for (int b = 0; b < 32; ++b) {
-        const int k = q * 32 + b;
-        if (k >= words) break;
-        const bool live = 32 * k + lane < P;
-        const uint32_t wk = __ballot_sync(0xffffffffu, live && ((bits[q] >> b) & 1u));
-        if (b == lane) keep = wk;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if (q * 1024 + c * 128 >= P) break;
+        uint32_t v = ((bits[q] >> (4 * c)) & 0xFu) << (4 * (lane & 7));
+        v |= __shfl_xor_sync(0xffffffffu, v, 1);
+        v |= __shfl_xor_sync(0xffffffffu, v, 2);
+        v |= __shfl_xor_sync(0xffffffffu, v, 4);
+        v = __shfl_sync(0xffffffffu, v, 8 * (lane & 3));
+        if ((lane >> 2) == c) keep = v;
       }
       mine[q] = keep;
     }
@@ -496,7 +592,8 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
   int n = p.num_new;
   if (p.num_new_dev) n = (p.skip_dev && *p.skip_dev) ? 0 : (int)*p.num_new_dev;
   // a block with no path leaves before staging anything (block-uniform)
-  if ((long long)blockIdx.x * kHsmcChunk >= n) return;
+  const int chunk = hsmc_chunk(n, gridDim.x);
+  if ((long long)blockIdx.x * chunk >= n) return;
   float *s_obs = reinterpret_cast<float *>(s_dyn4);
   float4 *hs = nullptr;
   uint8_t *hcnt = nullptr;
@@ -513,13 +610,13 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
   }
   __shared__ int s_next;
   const int lane = threadIdx.x & 31;
-  const long long nchunks = ((long long)n + kHsmcChunk - 1) / kHsmcChunk;
+  const long long nchunks = ((long long)n + chunk - 1) / chunk;
   for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {  // block-uniform
     __syncthreads();  // every warp is done with the previous chunk's counter
     if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
-    const long long base = ch * kHsmcChunk;
-    const int cnt = (int)((long long)n - base < kHsmcChunk ? (long long)n - base : kHsmcChunk);
+    const long long base = ch * chunk;
+    const int cnt = (int)((long long)n - base < chunk ? (long long)n - base : chunk);
     while (true) {
       int t = 0;
       if (lane == 0) t = atomicAdd(&s_next, 1);
@@ -552,6 +649,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
   __shared__ int s_next;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = g->nq;
+  const int share = (int)gridDim.x > nq ? (int)gridDim.x / nq : 1;  // blocks per query
   if (warp == 0) {
     int c = 0;
     if (lane < nq) {
@@ -559,7 +657,8 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
       if (*reinterpret_cast<const volatile int *>(&a->L.active)) {
         const HsmcParams &hp = a->hp;
         const int n = (hp.skip_dev && *hp.skip_dev) ? 0 : (int)*hp.num_new_dev;
-        c = (n + kHsmcChunk - 1) / kHsmcChunk;
+        const int chunk = hsmc_chunk(n, share);
+        c = (n + chunk - 1) / chunk;
       }
     }
     // inclusive scan over the queries (nq <= 32 lanes)
@@ -603,8 +702,9 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
     uint8_t *s_cnt = reinterpret_cast<uint8_t *>(s_hs + kHsmcWarps * hs_stride);
     int *s_klist = reinterpret_cast<int *>(s_cnt + kHsmcWarps * cnt_stride);
     const int n = (p.skip_dev && *p.skip_dev) ? 0 : (int)*p.num_new_dev;
-    const int base = (ch - s_first[q]) * kHsmcChunk;
-    const int cnt = n - base < kHsmcChunk ? n - base : kHsmcChunk;
+    const int chunk = hsmc_chunk(n, share);
+    const int base = (ch - s_first[q]) * chunk;
+    const int cnt = n - base < chunk ? n - base : chunk;
     while (true) {
       int t = 0;
       if (lane == 0) t = atomicAdd(&s_next, 1);
@@ -883,10 +983,8 @@ pump_status_t hsmc_staged_async(int num_new, int W, const int *d_edge, const int
   hp.error = d_error;
   hp.num_new_dev = d_num_new;
   hp.skip_dev = d_skip;
-  // with a device-side count, num_new bounds it
-  const long long want = ((long long)num_new + kHsmcChunk - 1) / kHsmcChunk;
-  const unsigned blocks = d_num_new ? (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks)
-                                    : grid_for(num_new, kHsmcChunk);
+  // (with a device-side count, num_new bounds it)
+  const unsigned blocks = hsmc_blocks(num_new);
   void *args[] = {(void *)&hp};
   PUMP_CUDA_TRY(cudaLaunchKernel(hsmc_kernel_for<false>(P), dim3(blocks), dim3(kHsmcThreads), args,
                                  0, stream));
@@ -965,10 +1063,8 @@ pump_status_t hsmc_boxes_async(int num_new, int W, const int *d_edge, const int 
   const size_t smem = hsmc_boxes_smem(numObs, W, maxHS);
   const void *kern = hsmc_kernel_for<true>(P);
   PUMP_TRY(smem_attr(kern, smem));
-  // with a device-side count, num_new bounds it
-  const long long want = ((long long)num_new + kHsmcChunk - 1) / kHsmcChunk;
-  const unsigned blocks = d_num_new ? (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks)
-                                    : grid_for(num_new, kHsmcChunk);
+  // (with a device-side count, num_new bounds it)
+  const unsigned blocks = hsmc_blocks(num_new);
   void *args[] = {(void *)&hp};
   PUMP_CUDA_TRY(cudaLaunchKernel(kern, dim3(blocks), dim3(kHsmcThreads), args, smem, stream));
   return launch_status("hsmc_kernel (boxes)");

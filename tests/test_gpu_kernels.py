@@ -654,6 +654,55 @@ def test_hsmc_propagate(P, gpu, pumplib, oracle, roadmap1000):
     assert 0 < valid_bytes[base:].mean() < 1
 
 
+@pytest.mark.parametrize("om", [0.3, 0.0, 1e-12])
+@pytest.mark.parametrize("P,Pmc,n_new", [(1, 5, 40), (33, 130, 700), (129, 132, 5000), (1025, 1500, 300),
+                                         (4096, 4097, 60)])
+def test_hsmc_particle_quads(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap1000):
+    """Four particles a lane: table rows of whole quads (16-byte loads) and of
+    ragged ones, particle counts that end inside a quad, a word and a group of
+    128; noise multipliers for which the comparison's bound is not formed (0,
+    1e-12); wavefronts below and above one path per warp."""
+    torch, _ = gpu
+    L = pumplib.load()
+    r = roadmap1000
+    maxHS, T, base = 5, 400, 20
+    maxd2 = np.float32(0.1 * 0.3 * 0.3)
+    a, b, _ = oracle.cache_halfspaces(r["disc"], r["fe"], r["obs"], maxHS, maxd2)
+    tm, _ = oracle.particle_tables(0x1234, Pmc, T, pmajor=False)
+    rng = np.random.default_rng(P)
+    edges = rng.choice(np.nonzero(r["fe"])[0], n_new).astype(np.int32)
+    prev = rng.integers(0, base, n_new).astype(np.int32)
+    times = np.zeros(base + n_new, np.float32)
+    times[:base] = rng.uniform(0, 6, base).astype(np.float32)
+    words = (P + 31) // 32
+    vb = np.zeros((base + n_new, words * 32), np.uint8)
+    vb[:base, :P] = rng.random((base, P)) < 0.9
+    want = np.ascontiguousarray(vb[:, :P])
+    d = [dev(torch, x) for x in (edges, prev, a, b, times, r["te"], tm, r["disc"], r["obs"])]
+    cp_o = np.zeros(base + n_new, np.float32)
+    oracle.lib().orc_hsmc_propagate(n_new, 9, edges, prev, base, a, b, times, r["te"], 0.05, maxHS,
+                                    tm.reshape(-1), np.float32(om), Pmc, want, P, cp_o)
+    for boxes in (False, True):
+        d_valid = dev(torch, np.packbits(vb, axis=1, bitorder="little").view(np.uint32))
+        d_cp, d_err = empty(torch, base + n_new, torch.float32), dev(torch, np.zeros(1, np.int32))
+        if boxes:
+            st = L.pump_hsmc_propagate_boxes(
+                n_new, 9, ptr(d[0]), ptr(d[1]), r["src"].size, base, ptr(d[8]), r["obs"].shape[0], ptr(d[7]),
+                float(maxd2), maxHS, ptr(d[4]), ptr(d[5]), 0.05, ptr(d[6]), Pmc, T, om, ptr(d_valid), P,
+                ptr(d_cp), ptr(d_err), stream(torch))
+        else:
+            st = L.pump_hsmc_propagate(
+                n_new, 9, ptr(d[0]), ptr(d[1]), r["src"].size, base, ptr(d[2]), ptr(d[3]), maxHS, ptr(d[4]),
+                ptr(d[5]), 0.05, ptr(d[6]), Pmc, T, om, ptr(d_valid), P, ptr(d_cp), ptr(d_err), None,
+                stream(torch))
+        pumplib.check(st)
+        torch.cuda.synchronize()
+        got = bits_to_bytes(host(d_valid).reshape(base + n_new, words), P)
+        assert np.array_equal(got[base:], want[base:])
+        assert same_bits(host(d_cp)[base:base + n_new], cp_o[base:])
+        assert int(host(d_err)[0]) == 0
+
+
 def test_hsmc_device_checks(gpu, pumplib, oracle, roadmap1000):
     """HSMC's device-side checks: an edge index outside [0, E) and a parent
     outside [0, base) skip their paths and record PUMP_ERR_BAD_INPUT; a time
