@@ -308,5 +308,13 @@ inline int bisect_chunk(long long npairs) {
   return c >= 512 ? 512 : (c <= 64 ? 64 : (int)(c & ~31LL));
 }
 
+// Explicit pairs per warp: a warp takes as many rounds as its longest
+// bisection, so a small call (a smoothing batch has about a hundred) spreads
+// its pairs over the SMs, up to two warps each, before it fills warps.
+inline int bisect_jobs_per_warp(long long total) {
+  const long long per = (total + 2 * kNumSMs - 1) / (2 * kNumSMs);
+  return per < 1 ? 1 : (per < 32 ? (int)per : 32);
+}
+
 }  // namespace
 }  // namespace pump

@@ -164,14 +164,14 @@ __global__ void __launch_bounds__(kBisectThreads, 6) bvp_pairs_parity_persistent
                                         left - first < chunk ? (int)(left - first) : chunk);
 }
 
-// Explicit pairs, 32 per warp.
-__global__ void __launch_bounds__(128) bvp_batch_kernel(const JobPairs src) {
+// Explicit pairs, `per` (at most 32) per warp (bisect_jobs_per_warp).
+__global__ void __launch_bounds__(128) bvp_batch_kernel(const JobPairs src, int per) {
   const long long total = (long long)src.jb.n * src.jb.jobs;
   __shared__ BisectQueue s_queue[kBisectWarps];
   const int warp = threadIdx.x >> 5;
-  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * 32;
+  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * per;
   if (first >= total) return;
-  bisect_warp<ParityCost, 32>(src, s_queue[warp], first, total - first < 32 ? (int)(total - first) : 32);
+  bisect_warp<ParityCost, 32>(src, s_queue[warp], first, total - first < per ? (int)(total - first) : per);
 }
 
 // One thread per edge: findDiscretizedPath, 2pBVP.cu:53-69.  The edge's end
@@ -529,25 +529,38 @@ __global__ void __launch_bounds__(kRowThreads) candidate_rows_kernel(
     const float *__restrict__ seg_cost, const int *__restrict__ node_cnt,
     const int *__restrict__ seg_base, float dt, int rows_cap, int *__restrict__ len,
     float *__restrict__ cost, int *__restrict__ hits, float *__restrict__ states,
-    unsigned int *done) {
-  extern __shared__ int s_seg[];  // per segment: first row, then toff
+    unsigned int *done, int preload) {
+  extern __shared__ int s_seg[];  // per segment: first row, toff; with preload, time and cost
   __shared__ int s_len;
   const int p = blockIdx.x;
   const int n = node_cnt[p], b = seg_base[p], ns = n > 1 ? n - 1 : 0;
   int *srow = s_seg;
   float *stoff = reinterpret_cast<float *>(s_seg + ns);
+  // the segments' times and costs, loaded side by side (the recurrence below
+  // waits for each in turn otherwise)
+  const float *stime = topt + b, *scost = seg_cost ? seg_cost + b : nullptr;
+  if (preload) {
+    float *pt = stoff + ns, *pc = pt + ns;
+    for (int i = threadIdx.x; i < ns; i += kRowThreads) {
+      pt[i] = stime[i];
+      if (scost) pc[i] = scost[i];
+    }
+    __syncthreads();
+    stime = pt;
+    if (scost) scost = pc;
+  }
   if (threadIdx.x == 0) {
     float toff = 0, t = 0, c = 0;
     int rows = 0;
     for (int i = 0; i + 1 < n; ++i) {
-      const float tp = topt[b + i];
+      const float tp = stime[i];
       const int T = (int)((tp - toff) / dt + 1);
       stoff[i] = toff;
       srow[i] = rows;
       if (T > 0) t = dt * (T - 1) + toff;  // the last sample's time
       rows += T;
       toff = (t - tp) + dt;
-      if (seg_cost) c += seg_cost[b + i];
+      if (scost) c += scost[i];
     }
     s_len = rows;
     if (blockIdx.y == 0) {
@@ -573,8 +586,8 @@ __global__ void __launch_bounds__(kRowThreads) candidate_rows_kernel(
       a[d] = x0[s * kDim + d];
       c[d] = x1[s * kDim + d];
     }
-    if (Mode == PUMP_BVP_PARITY) path_point_fast(dt * k + stoff[lo], topt[s], a, c, x);
-    else path_point_f32(dt * k + stoff[lo], topt[s], a, c, x);
+    if (Mode == PUMP_BVP_PARITY) path_point_fast(dt * k + stoff[lo], stime[lo], a, c, x);
+    else path_point_f32(dt * k + stoff[lo], stime[lo], a, c, x);
     const long long t = (long long)p * rows_cap + r;
 #pragma unroll
     for (int d = 0; d < kDim; ++d) states[t * kDim + d] = x[d];
@@ -604,9 +617,11 @@ pump_status_t candidate_paths_async(const CandidateBufs &cb, int n_paths, int n_
     jb.topt[1] = cb.topt2;
     PUMP_TRY(bvp_jobs_launch(jb, mode, s));
   }
-  const size_t smem = sizeof(int) * 2 * (size_t)(max_segs > 0 ? max_segs : 1);
+  size_t smem = sizeof(int) * 2 * (size_t)(max_segs > 0 ? max_segs : 1);
   if (smem > 200 * 1024)
     return set_error(PUMP_ERR_CAPACITY, "candidate path of %d segments exceeds the row stage", max_segs);
+  const int preload = 2 * smem <= 200 * 1024;
+  if (preload) smem *= 2;
   int ny = (rows_cap + kRowThreads - 1) / kRowThreads;
   if (ny > 64) ny = 64;
   if (ny < 1) ny = 1;
@@ -617,11 +632,11 @@ pump_status_t candidate_paths_async(const CandidateBufs &cb, int n_paths, int n_
   if (mode == PUMP_BVP_PARITY)
     candidate_rows_kernel<PUMP_BVP_PARITY><<<grid, kRowThreads, smem, s>>>(
         cb.x0, cb.x1, cb.topt, with_cost ? cb.seg_cost : nullptr, cb.node_cnt, cb.seg_base, dt,
-        rows_cap, cb.len, with_cost ? cb.cost : nullptr, cb.hits, cb.states, cb.done);
+        rows_cap, cb.len, with_cost ? cb.cost : nullptr, cb.hits, cb.states, cb.done, preload);
   else
     candidate_rows_kernel<PUMP_BVP_PRECISION><<<grid, kRowThreads, smem, s>>>(
         cb.x0, cb.x1, cb.topt, with_cost ? cb.seg_cost : nullptr, cb.node_cnt, cb.seg_base, dt,
-        rows_cap, cb.len, with_cost ? cb.cost : nullptr, cb.hits, cb.states, cb.done);
+        rows_cap, cb.len, with_cost ? cb.cost : nullptr, cb.hits, cb.states, cb.done, preload);
   return launch_status("candidate_rows");
 }
 
@@ -657,8 +672,9 @@ pump_status_t bvp_jobs_launch(const BvpJobs &jb, int mode, cudaStream_t stream) 
   if (mode == PUMP_BVP_PRECISION) return bvp_jobs_precision_launch(jb, stream);
   if (mode == PUMP_BVP_PARITY_GPU) return bvp_jobs_refgpu_launch(jb, stream);
   const long long total = (long long)jb.n * jb.jobs;
-  const int threads = total < 152LL * 128 ? 32 : 128;
-  bvp_batch_kernel<<<grid_for(total, threads), threads, 0, stream>>>(JobPairs{jb});
+  const int per = bisect_jobs_per_warp(total);
+  const int warps = per < 32 ? 1 : kBisectWarps;
+  bvp_batch_kernel<<<grid_for(total, warps * per), warps * 32, 0, stream>>>(JobPairs{jb}, per);
   return launch_status("bvp_batch");
 }
 

@@ -126,14 +126,14 @@ __global__ void __launch_bounds__(kBisectThreads, 5) bvp_pairs_refgpu_kernel(All
                                         left - first < chunk ? (int)(left - first) : chunk);
 }
 
-// Explicit pairs (the BvpJobs layout of ctx.h), 32 per warp.
-__global__ void __launch_bounds__(128) bvp_batch_refgpu_kernel(const JobPairs src) {
+// Explicit pairs (the BvpJobs layout of ctx.h), `per` per warp.
+__global__ void __launch_bounds__(128) bvp_batch_refgpu_kernel(const JobPairs src, int per) {
   const long long total = (long long)src.jb.n * src.jb.jobs;
   __shared__ BisectQueue s_queue[kBisectWarps];
   const int warp = threadIdx.x >> 5;
-  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * 32;
+  const long long first = (blockIdx.x * (long long)(blockDim.x >> 5) + warp) * per;
   if (first >= total) return;
-  bisect_warp<RefGpuCost, 32>(src, s_queue[warp], first, total - first < 32 ? (int)(total - first) : 32);
+  bisect_warp<RefGpuCost, 32>(src, s_queue[warp], first, total - first < per ? (int)(total - first) : per);
 }
 
 }  // namespace
@@ -152,8 +152,9 @@ pump_status_t bvp_pairs_refgpu_launch(const float *d_samples, int N, float tmax,
 pump_status_t bvp_jobs_refgpu_launch(const BvpJobs &jb, cudaStream_t stream) {
   if (jb.n <= 0) return PUMP_OK;
   const long long total = (long long)jb.n * jb.jobs;
-  const int threads = total < 152LL * 128 ? 32 : 128;
-  bvp_batch_refgpu_kernel<<<grid_for(total, threads), threads, 0, stream>>>(JobPairs{jb});
+  const int per = bisect_jobs_per_warp(total);
+  const int warps = per < 32 ? 1 : kBisectWarps;
+  bvp_batch_refgpu_kernel<<<grid_for(total, warps * per), warps * 32, 0, stream>>>(JobPairs{jb}, per);
   return launch_status("bvp_batch_refgpu");
 }
 

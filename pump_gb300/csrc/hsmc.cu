@@ -804,10 +804,17 @@ __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
         x[k][d] = path[t * kDim + d] + __ldg(&offsets_t[((long long)t * Pmc + p) * 3 + d]) * offset_mult;
     }
   };
-  if (t0 < t1) load(t0, v);
+  if (t0 < t1) {
+    load(t0, v);
+    if (K == 1) load(t0 + 1, w);
+  }
   for (int t = t0; t < t1; ++t) {
     if (!__any_sync(0xffffffffu, todo != 0u)) break;
-    load(t + 1, w);
+    // one particle per lane: the next segment's end is on its way during the
+    // tests (a small call waits on these loads)
+    float next[K][3];
+    if (K > 1) load(t + 1, w);
+    else if (t + 1 < t1) load(t + 2, next);
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     bool nan = false;
 #pragma unroll
@@ -849,6 +856,9 @@ __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
     for (int k = 0; k < K; ++k)
 #pragma unroll
       for (int d = 0; d < 3; ++d) v[k][d] = w[k][d];
+    if (K == 1 && t + 1 < t1)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) w[0][d] = next[0][d];
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
