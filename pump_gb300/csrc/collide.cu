@@ -8,6 +8,8 @@
 // for operation (binary32, no contraction): broadphase on the segment's
 // bounding box, then the face-projection narrow phase with lambda not
 // clamped to [0, 1], as in collisionCheck.cu:104-143.
+#include <math.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -225,119 +227,125 @@ __global__ void __launch_bounds__(256) halfspace_kernel(const float *__restrict_
   if (count) count[wp] = stored;
 }
 
-// The same computation for a block of 256 consecutive waypoints, staged in
-// shared memory: the block's waypoints (contiguous in disc) are loaded and
-// its half-spaces (contiguous in as / bs) stored as whole lines.  Before the
-// waypoints run, the boxes that cannot pass the distance gate anywhere on an
-// edge are dropped once per edge: if for some axis the gap g between the
-// edge's bounding box and the box has fl(g * g) > maxd2, every waypoint's
-// d2 (a rounded sum of non-negative squares, each at least as large by the
-// monotonicity of rounding) exceeds maxd2 as well.  Edges with a NaN
-// waypoint, or maps with more than kFilterObs boxes, are not filtered.  The
-// remaining boxes are visited in index order, so the first maxHS half-spaces
-// are the reference's.  Used when maxHS <= kStagedMaxHS and the stage fits in
-// shared memory.
-constexpr int kStagedMaxHS = 8;
-constexpr int kHsThreads = 256;
-constexpr int kHsMaxEdges = kHsThreads / 2 + 2;  // W >= 2
-
+// The same computation, a warp per 32 consecutive waypoints, one per lane.
+// The boxes that cannot pass the distance gate at any of the warp's waypoints
+// are dropped first, one box per lane: if for some axis the gap g between the
+// waypoints' bounding box (by warp reductions) and the box has fl(g * g) >
+// maxd2, every waypoint's d2 (a rounded sum of non-negative squares, each at
+// least as large by the monotonicity of rounding) exceeds maxd2 as well; with
+// a NaN or infinite waypoint no box is dropped.  The rest are visited in index order: first
+// every lane notes the indices of its first maxHS boxes within the gate, then
+// the lanes compute the half-spaces of what they noted side by side, so the
+// longer computation runs at most maxHS times a warp, not once for every box
+// that some lane passes.  A warp assembles its records in shared memory and
+// stores them as whole lines; no block barrier after the boxes are staged.
 // Dense: every slot written (unused ones get the defaults), int counts.
 // Sparse (!Dense): only the stored half-spaces are written, straight to
 // global memory, with one-byte counts; slots at or past a waypoint's count
-// are left as they are (their readers stop at the count).
+// are left as they are (their readers stop at the count).  Used when maxHS <=
+// kStagedMaxHS and the stage fits in shared memory.  Bound by instruction
+// issue: 499,500 waypoints, 40 boxes, five slots: 53 us with one bounding box
+// and box mask per edge behind block barriers and every box's half-space
+// computed as it was visited, 35 us so.
+constexpr int kStagedMaxHS = 8;
+constexpr int kHsThreads = 256;
+constexpr int kHsWarps = kHsThreads / 32;
+
+__host__ __device__ inline size_t halfspace_obs_floats(int numObs) { return (size_t)((numObs * 12 + 3) & ~3); }
+// Per warp: 32 records of maxHS half-spaces (dense), then the noted indices.
+__host__ __device__ inline size_t halfspace_warp_floats(int maxHS, bool dense) {
+  return (dense ? (size_t)32 * maxHS * 4 : 0) + (size_t)32 * kStagedMaxHS / 2;
+}
+
 template <bool Dense>
-__global__ void __launch_bounds__(kHsThreads) halfspace_staged_kernel(
+__global__ void __launch_bounds__(kHsThreads) halfspace_warp_kernel(
     const float *__restrict__ obs, int numObs, const float *__restrict__ disc,
     const uint8_t *__restrict__ is_free_edge, long long E, int W, int maxHS, float maxd2,
     float *__restrict__ as, float *__restrict__ bs, int *__restrict__ count,
     uint8_t *__restrict__ count8) {
   extern __shared__ float4 s_dyn4[];
-  __shared__ float s_eb[kHsMaxEdges][6];  // edge bounding box: min[3], max[3]
-  __shared__ uint32_t s_mask[kHsMaxEdges][kFilterObs / 32];
-  __shared__ uint8_t s_filter[kHsMaxEdges];  // 1: free edge whose boxes are filtered
   float *s_obs = reinterpret_cast<float *>(s_dyn4);
-  float *s_wp = s_obs + ((numObs * 12 + 3) & ~3);
-  float *s_a = s_wp + kHsThreads * kDim;
-  float *s_b = s_a + kHsThreads * maxHS * 3;
   stage_obstacles(obs, numObs, s_obs);
-  const long long wp0 = blockIdx.x * (long long)kHsThreads;
+  // a box with a lower corner above its upper one (block-uniform) and a
+  // waypoint that is not finite (warp-uniform) take the reference's own
+  // comparisons
+  bool inverted = false;
+  for (int k = threadIdx.x; k < numObs * 3; k += kHsThreads) {
+    const float *bx = &s_obs[k / 3 * 12 + k % 3];
+    inverted = inverted || bx[0] > bx[6];
+  }
+  inverted = __syncthreads_or(inverted);
+  const float4 *s_obs4 = reinterpret_cast<const float4 *>(s_obs);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float *s_a = s_obs + halfspace_obs_floats(numObs) + warp * halfspace_warp_floats(maxHS, Dense);
+  float *s_b = s_a + (Dense ? 32 * maxHS * 3 : 0);
+  uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_b + (Dense ? 32 * maxHS : 0)) + lane;  // [h][lane]
+  const bool pairs8 = (reinterpret_cast<uintptr_t>(disc) & 7) == 0;
   const long long total = E * W;
-  const int nv = (int)(total - wp0 < kHsThreads ? total - wp0 : kHsThreads);
-  const long long e0 = wp0 / W;
-  const int ne = (int)((wp0 + nv - 1) / W - e0) + 1;
-  const int t = threadIdx.x;
-  block_load(s_wp, disc + wp0 * kDim, nv * kDim);
-  const bool filter = numObs <= kFilterObs;
-  if (t < ne) {
-    const long long e = e0 + t;
-    bool use = filter && is_free_edge[e];
-    float mn[3], mx[3];
-    const float *w = disc + e * W * kDim;
+  for (long long wp0 = (blockIdx.x * (long long)kHsWarps + warp) * 32; wp0 < total;
+       wp0 += (long long)gridDim.x * kHsThreads) {
+    const long long wp = wp0 + lane;
+    const int nv = (int)(total - wp0 < 32 ? total - wp0 : 32);
+    const long long e0 = total <= 0x7fffffffLL ? (long long)((unsigned)wp0 / (unsigned)W) : wp0 / W;
+    const unsigned r = (unsigned)(wp0 - e0 * W) + (unsigned)lane;
+    bool open = lane < nv && is_free_edge[e0 + r / (unsigned)W];
+    float pos[3] = {0.0f, 0.0f, 0.0f}, vel[3] = {0.0f, 0.0f, 0.0f};
+    if (open) {
+      const float *w = disc + wp * kDim;
+      if (pairs8) {
+        const float2 *w2 = reinterpret_cast<const float2 *>(w);
+        const float2 x = __ldg(w2), y = __ldg(w2 + 1), z = __ldg(w2 + 2);
+        pos[0] = x.x; pos[1] = x.y; pos[2] = y.x;
+        vel[0] = y.y; vel[1] = z.x; vel[2] = z.y;
+      } else {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) mn[d] = mx[d] = __ldg(&w[d]);
-    for (int i = 0; i < W; ++i)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float x = __ldg(&w[i * kDim + d]);
-        use = use && x == x;
-        mn[d] = fminf(mn[d], x);
-        mx[d] = fmaxf(mx[d], x);
+        for (int d = 0; d < 3; ++d) {
+          pos[d] = __ldg(&w[d]);
+          vel[d] = __ldg(&w[3 + d]);
+        }
       }
+    }
+    float mn[3], mx[3];
+    const bool odd = __any_sync(0xffffffffu, open && !(fabsf(pos[0]) < INFINITY && fabsf(pos[1]) < INFINITY &&
+                                                       fabsf(pos[2]) < INFINITY));
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      s_eb[t][d] = mn[d];
-      s_eb[t][3 + d] = mx[d];
+      mn[d] = warp_min_f32(open ? pos[d] : INFINITY);
+      mx[d] = warp_max_f32(open ? pos[d] : -INFINITY);
     }
-    s_filter[t] = use;
-#pragma unroll
-    for (int k = 0; k < kFilterObs / 32; ++k) s_mask[t][k] = 0u;
-  }
-  __syncthreads();
-  if (filter) {
-    // (edge, box) pairs of the block: keep the boxes the gate can pass
-    for (int q = t; q < ne * numObs; q += kHsThreads) {
-      const int el = q / numObs, o = q - el * numObs;
-      if (!s_filter[el]) continue;
-      const bool keep = gate_keeps_box(s_eb[el], s_eb[el] + 3, &s_obs[o * 12], maxd2);
-      if (keep) atomicOr(&s_mask[el][o >> 5], 1u << (o & 31));
-    }
-  }
-  __syncthreads();
-  if (t < nv) {
-    const long long wp = wp0 + t;
-    const int el = (int)(wp / W - e0);
-    float *a = Dense ? s_a + t * maxHS * 3 : as + wp * maxHS * 3;
-    float *b = Dense ? s_b + t * maxHS : bs + wp * maxHS;
     int stored = 0;
-    if (is_free_edge[wp / W]) {
-      float pos[3], vel[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        pos[d] = s_wp[t * kDim + d];
-        vel[d] = s_wp[t * kDim + 3 + d];
-      }
-      const bool filt = s_filter[el];
-      const int words = filt ? (numObs + 31) / 32 : 0;
-      int o = -1;
-      uint32_t m = 0u;
-      int k = 0;
-      while (stored < maxHS) {
-        // next box in index order: from the edge's mask, or every box
-        if (filt) {
-          while (m == 0u && k < words) m = s_mask[el][k++];
-          if (m == 0u) break;
-          o = (k - 1) * 32 + __ffs(m) - 1;
-          m &= m - 1;
-        } else {
-          if (++o >= numObs) break;
+    for (int c0 = 0; c0 < numObs && __any_sync(0xffffffffu, open); c0 += 32) {
+      const bool keep = c0 + lane < numObs && (odd || gate_keeps_box(mn, mx, &s_obs[(c0 + lane) * 12], maxd2));
+      unsigned int boxes = __ballot_sync(0xffffffffu, keep);
+      while (boxes) {
+        const int o = c0 + __ffs(boxes) - 1;
+        boxes &= boxes - 1u;
+        // the squared distance from the greatest of the two gaps and 0 per
+        // axis: the closest point's offset up to its sign
+        const float4 bl = s_obs4[o * 3], bm = s_obs4[o * 3 + 1], bh = s_obs4[o * 3 + 2];
+        const float x = fmaxf(fmaxf(bl.x - pos[0], pos[0] - bm.z), 0.0f);
+        const float y = fmaxf(fmaxf(bl.y - pos[1], pos[1] - bm.w), 0.0f);
+        const float z = fmaxf(fmaxf(bl.z - pos[2], pos[2] - bh.x), 0.0f);
+        float d2 = x * x + y * y + z * z;
+        if (inverted || odd) d2 = gate_d2(pos, &s_obs[o * 12]);
+        if (open && !(d2 > maxd2)) {
+          s_idx[stored * 32] = (uint16_t)o;
+          ++stored;
+          open = stored < maxHS;
         }
-        float ah[3], bh;
-        if (!halfspace_of_box(pos, vel, &s_obs[o * 12], maxd2, ah, &bh)) continue;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) a[stored * 3 + d] = ah[d];
-        b[stored] = bh;
-        ++stored;
       }
+    }
+    // the noted boxes' half-spaces (a lane reads only its own indices)
+    const int most = __reduce_max_sync(0xffffffffu, stored);
+    float *a = Dense ? s_a + lane * maxHS * 3 : as + wp * maxHS * 3;
+    float *b = Dense ? s_b + lane * maxHS : bs + wp * maxHS;
+    for (int h = 0; h < most; ++h) {
+      if (h >= stored) continue;
+      float ah[3], bh;
+      halfspace_of_box(pos, vel, &s_obs[(int)s_idx[h * 32] * 12], maxd2, ah, &bh);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) a[h * 3 + d] = ah[d];
+      b[h] = bh;
     }
     if (Dense) {
       for (int h = stored; h < maxHS; ++h) {
@@ -346,21 +354,29 @@ __global__ void __launch_bounds__(kHsThreads) halfspace_staged_kernel(
         a[h * 3 + 2] = -1.0f;
         b[h] = 1111.0f;
       }
-      if (count) count[wp] = stored;
-    } else {
+      if (count && lane < nv) count[wp] = stored;
+      __syncwarp();
+      warp_store(as + wp0 * maxHS * 3, s_a, nv * maxHS * 3);
+      warp_store(bs + wp0 * maxHS, s_b, nv * maxHS);
+      __syncwarp();  // the records are rewritten by the warp's next waypoints
+    } else if (lane < nv) {
       count8[wp] = (uint8_t)stored;
     }
-  }
-  if (Dense) {
-    __syncthreads();
-    block_store(as + wp0 * maxHS * 3, s_a, nv * maxHS * 3);
-    block_store(bs + wp0 * maxHS, s_b, nv * maxHS);
   }
 }
 
 size_t halfspace_staged_smem(int numObs, int maxHS, bool dense) {
-  return sizeof(float) * ((size_t)((numObs * 12 + 3) & ~3) + (size_t)kHsThreads * kDim +
-                          (dense ? (size_t)kHsThreads * maxHS * 4 : 0));
+  return sizeof(float) * (halfspace_obs_floats(numObs) + kHsWarps * halfspace_warp_floats(maxHS, dense));
+}
+
+// Blocks of halfspace_warp_kernel: as many as are resident (the shared memory
+// allows one to eight an SM), so that the boxes are staged once for many
+// waypoints.
+unsigned int halfspace_grid(long long waypoints, size_t smem) {
+  const long long fit = (long long)(220 * 1024 / (smem + 1024));
+  const long long cap = (long long)kNumSMs * (fit < 1 ? 1 : (fit > 8 ? 8 : fit));
+  const long long want = (waypoints + kHsThreads - 1) / kHsThreads;
+  return (unsigned int)(want < cap ? want : cap);
 }
 
 pump_status_t obstacle_smem(int numObs, size_t *bytes) {
@@ -511,9 +527,8 @@ extern "C" pump_status_t pump_cache_halfspaces(const float *d_obstacles, int num
   PUMP_TRY(obstacle_smem(numObs, &smem));
   const size_t staged = halfspace_staged_smem(numObs, maxHS, true);
   if (maxHS <= kStagedMaxHS && staged <= 220 * 1024) {
-    PUMP_TRY(smem_attr((const void *)halfspace_staged_kernel<true>, staged));
-    halfspace_staged_kernel<true><<<grid_for(E * W, kHsThreads), kHsThreads, staged,
-                                    (cudaStream_t)stream>>>(
+    PUMP_TRY(smem_attr((const void *)halfspace_warp_kernel<true>, staged));
+    halfspace_warp_kernel<true><<<halfspace_grid(E * W, staged), kHsThreads, staged, (cudaStream_t)stream>>>(
         d_obstacles, numObs, d_disc, d_is_free_edge, E, W, maxHS, maxd2, d_as, d_bs, d_count,
         nullptr);
     return launch_status("cache_halfspaces");
@@ -542,10 +557,8 @@ extern "C" pump_status_t pump_cache_halfspaces_sparse(const float *d_obstacles, 
   const size_t staged = halfspace_staged_smem(numObs, maxHS, false);
   if (staged > 220 * 1024)
     return set_error(PUMP_ERR_CAPACITY, "%d obstacles exceed the shared-memory stage", numObs);
-  PUMP_TRY(smem_attr((const void *)halfspace_staged_kernel<false>, staged));
-  halfspace_staged_kernel<false><<<grid_for(E * W, kHsThreads), kHsThreads, staged,
-                                   (cudaStream_t)stream>>>(
-      d_obstacles, numObs, d_disc, d_is_free_edge, E, W, maxHS, maxd2, d_as, d_bs, nullptr,
-      d_count);
+  PUMP_TRY(smem_attr((const void *)halfspace_warp_kernel<false>, staged));
+  halfspace_warp_kernel<false><<<halfspace_grid(E * W, staged), kHsThreads, staged, (cudaStream_t)stream>>>(
+      d_obstacles, numObs, d_disc, d_is_free_edge, E, W, maxHS, maxd2, d_as, d_bs, nullptr, d_count);
   return launch_status("cache_halfspaces_sparse");
 }

@@ -8,10 +8,6 @@
 
 namespace pump {
 
-// Edge-level box filters keep one bit per box in registers for maps of up to
-// this many boxes (more boxes: every box is tested).
-constexpr int kFilterObs = 128;
-
 // Cooperative copy of the obstacle array into shared memory (48 B per box,
 // so 16-byte vector loads always apply when the base is 16-byte aligned).
 __device__ __forceinline__ void stage_obstacles(const float *__restrict__ obs, int numObs,
@@ -202,6 +198,22 @@ __device__ __forceinline__ bool warp_queue_hits(const float *s_wp_warp, int W, c
   return warp_queue_hits(s_wp_warp, UniformLanes{W}, s_obs, numObs, active, q, hit);
 }
 
+// The gate distance of halfspace_of_box: the squared distance from pos to the
+// box, the same operations.
+__device__ __forceinline__ float gate_d2(const float *pos, const float *box) {
+  float d2 = 0;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    float x;
+    if (pos[d] <= box[d]) x = box[d];
+    else if (pos[d] >= box[6 + d]) x = box[6 + d];
+    else x = pos[d];
+    x = x - pos[d];
+    d2 += x * x;
+  }
+  return d2;
+}
+
 // The half-space box o contributes at a waypoint (pos, vel): cacheHalfspaces,
 // hsmc.cu:10-99, with bvlsShortcut (bvls.cu:259-273) for the closest point.
 // False when the point is farther than the distance gate (d2 > maxd2);
@@ -258,7 +270,9 @@ __device__ __forceinline__ bool gate_keeps_box(const float *emin, const float *e
     const float above = l[d] - emax[d];  // box beyond the edge's max
     const float below = u[d] - emin[d];  // box below the edge's min
     if (above > 0.0f && above * above > maxd2) keep = false;
-    if (below < 0.0f && below * below > maxd2) keep = false;
+    // (a waypoint at or below the lower corner is measured from that corner,
+    // also when it lies above the upper one)
+    if (below < 0.0f && below * below > maxd2 && emin[d] > l[d]) keep = false;
   }
   return keep;
 }

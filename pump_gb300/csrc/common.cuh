@@ -70,7 +70,7 @@ __host__ __device__ __forceinline__ double p2f(float x) { double d = x; return d
 __host__ __device__ __forceinline__ double p3f(float x) { double d = x; return (d * d) * d; }
 __host__ __device__ __forceinline__ double p4f(float x) { double d = x; double s = d * d; return s * s; }
 
-// Block-wide contiguous copies between global and shared memory: 16-byte
+// Block-wide contiguous copy from shared to global memory: 16-byte
 // accesses when the global address and the count allow, so a block's
 // per-thread records (strided, uncoalesced when each thread stores its own)
 // move as whole 128-byte lines.  Callers synchronise around them.
@@ -83,14 +83,28 @@ __device__ __forceinline__ void block_store(float *__restrict__ dst, const float
     for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   }
 }
-__device__ __forceinline__ void block_load(float *dst, const float *__restrict__ src, int n) {
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (n & 3) == 0) {
+// The same from shared to global memory by one warp.
+__device__ __forceinline__ void warp_store(float *__restrict__ dst, const float *src, int n) {
+  const int lane = threadIdx.x & 31;
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0 && (n & 3) == 0) {
     float4 *d4 = reinterpret_cast<float4 *>(dst);
     const float4 *s4 = reinterpret_cast<const float4 *>(src);
-    for (int i = threadIdx.x; i < n / 4; i += blockDim.x) d4[i] = __ldg(&s4[i]);
+    for (int i = lane; i < n / 4; i += 32) d4[i] = s4[i];
   } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(&src[i]);
+    for (int i = lane; i < n; i += 32) dst[i] = src[i];
   }
+}
+
+// Least and greatest value of a warp (a NaN is passed over).
+__device__ __forceinline__ float warp_min_f32(float x) {
+  float y;
+  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float warp_max_f32(float x) {
+  float y;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // `const float g = -9.81;` (2pBVP.cu:3)

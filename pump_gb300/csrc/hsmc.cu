@@ -759,17 +759,6 @@ inline const void *hsmc_loop_kernel_for(int P) {
 // small call spreads over the SMs (K = 1).
 constexpr int kMcWarps = 16;
 
-__device__ __forceinline__ float warp_min_f32(float x) {
-  float y;
-  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float warp_max_f32(float x) {
-  float y;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // Grid (ceil(Pmc / (32 K)), paths).
 template <int K>
 __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(

@@ -581,6 +581,56 @@ def test_halfspaces_maps_and_gates(mapname, gpu, pumplib, oracle, roadmap1000):
         assert np.array_equal(host(d_n, E * 9)[free_wp], n[free_wp])
 
 
+@pytest.mark.parametrize("W,maxHS,E", [(2, 1, 17), (9, 8, 61), (33, 3, 5)])
+def test_halfspaces_odd_boxes(W, maxHS, E, gpu, pumplib, oracle):
+    """The warp's gate test against the reference's comparisons: boxes with
+    inverted, infinite and NaN corners, infinite and NaN waypoints, waypoints on
+    a box's faces; waypoint counts that leave a ragged last warp, one to eight
+    slots, dense and sparse."""
+    torch, _ = gpu
+    from pump_gb300 import workloads
+    L = pumplib.load()
+    rng = np.random.default_rng(W)
+    disc = rng.uniform(0, 1, (E, W, 6)).astype(np.float32)
+    fe = (rng.random(E) < 0.8).astype(np.uint8)
+    fe[:4] = 1
+    for kind in ("plain", "inverted", "infinite", "nan", "odd waypoints"):
+        obs = workloads.random_boxes(70, 3).copy()
+        x = disc.copy()
+        x[0, 0, :3] = obs[5, :3]
+        x[1, 1, :3] = obs[6, 6:9]
+        if kind == "inverted":
+            obs[4, [0, 6]] = obs[4, [6, 0]]
+        if kind == "infinite":
+            obs[7, 0], obs[8, 7], obs[9, 6] = -np.inf, np.inf, -np.inf
+        if kind == "nan":
+            obs[10, 1], obs[11, 8] = np.nan, np.nan
+        if kind == "odd waypoints":
+            x[2, 0, 0], x[3, 1, 2] = np.inf, np.nan
+        maxd2 = np.float32(0.03)
+        a, b, n = oracle.cache_halfspaces(x, fe, obs, maxHS, maxd2)
+        n = np.maximum(np.asarray(n).reshape(-1), 0)  # an edge that is not free: -1 there, 0 here
+        d_obs, d_x, d_fe = dev(torch, obs), dev(torch, x), dev(torch, fe)
+        d_a, d_b = empty(torch, a.size, torch.float32), empty(torch, b.size, torch.float32)
+        d_n, d_n8 = empty(torch, E * W, torch.int32), empty(torch, E * W, torch.uint8)
+        pumplib.check(L.pump_cache_halfspaces(ptr(d_obs), 70, ptr(d_x), ptr(d_fe), E, W, maxHS, float(maxd2),
+                                              ptr(d_a), ptr(d_b), ptr(d_n), stream(torch)))
+        torch.cuda.synchronize()
+        assert np.array_equal(host(d_n, E * W), n), kind
+        for got, want in ((host(d_a, a.size), a.reshape(-1)), (host(d_b, b.size), b.reshape(-1))):
+            assert np.array_equal(np.isnan(got), np.isnan(want)), kind
+            assert same_bits(got[~np.isnan(want)], want[~np.isnan(want)]), kind
+        d_b.fill_(-7.0)
+        pumplib.check(L.pump_cache_halfspaces_sparse(ptr(d_obs), 70, ptr(d_x), ptr(d_fe), E, W, maxHS,
+                                                     float(maxd2), ptr(d_a), ptr(d_b), ptr(d_n8), stream(torch)))
+        torch.cuda.synchronize()
+        cnt = host(d_n8, E * W)
+        assert np.array_equal(cnt, n.astype(np.uint8)), kind
+        slot = (np.arange(maxHS)[None, :] < cnt[:, None]).reshape(-1)
+        want = np.where(slot, b.reshape(-1), np.float32(-7.0))
+        assert np.array_equal(host(d_b, b.size), want, equal_nan=True), kind
+
+
 def test_collision_checks_many_obstacles(gpu, pumplib, oracle, roadmap1000):
     """More boxes than fit one block's threads (the reference's limit is 85)."""
     torch, _ = gpu
