@@ -27,10 +27,10 @@ namespace {
 
 constexpr int kFinishThreads = 1024;
 constexpr int kFinishWarps = kFinishThreads / 32;
-constexpr int kFinishChunk = 2 * kFinishThreads;  // masks per scan chunk
+constexpr int kFinishList = 8 * kFinishThreads;   // superset pairs listed at a time
 constexpr int kFinishBatch = 8;                   // loads in flight per thread
-constexpr int kFinishBatchA = 4;                  // the same, gathering the superset
-constexpr long long kBarrierSpin = 1ll << 22;  // polls (each with a 100 ns sleep)
+constexpr int kFinishBatchA = 8;                  // the same, gathering the superset
+constexpr long long kBarrierSpin = 1ll << 22;  // polls (each with a 20 ns sleep)
 
 template <class TSup>
 struct RnFinish {
@@ -52,7 +52,7 @@ struct RnFinish {
   int *go_start;                  // may be null
   unsigned int *hist;             // 3 x 2048 words, zero at launch
   unsigned long long *partial;    // 2 x gridDim.x words
-  unsigned int *bar;              // barrier count and generation, zero at launch
+  unsigned int *bar;              // barrier count, zero at launch
   unsigned long long *n_sup;      // out: the superset's size
   const int *err_in;              // an earlier pass's wait-bound error word, or null
   int *error;                     // this kernel's
@@ -60,32 +60,29 @@ struct RnFinish {
   long long spin_limit;
 };
 
-// Sense-counting grid barrier of a cooperative launch: false when the wait
-// gave up (the error word is set; every block then returns).
+// Grid barrier of a cooperative launch, an arrival counter (zero at launch)
+// that only grows: a block's arrival fixes the count its barrier ends at.  One
+// release per block and acquiring polls; data other blocks wrote is read
+// through L2 after it.  False when the wait gave up (the error word is set;
+// every block then returns).
 __device__ bool finish_barrier(unsigned int *bar, int *error, long long spin_limit) {
   using ref_t = cuda::atomic_ref<unsigned int, cuda::thread_scope_device>;
   __shared__ int s_ok;
-  __syncthreads();  // the block's writes are ordered before thread 0's fence
+  __syncthreads();  // the block's writes are ordered before thread 0's release
   if (threadIdx.x == 0) {
-    __threadfence();
-    ref_t gen(bar[1]);
-    const unsigned int g = gen.load(cuda::memory_order_acquire);
+    ref_t count(*bar);
+    const unsigned int mine = count.fetch_add(1u, cuda::memory_order_release);
+    const unsigned int end = (mine / gridDim.x + 1u) * gridDim.x;
     int ok = 1;
-    if (ref_t(bar[0]).fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
-      ref_t(bar[0]).store(0u, cuda::memory_order_relaxed);
-      gen.store(g + 1u, cuda::memory_order_release);
-    } else {
-      long long spins = 0;
-      while (gen.load(cuda::memory_order_acquire) == g) {
-        if (++spins > spin_limit || *(volatile int *)error) {
-          ok = 0;
-          atomicExch(error, 1);
-          break;
-        }
-        __nanosleep(100);
+    long long spins = 0;
+    while (count.load(cuda::memory_order_acquire) < end) {
+      if (++spins > spin_limit || *(volatile int *)error) {
+        ok = 0;
+        atomicExch(error, 1);
+        break;
       }
+      __nanosleep(20);
     }
-    __threadfence();
     s_ok = ok;
   }
   __syncthreads();
@@ -131,21 +128,6 @@ __device__ unsigned int finish_block_scan(unsigned int v, unsigned int *total) {
   return before + incl - v;
 }
 
-// Position of the k-th (from 0) set bit of m (k < popc(m)).
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int k) {
-  int pos = 0;
-#pragma unroll
-  for (int step = 16; step > 0; step >>= 1) {
-    const int c = __popc(m & ((1u << step) - 1u));
-    if (k >= c) {
-      k -= c;
-      m >>= step;
-      pos += step;
-    }
-  }
-  return pos;
-}
-
 // The slice [*q0, *q1) of n items for this block.
 __device__ __forceinline__ void finish_slice(long long n, long long *q0, long long *q1) {
   const long long B = gridDim.x, b = blockIdx.x;
@@ -156,8 +138,7 @@ __device__ __forceinline__ void finish_slice(long long n, long long *q0, long lo
 template <class TSup>
 __global__ void __launch_bounds__(kFinishThreads) rn_finish_kernel(const RnFinish<TSup> a) {
   __shared__ unsigned int s_hist[2048];
-  __shared__ unsigned int s_off[kFinishChunk + 1];
-  __shared__ uint32_t s_m[kFinishChunk];
+  __shared__ uint32_t s_list[kFinishList];
   __shared__ unsigned int s_wcnt[kFinishWarps];
   __shared__ uint32_t s_prefix, s_mask;
   __shared__ unsigned long long s_k;
@@ -188,67 +169,60 @@ __global__ void __launch_bounds__(kFinishThreads) rn_finish_kernel(const RnFinis
     before = finish_block_sum(before);
     total = finish_block_sum(total);
     unsigned long long run = before;
-    for (long long c0 = t0; c0 < t1; c0 += kFinishChunk) {
-      const int cn = (int)(t1 - c0 < kFinishChunk ? t1 - c0 : kFinishChunk);
-      // the chunk's masks and the exclusive offsets of their entries, two
-      // masks per thread
-      unsigned int v[2], sum = 0;
+    for (long long c0 = t0; c0 < t1; c0 += 2 * kFinishThreads) {
+      // two masks per thread, the exclusive offsets of their entries
+      uint32_t m[2], first[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int q = tid * 2 + u;
-        const uint32_t m = q < cn ? __ldg(&a.masks[c0 + q]) : 0u;
-        if (q < cn) s_m[q] = m;
-        v[u] = __popc(m);
-        sum += v[u];
+        const long long t = c0 + 2 * tid + u;
+        m[u] = t < t1 ? __ldg(&a.masks[t]) : 0u;
+        // (pair numbers are below 2^32, so mask numbers are below 2^28)
+        const uint32_t row = (uint32_t)t / (uint32_t)a.masks_per_row;
+        first[u] = row * (uint32_t)(a.N - 1) + ((uint32_t)t - row * (uint32_t)a.masks_per_row) * 32u;
       }
       unsigned int chunk = 0;
-      unsigned int ex = finish_block_scan(sum, &chunk);
+      unsigned int ex = finish_block_scan((unsigned int)(__popc(m[0]) + __popc(m[1])), &chunk);
+      // each thread lists its masks' pairs (a window of the chunk's entries at
+      // a time: all of them but for masks twice as full as usual), then the
+      // block takes the listed pairs' costs side by side
+      for (unsigned int e0 = 0; e0 < chunk; e0 += kFinishList) {
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int q = tid * 2 + u;
-        if (q < cn) s_off[q] = ex;
-        ex += v[u];
-      }
-      if (tid == 0) s_off[cn] = chunk;
-      __syncthreads();
-      // entry e of the chunk: the mask whose range holds e (the last with
-      // offset <= e), its (e - offset)-th set bit, the pair number
-      for (unsigned int e0 = 0; e0 < chunk; e0 += kFinishThreads * kFinishBatchA) {
+        for (int u = 0; u < 2; ++u)
+          while (m[u] && ex < e0 + kFinishList) {
+            s_list[ex - e0] = first[u] + (uint32_t)__ffs(m[u]) - 1u;
+            m[u] &= m[u] - 1u;
+            ++ex;
+          }
+        __syncthreads();
+        const unsigned int nl = chunk - e0 < kFinishList ? chunk - e0 : kFinishList;
         uint32_t vi[kFinishBatchA], vc[kFinishBatchA];
+        static_assert(kFinishBatchA * kFinishThreads == kFinishList, "one batch per window");
 #pragma unroll
         for (int u = 0; u < kFinishBatchA; ++u) {
-          const unsigned int e = e0 + u * kFinishThreads + tid;
-          if (e < chunk) {
-            int lo = 0, hi = cn;
-            while (hi - lo > 1) {
-              const int mid = (lo + hi) >> 1;
-              if (s_off[mid] <= e) lo = mid; else hi = mid;
-            }
-            const int bit = nth_set_bit(s_m[lo], (int)(e - s_off[lo]));
-            const long long t = c0 + lo;
-            const long long row = t / a.masks_per_row;
-            const long long col = (t - row * a.masks_per_row) * 32 + bit;
-            const long long idx = row * (a.N - 1) + col;
-            vi[u] = (uint32_t)idx;
-            vc[u] = __ldcg(reinterpret_cast<const uint32_t *>(a.copts) + idx);
+          const unsigned int e = u * kFinishThreads + tid;
+          if (e < nl) {
+            vi[u] = s_list[e];
+            vc[u] = __ldcg(reinterpret_cast<const uint32_t *>(a.copts) + vi[u]);
           }
         }
 #pragma unroll
         for (int u = 0; u < kFinishBatchA; ++u) {
-          const unsigned int e = e0 + u * kFinishThreads + tid;
-          const unsigned long long pos = run + e;
-          if (e < chunk && (long long)pos < a.cap) {
+          const unsigned int e = u * kFinishThreads + tid;
+          if (u * kFinishThreads >= (int)nl) break;  // block-uniform
+          const unsigned long long pos = run + e0 + e;
+          if (e < nl && (long long)pos < a.cap) {
             a.sup_idx[pos] = vi[u];
             reinterpret_cast<uint32_t *>(a.sup_c)[pos] = vc[u];
           }
-          const uint32_t bin = e < chunk ? key_of_bits(vc[u]) >> 21 : 0xFFFFFFFFu;
+          const uint32_t bin = e < nl ? key_of_bits(vc[u]) >> 21 : 0xFFFFFFFFu;
           const unsigned int peers = __match_any_sync(0xffffffffu, bin);
-          if (e < chunk && lane == __ffs(peers) - 1) atomicAdd(&s_hist[bin], __popc(peers));
+          if (e < nl && lane == __ffs(peers) - 1) atomicAdd(&s_hist[bin], __popc(peers));
         }
+        __syncthreads();  // the list is rewritten
       }
       run += chunk;
-      __syncthreads();
     }
+    __syncthreads();
     for (int q = tid; q < 2048; q += kFinishThreads)
       if (s_hist[q]) atomicAdd(&a.hist[q], s_hist[q]);
     if (!finish_barrier(a.bar, a.error, a.spin_limit)) return;
@@ -362,6 +336,24 @@ __global__ void __launch_bounds__(kFinishThreads) rn_finish_kernel(const RnFinis
   before = finish_block_sum(before);
   edges = finish_block_sum(edges);
   unsigned long long run = before + wbase;
+  const long long E = (long long)edges < a.max_edges ? (long long)edges : a.max_edges;
+  // the adjacency row starts with the edges (sorted by source): the edge at
+  // position e starts the rows after the previous edge's source up to its own;
+  // the last one also ends the rows after it.  The source of the edge before
+  // the warp's part comes from the superset entries before it.
+  int last_src = -1;
+  if (a.go_start && run > 0 && w0 < w1) {
+    for (long long b0 = w0; b0 > 0; b0 -= 32) {
+      const long long q = b0 - 1 - lane;
+      const unsigned int found = __ballot_sync(0xffffffffu, q >= 0 && __ldcg(&a.sup_c[q >= 0 ? q : 0]) < rn);
+      if (found) {
+        last_src = (int)(__ldcg(&a.sup_idx[b0 - __ffs(found)]) / (uint32_t)(a.N - 1));
+        break;
+      }
+    }
+  }
+  if (a.go_start && E == 0 && b == 0)
+    for (int r = tid; r <= a.N; r += kFinishThreads) a.go_start[r] = 0;
   for (long long b0 = w0; b0 < w1; b0 += 32 * kFinishBatch) {
     float c[kFinishBatch];
     uint32_t id[kFinishBatch];
@@ -395,20 +387,21 @@ __global__ void __launch_bounds__(kFinishThreads) rn_finish_kernel(const RnFinis
         a.e_copt[pos] = c[u];
         a.e_topt[pos] = t[u];
       }
+      if (a.go_start && bal) {
+        const unsigned int below = bal & lt;
+        const int from = below ? 31 - __clz(below) : 0;
+        const int before_src = __shfl_sync(0xffffffffu, ii[u], from);
+        if (f && (long long)pos < E) {
+          for (int r = (below ? before_src : last_src) + 1; r <= ii[u]; ++r) a.go_start[r] = (int)pos;
+          if ((long long)pos == E - 1)
+            for (int r = ii[u] + 1; r <= a.N; ++r) a.go_start[r] = (int)E;
+        }
+        last_src = __shfl_sync(0xffffffffu, ii[u], 31 - __clz(bal));
+      }
       run += __popc(bal);
     }
   }
-  if (!finish_barrier(a.bar, a.error, a.spin_limit)) return;
-  // ---- adjacency row starts (edges sorted by source) and the pack
-  const long long E = (long long)edges < a.max_edges ? (long long)edges : a.max_edges;
-  if (a.go_start) {
-    for (long long e = (long long)b * kFinishThreads + tid; e <= E;
-         e += (long long)B * kFinishThreads) {
-      const int prev = e > 0 ? __ldcg(&a.e_src[e - 1]) : -1;
-      const int cur = e < E ? __ldcg(&a.e_src[e]) : a.N;
-      for (int r = prev + 1; r <= cur; ++r) a.go_start[r] = (int)e;
-    }
-  }
+  // ---- the pack
   if (b == 0 && tid == 0) {
     *a.n_sup = total;
     RnEdgesPack pk;
