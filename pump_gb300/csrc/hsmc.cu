@@ -275,12 +275,12 @@ __device__ __forceinline__ bool hsmc_lhs_bound(float b, float om, float *bound) 
 // waypoint), slots at or past a waypoint's count are inactive without
 // reading them (they hold the defaults b = 1111 in the dense layout); stored
 // slots still need b < 1000.
-template <bool Boxes, int Q>
-__device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const float *s_obs,
-                                          float4 *hs, uint8_t *hcnt, int *klist) {
+// Epi: the search's epilogue (HsmcEpilogue) runs for each path.
+template <bool Boxes, int Q, bool Epi>
+__device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, int prev,
+                                          const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
   const int lane = threadIdx.x & 31;
   const unsigned int lt = (1u << lane) - 1u;
-  const int edge = p.wf_edge[w], prev = p.wf_prev[w];
   if (edge < 0 || edge >= p.num_edges || prev < 0 || prev >= p.num_prev) {
     if (lane == 0 && p.error) atomicExch(p.error, (int)PUMP_ERR_BAD_INPUT);
     return;
@@ -296,6 +296,17 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
       return;
     }
     W = (int)n;
+  }
+  // the epilogue's inputs, on their way while the path is propagated
+  float epi_time = 0.0f, epi_topt = 0.0f, epi_cost = 0.0f, epi_copt = 0.0f;
+  int epi_node = 0;
+  if (Epi && lane == 0) {
+    const HsmcEpilogue &e = p.epi;
+    epi_time = e.path_time[prev];
+    epi_topt = __ldg(&e.topt[edge]);
+    epi_cost = e.path_cost[prev];
+    epi_copt = __ldg(&e.copt[edge]);
+    epi_node = e.wf_node[w];
   }
   const int maxHS = p.maxHS, P = p.P;
   const int words = (P + 31) >> 5;
@@ -333,12 +344,10 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
         mx[d] = fmaxf(mx[d], x);
       }
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-        mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-      }
+    for (int d = 0; d < 3; ++d) {
+      mn[d] = warp_min_f32(mn[d]);
+      mx[d] = warp_max_f32(mx[d]);
+    }
     nan = __any_sync(0xffffffffu, nan);
     const bool filt = !nan && p.numObs <= kHsmcFilterObs;
     int nk = p.numObs;
@@ -566,26 +575,42 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, const floa
       valid_count += __popc(mine[q]);
     }
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) valid_count += __shfl_down_sync(0xffffffffu, valid_count, off);
+  valid_count = __reduce_add_sync(0xffffffffu, valid_count);
   if (lane == 0) {
     const float cp = ((float)(P - valid_count)) / P;
     p.cp_out[w] = cp;
     if (overflow && p.error) atomicExch(p.error, (int)PUMP_ERR_CAPACITY);
-    if (p.epi_on) {
+    if (Epi) {
       // PUMP.cu:164-185: time, cost and the CP cut-off of new path w
       const HsmcEpilogue &e = p.epi;
-      const int f = e.wf_open[w];
-      e.new_time[w] = e.path_time[prev] + e.topt[f];
-      e.new_cost[w] = e.path_cost[prev] + e.copt[f];
+      e.new_time[w] = epi_time + epi_topt;
+      e.new_cost[w] = epi_cost + epi_copt;
       const bool alive = !(cp > e.cp_cutoff);
       e.alive[w] = alive ? 1 : 0;
-      if (alive) e.new_next[w] = atomicExch(&e.new_head[e.wf_node[w]], w);
+      if (alive) e.new_next[w] = atomicExch(&e.new_head[epi_node], w);
     }
   }
 }
 
-template <bool Boxes, int Q>
+// The chunk's paths base .. base + cnt - 1 by the block's warps, each taking
+// the next path from the block's counter when it is free.  (Taking the next
+// path ahead, to load its edge and parent during the one before, lets a warp
+// with a long path hold back another: 221 instead of 197 us for 12,000 such
+// paths.)
+template <bool Boxes, int Q, bool Epi>
+__device__ __forceinline__ void hsmc_chunk_paths(const HsmcParams &p, int base, int cnt, int *s_next,
+                                                 const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
+  while (true) {
+    int t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(s_next, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= cnt) break;  // warp-uniform
+    hsmc_path<Boxes, Q, Epi>(p, base + t, p.wf_edge[base + t], p.wf_prev[base + t], s_obs, hs, hcnt, klist);
+    __syncwarp();  // the warp's half-space slots are rewritten by its next path
+  }
+}
+
+template <bool Boxes, int Q, bool Epi>
 __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
   extern __shared__ float4 s_dyn4[];
   const int warp = threadIdx.x >> 5;
@@ -609,7 +634,6 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
     klist = s_klist + warp * kHsmcFilterObs;
   }
   __shared__ int s_next;
-  const int lane = threadIdx.x & 31;
   const long long nchunks = ((long long)n + chunk - 1) / chunk;
   for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {  // block-uniform
     __syncthreads();  // every warp is done with the previous chunk's counter
@@ -617,21 +641,14 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
     __syncthreads();
     const long long base = ch * chunk;
     const int cnt = (int)((long long)n - base < chunk ? (long long)n - base : chunk);
-    while (true) {
-      int t = 0;
-      if (lane == 0) t = atomicAdd(&s_next, 1);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (t >= cnt) break;  // warp-uniform
-      hsmc_path<Boxes, Q>(p, (int)(base + t), s_obs, hs, hcnt, klist);
-      __syncwarp();  // the warp's half-space slots are rewritten by its next path
-    }
+    hsmc_chunk_paths<Boxes, Q, Epi>(p, (int)base, cnt, &s_next, s_obs, hs, hcnt, klist);
   }
 }
 
 // Q = 32-bit particle words per lane: P <= 1024 Q.
-template <bool Boxes, int Q>
+template <bool Boxes, int Q, bool Epi>
 __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_kernel(const HsmcParams p) {
-  hsmc_run<Boxes, Q>(p);
+  hsmc_run<Boxes, Q, Epi>(p);
 }
 
 // The search loop on the device, for every query of a group: the chunks of
@@ -705,15 +722,8 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
     const int chunk = hsmc_chunk(n, share);
     const int base = (ch - s_first[q]) * chunk;
     const int cnt = n - base < chunk ? n - base : chunk;
-    while (true) {
-      int t = 0;
-      if (lane == 0) t = atomicAdd(&s_next, 1);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (t >= cnt) break;  // warp-uniform
-      hsmc_path<true, Q>(p, base + t, s_obs, s_hs + warp * hs_stride, s_cnt + warp * cnt_stride,
-                         s_klist + warp * kHsmcFilterObs);
-      __syncwarp();  // the warp's half-space slots are rewritten by its next path
-    }
+    hsmc_chunk_paths<true, Q, true>(p, base, cnt, &s_next, s_obs, s_hs + warp * hs_stride,
+                              s_cnt + warp * cnt_stride, s_klist + warp * kHsmcFilterObs);
   }
 }
 
@@ -722,12 +732,12 @@ inline int hsmc_q(int P) {
   const int q = (P + 1023) / 1024;
   return q <= 1 ? 1 : (q <= 2 ? 2 : 4);
 }
-template <bool Boxes>
+template <bool Boxes, bool Epi>
 const void *hsmc_kernel_for(int P) {
   switch (hsmc_q(P)) {
-    case 1: return (const void *)hsmc_kernel<Boxes, 1>;
-    case 2: return (const void *)hsmc_kernel<Boxes, 2>;
-    default: return (const void *)hsmc_kernel<Boxes, 4>;
+    case 1: return (const void *)hsmc_kernel<Boxes, 1, Epi>;
+    case 2: return (const void *)hsmc_kernel<Boxes, 2, Epi>;
+    default: return (const void *)hsmc_kernel<Boxes, 4, Epi>;
   }
 }
 inline const void *hsmc_loop_kernel_for(int P) {
@@ -985,7 +995,7 @@ pump_status_t hsmc_staged_async(int num_new, int W, const int *d_edge, const int
   // (with a device-side count, num_new bounds it)
   const unsigned blocks = hsmc_blocks(num_new);
   void *args[] = {(void *)&hp};
-  PUMP_CUDA_TRY(cudaLaunchKernel(hsmc_kernel_for<false>(P), dim3(blocks), dim3(kHsmcThreads), args,
+  PUMP_CUDA_TRY(cudaLaunchKernel(hsmc_kernel_for<false, false>(P), dim3(blocks), dim3(kHsmcThreads), args,
                                  0, stream));
   return launch_status("hsmc_kernel");
 }
@@ -1036,10 +1046,7 @@ pump_status_t hsmc_boxes_fill(int num_new, int W, const int *d_edge, const int *
   hp.error = d_error;
   hp.num_new_dev = d_num_new;
   hp.skip_dev = d_skip;
-  if (epi) {
-    hp.epi = *epi;
-    hp.epi_on = 1;
-  }
+  if (epi) hp.epi = *epi;
   *out = hp;
   return PUMP_OK;
 }
@@ -1060,7 +1067,7 @@ pump_status_t hsmc_boxes_async(int num_new, int W, const int *d_edge, const int 
                            d_valid_in, d_valid_out, P, d_cp_out, d_error, d_num_new, d_skip, epi,
                            &hp, d_disc_off));
   const size_t smem = hsmc_boxes_smem(numObs, W, maxHS);
-  const void *kern = hsmc_kernel_for<true>(P);
+  const void *kern = epi ? hsmc_kernel_for<true, true>(P) : hsmc_kernel_for<true, false>(P);
   PUMP_TRY(smem_attr(kern, smem));
   // (with a device-side count, num_new bounds it)
   const unsigned blocks = hsmc_blocks(num_new);

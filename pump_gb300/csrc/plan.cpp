@@ -633,7 +633,7 @@ pump_status_t Planner::explore() {
   PUMP_TRY(d_wfPrev_.alloc(cap));
   PUMP_TRY(d_wfEdge_.alloc(cap));
   PUMP_TRY(d_err_.alloc(1));
-  DevBuf<int> d_prev, d_node, d_g0, d_g1, d_nhead, d_nnext, d_wnode, d_wopen, d_newhead, d_newnext;
+  DevBuf<int> d_prev, d_node, d_g0, d_g1, d_nhead, d_nnext, d_wnode, d_newhead, d_newnext;
   DevBuf<float> d_cost, d_cp, d_ncost, d_ntime;
   DevBuf<unsigned int> d_off;
   DevBuf<uint8_t> d_alive;
@@ -647,7 +647,6 @@ pump_status_t Planner::explore() {
   PUMP_TRY(d_nhead.alloc(N_));
   PUMP_TRY(d_nnext.alloc(cap));
   PUMP_TRY(d_wnode.alloc(cap));
-  PUMP_TRY(d_wopen.alloc(cap));
   PUMP_TRY(d_off.alloc(cap));
   PUMP_TRY(d_ncost.alloc(cap));
   PUMP_TRY(d_ntime.alloc(cap));
@@ -698,7 +697,6 @@ pump_status_t Planner::explore() {
   sd.wf_prev = d_wfPrev_.p;
   sd.wf_node = d_wnode.p;
   sd.wf_edge = d_wfEdge_.p;
-  sd.wf_open = d_wopen.p;
   sd.wf_off = d_off.p;
   sd.new_cost = d_ncost.p;
   sd.new_time = d_ntime.p;

@@ -401,7 +401,6 @@ __device__ __forceinline__ void expand_body(const SearchDev &sd, const int *g, i
             sd.wf_prev[q] = prev;
             sd.wf_node[q] = dst[c];
             sd.wf_edge[q] = e;
-            sd.wf_open[q] = e;
             sd.new_head[dst[c]] = -1;
           }
           off += __popc(bal);
@@ -920,7 +919,6 @@ pump_status_t search_expand(const SearchDev &sd, int g_idx, int n_g, int num_pat
 
 HsmcEpilogue search_hsmc_epilogue(const SearchDev &sd, float cp_cutoff) {
   HsmcEpilogue e{};
-  e.wf_open = sd.wf_open;
   e.wf_node = sd.wf_node;
   e.path_time = sd.path_time;
   e.path_cost = sd.path_cost;

@@ -51,7 +51,7 @@ struct SearchDev {
   int *g_list[2];
   int *node_head, *node_next;  // stored paths per node (linked lists)
   // the wavefront of the current iteration
-  int *wf_prev, *wf_node, *wf_edge, *wf_open;
+  int *wf_prev, *wf_node, *wf_edge;
   unsigned int *wf_off;          // expansion offsets per bucket entry
   float *new_cost, *new_time;
   const float *new_cp;           // HSMC output
@@ -81,7 +81,7 @@ struct CheckArgs {
 // CP cut-off, and each survivor linked into its node's list of new paths
 // (emptied by the expansion).
 struct HsmcEpilogue {
-  const int *wf_open, *wf_node;
+  const int *wf_node;
   const float *path_time, *path_cost, *topt, *copt;
   float *new_time, *new_cost;
   uint8_t *alive;
@@ -119,9 +119,7 @@ struct HsmcParams {
   int P;
   float *cp_out;
   int *error;
-  // the search's new-path step after each CP (when epi_on)
   HsmcEpilogue epi;
-  int epi_on;
 };
 
 // The search loop run on the device: a CUDA graph whose conditional while
