@@ -1302,10 +1302,13 @@ pump_status_t Planner::search_and_smooth() {
     // alphas the next D steps can visit are evaluated in one batch (dense
     // paths, costs and MC CPs of all of them), then the reference's decisions
     // are replayed in order over the results: the same sequence of alphas,
-    // best-path updates and early exit as PUMP.cu:492-541.  D = 3 (7 paths
-    // per batch): deeper batches save round trips but most of their Monte
-    // Carlo work is for alphas the bisection never visits.
-    const int D = 3, K = (1 << D) - 1;
+    // best-path updates and early exit as PUMP.cu:492-541.  Most of a deep
+    // batch's work is for alphas the bisection never visits, but a query alone
+    // on the GPU leaves it nearly idle: D = 5 (31 paths, 6 batches of up to 30
+    // steps) took 1063 us where D = 3 (10 batches) took 1187, D = 4 1135 and
+    // D = 6 1107 for a whole query at N = 1000.  Batch workers share the GPU
+    // and keep D = 3.
+    const int D = lazy_ ? 3 : 5, K = (1 << D) - 1;
     int it = 0;
     bool stop = false;
     while (it < 30 && !stop) {
