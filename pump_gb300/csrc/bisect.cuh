@@ -47,10 +47,10 @@ constexpr float kDcvalTol = 0.0001f;
 constexpr float kDeltaMin = 2e-10f;
 // Steps stage A takes at most by the derivative and by the difference: a pair
 // with more of them continues in stage B, so that the warp does not wait for
-// its longest.  Warp instructions a pair, from a count of the steps of random
-// pairs: 139 without limits, 112 with (8, 5), 108 with (6, 4), 113 with (0, 9).
-constexpr int kSlopeSteps = 6;
-constexpr int kDeltaSteps = 4;
+// its longest.  N = 4000, us (limits in this order): none 2855; (0, 9) 1964,
+// (2, 7) 1948, (4, 6) 1922, (4, 5) 1902, (5, 5) 1913, (6, 4) 1935, (7, 3) 2007.
+constexpr int kSlopeSteps = 4;
+constexpr int kDeltaSteps = 5;
 
 __device__ __forceinline__ bool delta_sign(const PairFF &f, float ta, float tb, int *sign) {
   float dv, err, ulp;
@@ -298,14 +298,14 @@ constexpr int kBisectThreads = 128;
 constexpr int kBisectWarps = kBisectThreads / 32;
 constexpr int kBisectRefill = 4;
 
-// Pairs per warp of the all-pairs kernels: 512 (16 per lane, so lanes idle
-// only while a chunk's last pairs finish) once that gives every SM several
-// rounds of blocks; smaller counts are split finer, down to 64 a warp, so that
-// the last round of blocks is not most of the work.
+// Pairs per warp of the all-pairs kernels: two rounds of the resident warps
+// (fewer pairs a warp end in more partly filled last queues, one round ends
+// with its slowest warp: N = 1000, reference-GPU arithmetic, 246 us in four
+// rounds, 209 in two, 231 in one), at least 64, and at most 768 (24 per lane).
 inline int bisect_chunk(long long npairs) {
-  const long long warps = (long long)kNumSMs * 24 * 4;
-  const long long c = npairs / warps;
-  return c >= 512 ? 512 : (c <= 64 ? 64 : (int)(c & ~31LL));
+  const long long warps = (long long)kNumSMs * 24 * 2;
+  const long long c = ((npairs + warps - 1) / warps + 31) & ~31LL;
+  return c >= 768 ? 768 : (c <= 64 ? 64 : (int)c);
 }
 
 // Explicit pairs per warp: a warp takes as many rounds as its longest

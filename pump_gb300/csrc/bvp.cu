@@ -150,7 +150,7 @@ struct ParityCost {
 // All pairs: each warp walks `chunk` consecutive pairs (bisect.cuh).  Bound by
 // instruction issue.  N = 4000 (16 M pairs): 6.11 ms with two float-float costs
 // per finite difference, 3.64 ms with the differences' signs from cost_delta
-// where it settles them, 1.93 ms in two stages with their step limits (about
+// where it settles them, 1.90 ms in two stages with their step limits (about
 // 110 warp instructions a pair; 31 KB of queue a block, 80 registers, 6 blocks
 // an SM).
 __global__ void __launch_bounds__(kBisectThreads, 6) bvp_pairs_parity_persistent(AllPairs src,
