@@ -70,8 +70,8 @@ __device__ __noinline__ float path_state_now(int d, float t, float tau, float p0
 // estimate and one residual to 7 u^2 (u = 2^-24), products by a binary32 value
 // 3 u^2 and by a float-float one 6 u^2, so r, r^2 and r^3 to 10, 26 and 42 u^2,
 // the edge's sums to 9 u^2 and the terms to at most 54 u^2; a sum of n terms
-// (their high parts by TwoSum, the errors and low parts in binary32) adds at
-// most 16 u^2: at most 70 u^2 M = 2^-41.9 M.  When the interval of half-width
+// (their high parts by TwoSum, the errors and unnormalised low parts in
+// binary32) adds at most 30 u^2: at most 84 u^2 M = 2^-41.6 M.  When the interval of half-width
 // 2^-41 M around the float-float value lies inside the binary32 rounding cell
 // of its high part, that is the expression's (float) conversion; otherwise (or
 // for tau outside [2^-20, 2^20], values outside [2^-40, 2^60] and non-finite
@@ -143,19 +143,32 @@ __device__ __forceinline__ PathFF path_ff_edge(float tau, const float *x0, const
 
 // *out = the binary32 rounding of every value within 2^-41 M + 2^-80 of v
 // (true), or false when the interval reaches a rounding boundary (or leaves
-// range).  The absolute 2^-80 covers float-float parts that fall below
-// binary32's normal range (each at most 2^-149 off, scaled by at most 2^60
-// through 1 / tau^3).
+// range).  The boundary taken on both sides is the nearer one (half a unit in
+// the last place; a quarter at a power of two).  The absolute 2^-80 covers
+// float-float parts that fall below binary32's normal range (each at most
+// 2^-149 off, scaled by at most 2^60 through 1 / tau^3).
 __device__ __forceinline__ bool ff_certify(FF v, float M, float *out) {
-  const float f = v.hi, af = fabsf(f);
-  if (!(af >= 0x1p-40f && af <= 0x1p60f && M <= 0x1p60f)) return false;  // also NaN
-  const unsigned bits = __float_as_uint(af);
-  const float ulp = __uint_as_float((bits & 0x7f800000u) - (23u << 23));
-  const float up = 0.5f * ulp, down = (bits & 0x7fffffu) ? 0.5f * ulp : 0.25f * ulp;
-  const float a = f >= 0.0f ? v.lo : -v.lo;  // offset towards larger magnitude
-  const float B = M * (0x1p-41f * 1.01f) + 0x1p-80f;
-  *out = f;
-  return a + B < up && B - a < down;
+  const unsigned bits = __float_as_uint(v.hi) & 0x7fffffffu;
+  // |v| in [2^-40, 2^60], which also rules out NaN; M up to 2^60 in B
+  const bool in = bits - 0x2b800000u <= 0x5d800000u - 0x2b800000u;
+  const unsigned low = (bits & 0x7fffffu) ? 24u << 23 : 25u << 23;
+  const float room = __uint_as_float((bits & 0x7f800000u) - low);
+  const float B = fmaf(M, 0x1p-41f * 1.01f, 0x1p-80f);
+  *out = v.hi;
+  return in && B <= 0x1p19f && fabsf(v.lo) + B < room;
+}
+
+// Products that only enter a sum, left unnormalised (the low part up to 4 u
+// of the high part).
+__device__ __forceinline__ FF ff_term(FF x, FF y) {
+  FF p = ff_two_prod(x.hi, y.hi);
+  p.lo = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, p.lo));
+  return p;
+}
+__device__ __forceinline__ FF ff_term_f(FF x, float b) {
+  FF p = ff_two_prod(x.hi, b);
+  p.lo = fmaf(x.lo, b, p.lo);
+  return p;
 }
 
 // The certified states of x; returns a bit per state that is not (its x is
@@ -167,8 +180,8 @@ __device__ __forceinline__ unsigned path_point_try(float t, float tau, const flo
   const FF r3 = ff_mul(r2, r);
   unsigned bad = 0u;
   // the velocities' 1 - (4 t tau) / tau^2 + 3 r^2, the binary32 product rounded
-  const FF r2x3 = ff_mul_f(r2, 3.0f);
-  const FF F = ff_mul_f(e.ru2, -(4 * t * tau));
+  const FF r2x3 = ff_term_f(r2, 3.0f);
+  const FF F = ff_term_f(e.ru2, -(4 * t * tau));
   const FF in = ff_sum(1.0f, F, r2x3);
   const float min = 1.0f + (fabsf(F.hi) + r2x3.hi);
 #pragma unroll
@@ -176,13 +189,13 @@ __device__ __forceinline__ unsigned path_point_try(float t, float tau, const flo
     const int a = k, b = k + 3;
     // position: A + X r^3 - Y r^2
     const float A = t * x0[b] + x0[a];
-    const FF T1 = ff_mul_f(r3, e.X[k]), T2 = ff_mul_f(r2, -e.Y[k]);
+    const FF T1 = ff_term_f(r3, e.X[k]), T2 = ff_term_f(r2, -e.Y[k]);
     if (!ff_certify(ff_sum(A, T1, T2), fabsf(A) + fabsf(T1.hi) + fabsf(T2.hi), &x[k])) bad |= 1u << k;
     // velocity: f1 / tau^2 + r^2 3 Z / tau + x0v (1 - F / tau^2 + 3 r^2)
     const float f1 = -(2 * t * e.inner[k]);
-    const FF S1 = ff_mul_f(e.ru2, f1);
-    const FF S2 = ff_mul(r2, e.Z[k]);
-    const FF S3 = ff_mul_f(in, x0[b]);
+    const FF S1 = ff_term_f(e.ru2, f1);
+    const FF S2 = ff_term(r2, e.Z[k]);
+    const FF S3 = ff_term_f(in, x0[b]);
     const FF s = ff_two_sum(S1.hi, S2.hi);
     const FF u = ff_two_sum(s.hi, S3.hi);
     const FF W = ff_fast_two_sum(u.hi, (s.lo + u.lo) + ((S1.lo + S2.lo) + S3.lo));
@@ -191,7 +204,7 @@ __device__ __forceinline__ unsigned path_point_try(float t, float tau, const flo
   {
     // z: t x0vz + x0z + r^2 q1 + r^3 q2
     const float P = t * x0[5];
-    const FF T1 = ff_mul(r2, e.q1), T2 = ff_mul(r3, e.q2);
+    const FF T1 = ff_term(r2, e.q1), T2 = ff_term(r3, e.q2);
     const FF A = ff_two_sum(P, x0[2]);
     const FF s = ff_two_sum(A.hi, T1.hi);
     const FF u = ff_two_sum(s.hi, T2.hi);
@@ -202,7 +215,7 @@ __device__ __forceinline__ unsigned path_point_try(float t, float tau, const flo
   {
     // vz: x0vz + (t tau) c1 + r^2 c2
     const float tt = t * tau;
-    const FF T1 = ff_mul_f(e.c1, tt), T2 = ff_mul(r2, e.c2);
+    const FF T1 = ff_term_f(e.c1, tt), T2 = ff_term(r2, e.c2);
     const float M = fabsf(x0[5]) + fabsf(tt) * e.mc1 + r2.hi * e.mc2;
     if (!ff_certify(ff_sum(x0[5], T1, T2), M, &x[5])) bad |= 1u << 5;
   }
