@@ -38,8 +38,8 @@ namespace {
 //     its square, one rounding more per term).  The six squares of s7 and of
 //     the t^2 coefficient (make_pair_ff): 36 u^2, with the product by 12 and
 //     the binary32 products' sums 6 u^2 more; s7's high part and the ten
-//     rounded terms: 66 u^2, and 11 u^2 for the closing fast sum should the
-//     high parts cancel below the errors: at most 119 u^2;
+//     rounded terms: 66 u^2, and 11 u^2 for the errors' sum in the closing fast
+//     sum: at most 119 u^2;
 //   - the t^2, t^3 and t^4 terms by Horner's rule: two products by t (3 u^2
 //     each), two fast sums (8 u^2 each), the product by t^2 (6 u^2), and the
 //     t^2 coefficient's own 42 u^2: at most 70 u^2; the last fast sum 8 u^2;
@@ -106,18 +106,23 @@ __device__ __forceinline__ FF ff_mul_f(FF x, float b) {
   p.lo = fmaf(x.lo, b, p.lo);
   return ff_fast_two_sum(p.hi, p.lo);
 }
+// Products that only enter a sum, left unnormalised (the low part up to 4 u
+// of the high part).
+__device__ __forceinline__ FF ff_term(FF x, FF y) {
+  FF p = ff_two_prod(x.hi, y.hi);
+  p.lo = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, p.lo));
+  return p;
+}
+__device__ __forceinline__ FF ff_term_f(FF x, float b) {
+  FF p = ff_two_prod(x.hi, b);
+  p.lo = fmaf(x.lo, b, p.lo);
+  return p;
+}
 // Reciprocal estimate (one instruction, within 1 ulp).
 __device__ __forceinline__ float ff_rcp(float x) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-__device__ __forceinline__ FF ff_div(FF x, FF y) {
-  const float q1 = __fdiv_rn(x.hi, y.hi);
-  const FF qy = ff_mul_f(y, q1);
-  const FF r = ff_add(x, {-qy.hi, -qy.lo});
-  const float q2 = __fdiv_rn(r.hi, y.hi);
-  return ff_fast_two_sum(q1, q2);
 }
 
 // Per-pair data of cost_ff, built without binary64 arithmetic (the GB300's
@@ -233,9 +238,9 @@ __device__ __forceinline__ bool cost_ff_value(const PairFF &f, float tau, CostFF
   // 1 + g^2, the t^4 coefficient (g^2 exact as a TwoProduct)
   const float g = PUMP_G;
   const FF d4 = ff_add_f(ff_two_prod(g, g), 1.0f);
-  FF h = ff_add_fast(ff_mul_f(d4, tau), f.d3);
-  h = ff_add_fast(ff_mul_f(h, tau), f.d2);
-  const FF v = ff_add_fast(ff_fast_two_sum(sum, err), ff_mul(h, t2));
+  FF h = ff_add_fast(ff_term_f(d4, tau), f.d3);
+  h = ff_add_fast(ff_term_f(h, tau), f.d2);
+  const FF v = ff_add_fast({sum, err}, ff_term(h, t2));
   // |k[q]| = |k_q| tau to within 2^-24 of each, and abs_k is the sum of the
   // |k_q| to within 2^-21: inside the bound's 1 % margin
   const float mag = fmaf(fmaf(fmaf(d4.hi, tau, f.abs_d3), tau, f.abs_d2), t2.hi,

@@ -158,19 +158,6 @@ __device__ __forceinline__ bool ff_certify(FF v, float M, float *out) {
   return in && B <= 0x1p19f && fabsf(v.lo) + B < room;
 }
 
-// Products that only enter a sum, left unnormalised (the low part up to 4 u
-// of the high part).
-__device__ __forceinline__ FF ff_term(FF x, FF y) {
-  FF p = ff_two_prod(x.hi, y.hi);
-  p.lo = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, p.lo));
-  return p;
-}
-__device__ __forceinline__ FF ff_term_f(FF x, float b) {
-  FF p = ff_two_prod(x.hi, b);
-  p.lo = fmaf(x.lo, b, p.lo);
-  return p;
-}
-
 // The certified states of x; returns a bit per state that is not (its x is
 // then unspecified).
 __device__ __forceinline__ unsigned path_point_try(float t, float tau, const float *x0,
