@@ -220,6 +220,20 @@ struct PairCoefs {
   FF dd, ds, A2s, A3;  // |D|^2, D.S, A2 / 4, A3
   float abs_ds;        // sum of |D_d S_d|
 };
+// Products and sums whose low part is left unnormalised (up to a few u of the
+// operands' magnitudes): what enters further products and sums.
+__device__ __forceinline__ FF ff_mul_raw(FF x, FF y) {
+  const FF p = two_prod(x.h, y.h);
+  return {p.h, fmaf(x.h, y.l, fmaf(x.l, y.h, p.l))};
+}
+__device__ __forceinline__ FF ff_mulf_raw(FF x, float c) {
+  const FF p = two_prod(x.h, c);
+  return {p.h, fmaf(x.l, c, p.l)};
+}
+__device__ __forceinline__ FF ff_add_raw(FF x, FF y) {
+  const FF s = two_sum(x.h, y.h);
+  return {s.h, s.l + (x.l + y.l)};
+}
 // x y added to the float-float sum s: the product exact to u^2, its high part
 // by TwoSum, the errors in binary32.
 __device__ __forceinline__ void ff_accum(FF x, FF y, FF *s) {
@@ -237,18 +251,19 @@ __device__ __forceinline__ PairCoefs make_pair_coefs(const SampleF &a, const Sam
     D[d] = two_sum(b.p[d], -a.p[d]);
     S[d] = two_sum(a.v[d], b.v[d]);
   }
-  FF dd = {0.0f, 0.0f}, ds = {0.0f, 0.0f}, vv = a.vv;
-  r.abs_ds = 0.0f;
+  FF dd = ff_mul_raw(D[0], D[0]), ds = ff_mul_raw(D[0], S[0]), vv = a.vv;
+  r.abs_ds = fabsf(D[0].h) * fabsf(S[0].h);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
+  for (int d = 1; d < 3; ++d) {
     ff_accum(D[d], D[d], &dd);
     ff_accum(D[d], S[d], &ds);
-    ff_accum({a.v[d], 0.0f}, {b.v[d], 0.0f}, &vv);
     r.abs_ds = fmaf(fabsf(D[d].h), fabsf(S[d].h), r.abs_ds);
   }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) vv = ff_add_raw(vv, two_prod(a.v[d], b.v[d]));
   r.dd = fast_two_sum(dd.h, dd.l);
   r.ds = two_sum(ds.h, ds.l);
-  r.A2s = ff_add({vv.h, vv.l}, b.vv);
+  r.A2s = ff_add(vv, b.vv);
   r.A3 = ff_mulf(two_sum(a.v[2], -b.v[2]), 2.0f * PUMP_G);
   return r;
 }
@@ -358,8 +373,9 @@ __device__ __forceinline__ float sqrt_f32(float x) {
 // cost at the root is c(x) + c'(x) dx / 2 (c' vanishes at the root; third
 // order), c(x) in float-float.  Errors, u = 2^-24, as multiples of the terms'
 // magnitudes: the coefficients at most 36 u^2, 1/x 6 u^2 a factor, each product
-// 6 u^2 and sum 8 u^2: under 140 u^2 for the cost, 100 u^2 for Q.  The bounds
-// take 2^-40 (256 u^2).  Where a bound reaches a rounding boundary (about 1e-4
+// 6 u^2 and sum 8 u^2, and 6 u^2 more an operation for the low parts left
+// unnormalised between them: under 190 u^2 for the cost, 140 u^2 for Q.  The
+// bounds take 2^-40 (256 u^2).  Where a bound reaches a rounding boundary (about 1e-4
 // of pairs) and wherever a condition fails, precise_general decides.
 //
 // Why float-float: the binary64 pipe runs at 1/64 of the binary32 rate here,
@@ -399,30 +415,31 @@ __device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const Sampl
   // Q(x), the Newton step and its error
   const FF x2 = two_prod(x, x);
   const FF A2 = {4.0f * pc.A2s.h, 4.0f * pc.A2s.l};
-  FF q = ff_mul({kA4, kA4l}, x2);
+  FF q = ff_mul_raw({kA4, kA4l}, x2);
   const float dq = fmaf(fmaf(4.0f, q.h, -2.0f * A2.h), x, 24.0f * pc.ds.h);
   const float ddq = fmaf(12.0f, q.h, 2.0f * A2.h) * 1.01f;  // (over its magnitude)
   const float mq = fmaf(fmaf(q.h + 3.0f * A2.h, x, 24.0f * pc.abs_ds), x, 36.0f * pc.dd.h);
-  q = ff_mulf(ff_add(q, {-A2.h, -A2.l}), x);
-  q = ff_mulf(ff_add(q, ff_mulf(pc.ds, 24.0f)), x);
-  q = ff_add(q, ff_mulf(pc.dd, -36.0f));
+  q = ff_mulf_raw(ff_add_raw(q, {-A2.h, -A2.l}), x);
+  q = ff_mulf_raw(ff_add_raw(q, ff_mulf_raw(pc.ds, 24.0f)), x);
+  q = ff_add_raw(q, ff_mulf_raw(pc.dd, -36.0f));
+  const float qv = q.h + q.l;
   const float r = rcp_f32(x);
   const float rq = rcp_f32(dq);
-  float dx = -(q.h * rq);
+  float dx = -(qv * rq);
   if (x >= tmax) dx = beyond ? 0.0f : fminf(dx, 0.0f);
   const float bt = beyond ? 0.0f
                           : fabsf(rq) * fmaf(fabsf(dx), fmaf(mq * r, 0x1p-18f, fabsf(dx) * ddq), mq * 0x1p-40f);
   ok = ok && fabsf(dx) <= 0x1p-18f * x && (beyond || dq > 0.0f);
   // c(x) = A3 + A4 x + r (A2 + r (A1 + r A0)), 1/x in float-float
   const FF rr = {r, r * fmaf(-x, r, 1.0f)};
-  FF v = ff_add(ff_mul(ff_mulf(pc.dd, 12.0f), rr), ff_mulf(pc.ds, -12.0f));
-  v = ff_add(ff_mul(v, rr), A2);
-  v = ff_add(ff_mul(v, rr), pc.A3);
-  v = ff_add(v, ff_mulf({kA4, kA4l}, x));
+  FF v = ff_add_raw(ff_mul_raw(ff_mulf_raw(pc.dd, 12.0f), rr), ff_mulf_raw(pc.ds, -12.0f));
+  v = ff_add_raw(ff_mul_raw(v, rr), A2);
+  v = ff_add_raw(ff_mul_raw(v, rr), pc.A3);
+  v = ff_add_raw(v, ff_mulf_raw({kA4, kA4l}, x));
   const float r2 = r * r;
   const float mc = fmaf(r, fmaf(r, fmaf(r, 12.0f * pc.dd.h, 12.0f * pc.abs_ds), 3.0f * A2.h),
                         fmaf(kA4, x, fabsf(pc.A3.h)));
-  v = fast_two_sum(v.h, fmaf(q.h * r2 * r2, beyond ? 0.0f : 0.5f * dx, v.l));
+  v = two_sum(v.h, fmaf(qv * r2 * r2, beyond ? 0.0f : 0.5f * dx, v.l));
   PreciseMin m;
   const FF t = fast_two_sum(x, dx);
   m.t = t.h;
