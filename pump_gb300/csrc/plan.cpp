@@ -1137,7 +1137,9 @@ pump_status_t Planner::eval_launch(CandSet &c, const std::vector<std::vector<flo
   const bool copy_out = with_cp && n <= 65535;
   char *hout = nullptr;
   PUMP_TRY(ctx_->pinned(c.pin_out, st_off + sizeof(float) * st_f, (void **)&hout));
-  cb.done = copy_out ? reinterpret_cast<unsigned int *>(c.out.p + head_words) : nullptr;
+  // (a word of its own past the segments' times: the row kernel clears it
+  // while other blocks still read the times)
+  cb.done = copy_out ? reinterpret_cast<unsigned int *>(c.out.p + 3 * (size_t)n + sg + seg_f) : nullptr;
   c.head_bytes = head;
   c.seq = copy_out ? next_seq() : 0u;
   if (copy_out) *reinterpret_cast<volatile unsigned int *>(hout + head) = c.seq - 1u;

@@ -211,3 +211,25 @@ def test_path_cp_matches_oracle(gpu, pumplib, oracle):
         assert np.float32(cost[k]) == np.float32(cost64)
         hit += cp[k] > 0
     assert hit > 0
+
+
+def test_path_cp_first_path_many_calls(gpu, pumplib, oracle):
+    """The first path's CP over many calls: the MC CP's counter of finished
+    blocks is cleared while the row kernel's blocks read the segments' times,
+    the first path's first segment among them."""
+    torch, ctx = gpu
+    from pump_gb300 import workloads
+    tm, pm = oracle.particle_tables(P=2048, T=400)
+    d_tm = dev(torch, tm)
+    for call in range(30):
+        obs = workloads.random_boxes(40, 50 + call)
+        nodes, offs, cnts = workloads.perturbed_paths(2 + call, 100 + call, obs, n_range=(3, 9))
+        d_obs = dev(torch, obs)
+        n = len(offs)
+        cp, cost, ln = np.zeros(n, np.float32), np.zeros(n, np.float32), np.zeros(n, np.int32)
+        pumplib.check(pumplib.load().pump_path_cp(
+            ctx.handle, nodes.ctypes.data, offs.ctypes.data, cnts.ctypes.data, n, pumplib.PUMP_BVP_PARITY,
+            ptr(d_tm), 2048, 400, 0.2, ptr(d_obs), obs.shape[0], cp.ctypes.data, cost.ctypes.data,
+            ln.ctypes.data, None))
+        c64, _, _ = oracle.path_cp(nodes[:cnts[0]], pm, np.float32(0.2), obs)
+        assert np.float32(cp[0]) == np.float32(c64), call
