@@ -189,8 +189,8 @@ __global__ void position_variance_kernel(int T, double *__restrict__ var) {
 // bit each, so the offsets of a c-step are 128 consecutive particles, three
 // 16-byte loads a lane (12-byte records of 32 particles, three 4-byte loads:
 // 311 us for 12,000 paths x 1024 particles with about 38 active half-spaces a
-// path; 203 us so, with two half-spaces of a waypoint tested on each loaded
-// particle and the comparison's product folded into its bound).  Such
+// path; 155 us so, with up to five half-spaces of a waypoint tested on each
+// loaded particle and the comparison's product folded into its bound).  Such
 // wavefronts are bound by instruction issue.  The warp first finds the edge's W x H
 // half-space slots that are active (the reference skips a half-space when
 // b >= 1000, PUMP.cu:642); with none active the new mask is the parent's and
@@ -233,6 +233,11 @@ inline unsigned hsmc_blocks(long long n) {
   const long long want = (n + kHsmcWarps - 1) / kHsmcWarps;
   return (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks);
 }
+// Half-spaces of one waypoint tested on each loaded quad of particles (12,000
+// paths, about 38 active half-spaces each: 225 us with 2, 194 with 3 or 4, 167
+// with 5, the reference's limit; the quads' loop is not unrolled: 224 us with
+// two quads in flight, whose code is twice as long).
+constexpr int kHsmcGroup = 5;
 constexpr int kHsmcFilterObs = 128;
 
 
@@ -452,7 +457,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
     // largest LHS that passes (hsmc_lhs_bound), which saves the product.  The
     // tests of a particle already dead are computed and discarded, so the loads
     // do not wait on the bits.
-    auto test = [&](const float *row, auto count, auto bounded, const float (&h)[2][4]) {
+    auto test = [&](const float *row, auto count, auto bounded, const float (&h)[kHsmcGroup][4]) {
       constexpr int N = decltype(count)::value;
       constexpr bool Bounded = decltype(bounded)::value;
 #pragma unroll
@@ -460,7 +465,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
         if (q * 1024 >= P) break;
         uint32_t bq = bits[q];
         if (bq == 0u) continue;  // this lane's particles of the group are all dead
-#pragma unroll 2
+#pragma unroll 1
         for (int c = 0; c < 8; ++c) {
           const int p0 = q * 1024 + c * 128 + 4 * lane;
           if (p0 >= P) continue;
@@ -496,7 +501,8 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
       }
     };
     for (int c = 0; c * 32 < slots; ++c) {
-      uint32_t m = __shfl_sync(0xffffffffu, act, c);
+      const uint32_t act_word = __shfl_sync(0xffffffffu, act, c);
+      uint32_t m = act_word;
       // lane l: the bound of slot 32 c + l
       float lhs_bound = 0.0f;
       bool exact = false;
@@ -507,9 +513,8 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
       }
       const uint32_t exact_mask = __ballot_sync(0xffffffffu, exact);
       while (m) {
-        // the waypoint's next one or two active slots
+        // the waypoint's next active slots, up to kHsmcGroup of them
         const int sidx = c * 32 + __ffs(m) - 1;
-        m &= m - 1;
         const int i = sidx / maxHS;
         const float time = t0 + i * dtLocal;
         int dtIdx = (int)(time / p.dt);
@@ -518,32 +523,40 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
           dtIdx = dtIdx < 0 ? 0 : p.T_rows - 1;
         }
         const float *row = p.offsets_t + (long long)dtIdx * p.Pmc * 3;
-        float h[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
-        half_space(sidx, h[0]);
-        const int second = m ? c * 32 + __ffs(m) - 1 : slots;
-        const bool two = second < (i + 1) * maxHS;
-        if (two) {
-          half_space(second, h[1]);
-          m &= m - 1;
-        }
-        const float bound0 = __shfl_sync(0xffffffffu, lhs_bound, sidx & 31);
-        const float bound1 = __shfl_sync(0xffffffffu, lhs_bound, second & 31);
-        const uint32_t used = (1u << (sidx & 31)) | (two ? 1u << (second & 31) : 0u);
-        if ((exact_mask & used) == used) {
-          h[0][3] = bound0;
-          if (two) {
-            h[1][3] = bound1;
-            test(row, std::integral_constant<int, 2>{}, std::true_type{}, h);
-          } else {
-            test(row, std::integral_constant<int, 1>{}, std::true_type{}, h);
-          }
-        } else {
-          test(row, std::integral_constant<int, 1>{}, std::false_type{}, h);
-          if (two) {
+        float h[kHsmcGroup][4];
+        int group = 0;
+        bool bounded = true;
 #pragma unroll
-            for (int d = 0; d < 4; ++d) h[0][d] = h[1][d];
-            test(row, std::integral_constant<int, 1>{}, std::false_type{}, h);
+        for (int n = 0; n < kHsmcGroup; ++n) {
+          const int bit = __ffs(m) - 1;
+          if (m == 0u || c * 32 + bit >= (i + 1) * maxHS) break;  // warp-uniform
+          m &= m - 1;
+          half_space(c * 32 + bit, h[n]);
+          if ((exact_mask >> bit) & 1u) h[n][3] = __shfl_sync(0xffffffffu, lhs_bound, bit);
+          else bounded = false;
+          ++group;
+        }
+        if (!bounded) {
+          // (rare: the bounds of the group's others are dropped again)
+          uint32_t back = 0u;
+          int at = sidx & 31;
+          for (int n = 0; n < group; ++n) {
+            float one[kHsmcGroup][4];
+            half_space(c * 32 + at, one[0]);
+            test(row, std::integral_constant<int, 1>{}, std::false_type{}, one);
+            back = act_word & ~((2u << at) - 1u);
+            at = back ? __ffs(back) - 1 : 0;
           }
+        } else if (group == 1) {
+          test(row, std::integral_constant<int, 1>{}, std::true_type{}, h);
+        } else if (group == 2) {
+          test(row, std::integral_constant<int, 2>{}, std::true_type{}, h);
+        } else if (group == 3) {
+          test(row, std::integral_constant<int, kHsmcGroup < 3 ? 1 : 3>{}, std::true_type{}, h);
+        } else if (group == 4) {
+          test(row, std::integral_constant<int, kHsmcGroup < 4 ? 1 : 4>{}, std::true_type{}, h);
+        } else {
+          test(row, std::integral_constant<int, kHsmcGroup < 5 ? 1 : 5>{}, std::true_type{}, h);
         }
       }
     }
