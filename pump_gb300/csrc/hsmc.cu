@@ -770,8 +770,7 @@ inline const void *hsmc_loop_kernel_for(int P) {
 // Block = 32 K particles (K per lane) of one path x kMcWarps warps, which
 // split the path's segments into consecutive runs (a run carries a segment's
 // end over as the next one's start).  Per segment the warp takes the bounding
-// box of its particles' segments (the ones that have not collided) by warp
-// reductions, tests the boxes against it one per lane, and only those that it
+// box of its particles' segments by warp reductions, tests the boxes against it one per lane, and only those that it
 // is not broadphase-disjoint from are tested per particle: a box disjoint
 // from the common bounding box is disjoint from every particle's, whose
 // reference test then passes.  With a NaN coordinate every box is kept.  (One
@@ -816,8 +815,30 @@ __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
         x[k][d] = path[t * kDim + d] + __ldg(&offsets_t[((long long)t * Pmc + p) * 3 + d]) * offset_mult;
     }
   };
+  struct Ends {
+    float lo[3], hi[3], sum;
+  };
+  auto ends = [&](const float (&x)[K][3]) {
+    Ends e;
+    e.sum = 0.0f;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      e.lo[d] = e.hi[d] = x[0][d];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        e.sum += x[k][d];  // (infinities of both signs also keep every box)
+        if (k > 0) {
+          e.lo[d] = fminf(e.lo[d], x[k][d]);
+          e.hi[d] = fmaxf(e.hi[d], x[k][d]);
+        }
+      }
+    }
+    return e;
+  };
+  Ends ve{};
   if (t0 < t1) {
     load(t0, v);
+    ve = ends(v);
     if (K == 1) load(t0 + 1, w);
   }
   for (int t = t0; t < t1; ++t) {
@@ -827,23 +848,17 @@ __global__ void __launch_bounds__(32 * kMcWarps) mc_cp_kernel(
     float next[K][3];
     if (K > 1) load(t + 1, w);
     else if (t + 1 < t1) load(t + 2, next);
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool nan = false;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if ((todo >> k) & 1u)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          nan = nan || v[k][d] != v[k][d] || w[k][d] != w[k][d];
-          lo[d] = fminf(lo[d], fminf(v[k][d], w[k][d]));
-          hi[d] = fmaxf(hi[d], fmaxf(v[k][d], w[k][d]));
-        }
-    nan = __any_sync(0xffffffffu, nan);
+    // the lane's particles' bounding box, from those of the segment's two
+    // ends (the start's was the end's before); a NaN coordinate shows in the sum
+    const Ends we = ends(w);
+    const bool nan = __any_sync(0xffffffffu, ve.sum != ve.sum || we.sum != we.sum);
+    float lo[3], hi[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      lo[d] = warp_min_f32(lo[d]);
-      hi[d] = warp_max_f32(hi[d]);
+      lo[d] = warp_min_f32(fminf(ve.lo[d], we.lo[d]));
+      hi[d] = warp_max_f32(fmaxf(ve.hi[d], we.hi[d]));
     }
+    ve = we;
     for (int c0 = 0; c0 < numObs; c0 += 32) {
       bool keep = false;
       if (c0 + lane < numObs) {
