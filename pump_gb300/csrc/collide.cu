@@ -119,17 +119,8 @@ __global__ void __launch_bounds__(T) free_edges_queue_kernel(
   const int W = numDisc + 1;
   const long long e0 = blockIdx.x * (long long)T;
   const int nv = (int)(E - e0 < T ? E - e0 : T);
-  {  // the block's waypoints are contiguous in disc; keep their positions
-    // (24-byte records: an 8-byte load of x, y and a 4-byte load of z)
-    const float *src = disc + e0 * W * kDim;
-    for (int r = threadIdx.x; r < nv * W; r += T) {
-      const float2 xy = __ldg(reinterpret_cast<const float2 *>(src + (long long)r * kDim));
-      const float z = __ldg(src + (long long)r * kDim + 2);
-      s_wp[r * 3] = xy.x;
-      s_wp[r * 3 + 1] = xy.y;
-      s_wp[r * 3 + 2] = z;
-    }
-  }
+  // the block's waypoints are contiguous in disc; their positions are kept
+  stage_positions(disc + e0 * W * kDim, nv * W, s_wp);
   stage_obstacles(obs, numObs, s_obs);  // ends with __syncthreads
   const int t = threadIdx.x, warp = t >> 5;
   const bool hit = warp_queue_hits(s_wp + warp * 32 * W * 3, W, s_obs, numObs, t < nv,
@@ -167,16 +158,7 @@ __global__ void __launch_bounds__(T) free_edges_off_kernel(
   s_first[t] = t < nv ? (int)(off[e0 + t] - wbase) : 0;
   s_cnt[t] = (int)cnt;
   const int total = (int)(off[e0 + nv] - base);
-  {
-    const float *src = disc + base * kDim;
-    for (int r = t; r < total; r += T) {
-      const float2 xy = __ldg(reinterpret_cast<const float2 *>(src + (long long)r * kDim));
-      const float z = __ldg(src + (long long)r * kDim + 2);
-      s_wp[r * 3] = xy.x;
-      s_wp[r * 3 + 1] = xy.y;
-      s_wp[r * 3 + 2] = z;
-    }
-  }
+  stage_positions(disc + base * kDim, total, s_wp);
   stage_obstacles(obs, numObs, s_obs);  // ends with __syncthreads
   const bool hit = warp_queue_hits(s_wp + (wbase - base) * 3,
                                    RaggedLanes{s_first + warp * 32, s_cnt + warp * 32}, s_obs, numObs,

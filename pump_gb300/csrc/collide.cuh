@@ -20,7 +20,22 @@ __device__ __forceinline__ void stage_obstacles(const float *__restrict__ obs, i
   } else {
     for (int i = threadIdx.x; i < n; i += blockDim.x) s_obs[i] = __ldg(&obs[i]);
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // the callers' asynchronous copies
   __syncthreads();
+}
+
+// The positions of n consecutive 24-byte waypoint records as 12-byte records
+// in shared memory, by asynchronous copies that all of the block's threads
+// issue at once (one round trip to memory instead of one per few records and
+// thread).  stage_obstacles after it waits for them.
+__device__ __forceinline__ void stage_positions(const float *__restrict__ src, int n, float *dst) {
+  const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+  for (int r = threadIdx.x; r < n; r += blockDim.x)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to + (unsigned)(r * 3 + d) * 4u),
+                   "l"(src + (long long)r * kDim + d)
+                   : "memory");
 }
 
 // broadphaseValidQ, collisionCheck.cu:104-112
