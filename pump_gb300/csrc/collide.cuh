@@ -169,18 +169,46 @@ __device__ __forceinline__ bool warp_queue_hits(const float *s_wp_warp, Lanes la
     const float *wp = s_wp_warp + lay.first(el) * kPos;
     const int numDisc = lay.count(el) - 1;
     const float *ob = &s_obs[o * 12];
-    float v[3], w[3];
+    // the segments that the broadphase leaves, 32 at a time, then their narrow
+    // tests: a lane has one or two of them, at other places than its
+    // neighbours, so the narrow test would run for almost every segment
+    for (int i0 = 0; i0 < numDisc; i0 += 32) {
+      const int n = numDisc - i0 < 32 ? numDisc - i0 : 32;
+      const float *p = wp + i0 * kPos;
+      float v[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) v[d] = wp[d];
-    for (int i = 0; i < numDisc; ++i) {
+      for (int d = 0; d < 3; ++d) v[d] = p[d];
+      unsigned int left = 0u;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) {
+        float w[3], bbMin[3], bbMax[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) w[d] = wp[(i + 1) * kPos + d];
-      if (segment_box_hit(v, w, ob)) {
-        hit[el] = 1;
-        return;
+        for (int d = 0; d < 3; ++d) {
+          w[d] = p[(i + 1) * kPos + d];
+          const bool down = v[d] > w[d];
+          bbMin[d] = down ? w[d] : v[d];
+          bbMax[d] = down ? v[d] : w[d];
+        }
+        const bool apart = (bbMax[0] <= ob[0]) | (ob[6] <= bbMin[0]) | (bbMax[1] <= ob[1]) |
+                           (ob[7] <= bbMin[1]) | (bbMax[2] <= ob[2]) | (ob[8] <= bbMin[2]);
+        left |= apart ? 0u : 1u << i;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[d] = w[d];
       }
+      while (left) {
+        const float *a = p + (__ffs(left) - 1) * kPos;
+        left &= left - 1u;
+        float b[3], e[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) v[d] = w[d];
+        for (int d = 0; d < 3; ++d) {
+          b[d] = a[d];
+          e[d] = a[kPos + d];
+        }
+        if (!motion_valid(b, e, ob)) {
+          hit[el] = 1;
+          return;
+        }
+      }
     }
   };
   int head = 0, tail = 0;  // warp-uniform
