@@ -808,41 +808,32 @@ def mode_record(lib, L, ctx, torch, w, mode, args, flush, batch, steps=None, war
 
 
 # Binary64 flops per ordered pair of the 2pBVP kernels (a fused multiply-add
-# counts two), counted from the kernels' source and confirmed by ncu's
-# instruction mix on this workload (per pair: 10 DFMA, 6 DADD, 2 DMUL):
-#  precision: coefficient assembly in float-float on the FP32 pipe; binary64
-#             only for the six coefficients (hi + lo), the Newton residual
-#             Q(x) and step, and the cost at the root;
-#  parity:    40 per binary64 cost evaluation (23 additions, 15
-#             multiplications, one division, one scaling) x 23 evaluations
-#             per pair (the mean over 20,000 pairs of this workload's
-#             samples) + 20 for the pair's hoisted coefficients, the kernel's
-#             work before its evaluations moved to float-float; now most
-#             evaluations are binary32 arithmetic and the kernel is rated by
-#             instruction issue (below), this figure kept as the
-#             arithmetic a binary64 evaluation would do.
-# the reference's GPU kernel evaluates the same binary64 expression as its
-# CPU build (one cost: 40 operations; topt: 23 cost pairs less the shared ones)
-BVP_FP64_FLOPS_PER_PAIR = {"precision": 28.0, "parity": 40.0 * 23 + 20.0,
-                           "parity_gpu": 40.0 * 23 + 20.0}
+# counts two): ncu's counts of the add, multiply and fused instructions' lanes
+# (smsp__sass_thread_inst_executed_op_d*_pred_on.sum) of one launch, per pair,
+# at N = 4000 (precision: 48,624 + 16,291 + 2 x 81,870 over 15,996,000 pairs)
+# and N = 1000 (parity 18,763 + 25,880 + 2 x 3,235, parity_gpu 24,765 + 7,915
+# + 2 x 38,040 over 999,000).  All three evaluate in float-float on the binary32
+# pipe; binary64 is left for the values whose certificate fails.
+BVP_FP64_FLOPS_PER_PAIR = {"precision": 228655 / 15996000,
+                           "parity": 51113 / 999000,
+                           "parity_gpu": 108760 / 999000}
 # ncu smsp__inst_executed.sum of one parity pair-kernel launch at N = 1000
 # (999,000 pairs), per pair; the same for the reference-GPU arithmetic's
 # pair kernel
-BVP_PARITY_WARP_INST_PER_PAIR = 395849939 / 999000
-BVP_REFGPU_WARP_INST_PER_PAIR = 416223561 / 999000
+BVP_PARITY_WARP_INST_PER_PAIR = 135950305 / 999000
+BVP_REFGPU_WARP_INST_PER_PAIR = 123397391 / 999000
 # The precision kernel is bound by instruction issue, not by one pipe: warp
 # instructions executed per pair on this workload (ncu smsp__inst_executed.sum
 # over one launch of the N = 4000 workload's pair kernel, the one marking the
 # rn superset, / its pairs), and DRAM bytes per launch
 # (dram__bytes_read.sum + dram__bytes_write.sum of the same launch).
-BVP_PRECISION_WARP_INST_PER_PAIR = 703111934 / 15996000
+BVP_PRECISION_WARP_INST_PER_PAIR = 251946845 / 15996000
 # ncu smsp__inst_executed.sum on indoor4000: the edge check (pair-queue
-# kernel) at block size 128, the autotuner's choice there (64 and 256 differ
-# by under 0.3 %), per edge; the waypoint kernel (thread per edge, block size
-# 128), per waypoint
-FREE_EDGES_WARP_INST_PER_EDGE_N4000 = 88103877 / 799800
+# kernel) at block size 256, the autotuner's choice there, per edge; the
+# waypoint kernel (thread per edge, block size 128), per waypoint
+FREE_EDGES_WARP_INST_PER_EDGE_N4000 = 69340262 / 799800
 DISCRETIZE_WARP_INST_PER_WAYPOINT = 18258294 / (799800 * 9)
-BVP_PRECISION_DRAM_BYTES_N4000 = 0.16e6 + 69.18e6
+BVP_PRECISION_DRAM_BYTES_N4000 = 0.17e6 + 68.43e6
 SMSP_PER_SM = 4
 NUM_SMS = 152
 
@@ -875,9 +866,9 @@ def roofline(dom, ks, N, E, M, W, H, P, mode, fp64_tflops, sm_mhz):
     pairs = N * (N - 1)
     t_bvp = ks["bvp_pairs"] / 1e3
     fp64 = BVP_FP64_FLOPS_PER_PAIR[mode] * pairs / t_bvp / 1e12
-    table["bvp_pairs_fp64"] = {"bound": "fp64", "achieved_tflops": round(fp64, 4),
-                               "frac": round(fp64 / fp64_tflops, 4),
-                               "flops_per_pair": BVP_FP64_FLOPS_PER_PAIR[mode]}
+    table["bvp_pairs_fp64"] = {"bound": "fp64", "achieved_tflops": round(fp64, 6),
+                               "frac": round(fp64 / fp64_tflops, 6),
+                               "flops_per_pair": round(BVP_FP64_FLOPS_PER_PAIR[mode], 4)}
     issue_peak = NUM_SMS * SMSP_PER_SM * sm_mhz * 1e6 / 1e9  # warp instructions, G/s
     if mode == "precision" and N == 4000:
         issue = BVP_PRECISION_WARP_INST_PER_PAIR * pairs / t_bvp / 1e9
