@@ -424,7 +424,13 @@ __global__ void __launch_bounds__(kExpThreads) expand_kernel(SearchDev sd, const
 // pass, which prepends its survivors to the stored lists meanwhile: the walk
 // reads the lists through L2 and skips entries stored in this pass (index
 // num_paths or above), so it sees each list as it was when the pass began (a
-// survivor is published only after its link is written).
+// survivor is published only after its link is written).  A walk is a chain of
+// dependent loads from L2 (about 650 cycles each, up to 46 entries in the
+// N = 4000 query): both lists are followed side by side and an entry's link is
+// loaded with its values, which took the whole query from 1.535 to 1.488 ms
+// at N = 4000 and from 1.016 to 1.006 ms at N = 1000.  Four or eight lists per
+// node instead of one, walked together, measured the same, and tiles of 64 or
+// 128 paths within 1 %.
 __device__ __forceinline__ bool dominated_in_store(const SearchDev &sd, int i, int node,
                                                    int num_paths, float eps_cp, float eps_cost) {
   const int path_idx = num_paths + i;
@@ -436,12 +442,22 @@ __device__ __forceinline__ bool dominated_in_store(const SearchDev &sd, int i, i
     }
     return false;
   };
-  for (int c = __ldcg(&sd.node_head[node]); c >= 0; c = __ldcg(&sd.node_next[c])) {
-    if (c >= num_paths) continue;
-    if (dominated_by(sd.path_cp[c], sd.path_cost[c], c)) return true;
+  int a = __ldcg(&sd.node_head[node]), b = sd.new_head[node];
+  while (a >= 0 || b >= 0) {
+    // both lists' entries and links in one round of independent loads; the
+    // place of an ended list, and of an entry of this pass, is taken by path
+    // 0 or i, whose values are not used
+    const bool in_a = a >= 0 && a < num_paths, in_b = b >= 0 && b != i;
+    const int ca = in_a ? a : 0, cb = in_b ? b : i;
+    const int na = a >= 0 ? __ldcg(&sd.node_next[a]) : -1;
+    const int nb = b >= 0 ? sd.new_next[b] : -1;
+    const float a_cp = sd.path_cp[ca], a_cost = sd.path_cost[ca];
+    const float b_cp = sd.new_cp[cb], b_cost = sd.new_cost[cb];
+    if ((in_a && dominated_by(a_cp, a_cost, ca)) || (in_b && dominated_by(b_cp, b_cost, num_paths + cb)))
+      return true;
+    a = na;
+    b = nb;
   }
-  for (int j = sd.new_head[node]; j >= 0; j = sd.new_next[j])
-    if (j != i && dominated_by(sd.new_cp[j], sd.new_cost[j], num_paths + j)) return true;
   return false;
 }
 
