@@ -19,9 +19,9 @@
 // A warp works in two stages, so that its lanes stay together although every
 // bisection has its own length.  Stage A takes 32 pairs, one per lane, and runs
 // the steps the derivative and then the difference settle, which are nearly as
-// many for one pair as for another; the pairs' coefficients and brackets then go to a queue in
-// shared memory.  Stage B runs the remaining steps: a lane whose pair is done
-// stores it and takes the queue's next, once kRefillLanes lanes wait for one.
+// many for one pair as for another; the pairs' coefficients and brackets then
+// go to a queue in shared memory.  Stage B runs the remaining steps: a lane whose pair is done
+// stores it and takes the queue's next, once kBisectRefill lanes wait for one.
 // Every pair walks the same sequence of finite differences as toptBisection.
 //
 // Bound by instruction issue (no DRAM traffic but the results).

@@ -150,9 +150,9 @@ struct ParityCost {
 // All pairs: each warp walks `chunk` consecutive pairs (bisect.cuh).  Bound by
 // instruction issue.  N = 4000 (16 M pairs): 6.11 ms with two float-float costs
 // per finite difference, 3.64 ms with the differences' signs from cost_delta
-// where it settles them, 1.90 ms in two stages with their step limits (about
-// 110 warp instructions a pair; 31 KB of queue a block, 80 registers, 6 blocks
-// an SM).
+// where it settles them, 1.87 ms in two stages with their step limits (31 KB of
+// queue a block, 80 registers, 6 blocks an SM).  N = 1000: 136 warp instructions
+// a pair instead of 396, 20.7 of 32 lanes in use, 78 % of the issue slots.
 __global__ void __launch_bounds__(kBisectThreads, 6) bvp_pairs_parity_persistent(AllPairs src,
                                                                                  int chunk) {
   __shared__ BisectQueue s_queue[kBisectWarps];
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(128) bvp_batch_kernel(const JobPairs src, int 
 // waypoint records it writes.  The block size T (64, 128, 256) is picked by
 // the autotuner.  The bit-exact arithmetics are bound by instruction issue
 // (the 799,800 edges of the N = 4000 query: 524 us with every uncertified
-// waypoint's six states in binary64 by its own lane, 125 us now).
+// waypoint's six states in binary64 by its own lane, 97 us now).
 template <int T>
 size_t discretize_smem(int numDisc) {
   return sizeof(float) * (size_t)T * (numDisc + 1) * kDim;

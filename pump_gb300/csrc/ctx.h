@@ -221,8 +221,8 @@ pump_status_t bvp_pairs_precision_superset(Ctx *ctx, const float *d_samples, int
 // Explicit pairs (x0[k], x1[k]), k < n (x1[0] for every k with x1_same),
 // each bisected for `jobs` (1 or 2)
 // optimal-time limits: job j writes topt[j][k] and cost[j][k] (either may be
-// null).  One thread per (job, pair); small batches use 32-thread blocks so
-// their binary64 bisections spread over more SMs.
+// null).  A warp takes 32 to 1 of the (job, pair) items, fewer the smaller the
+// batch (bisect_jobs_per_warp), so that a small one spreads over the SMs.
 struct BvpJobs {
   const float *x0, *x1;
   int n, jobs;

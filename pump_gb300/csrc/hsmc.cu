@@ -770,12 +770,13 @@ inline const void *hsmc_loop_kernel_for(int P) {
 // Block = 32 K particles (K per lane) of one path x kMcWarps warps, which
 // split the path's segments into consecutive runs (a run carries a segment's
 // end over as the next one's start).  Per segment the warp takes the bounding
-// box of its particles' segments by warp reductions, tests the boxes against it one per lane, and only those that it
-// is not broadphase-disjoint from are tested per particle: a box disjoint
+// box of its particles' segments by warp reductions, tests the boxes against it
+// one per lane, and only those that it is not broadphase-disjoint from are
+// tested per particle: a box disjoint
 // from the common bounding box is disjoint from every particle's, whose
 // reference test then passes.  With a NaN coordinate every box is kept.  (One
 // particle per lane and every box tested by every particle: 268 us for 64
-// paths x 2048 particles and 40 boxes.)  Bound by instruction issue for large
+// paths x 2048 particles and 40 boxes, 45 us so.)  Bound by instruction issue for large
 // calls, by one warp's chain of segments for small ones; hence K: particles
 // per lane share the reductions and box tests of a large call (K = 4), and a
 // small call spreads over the SMs (K = 1).

@@ -20,7 +20,7 @@ namespace pump {
 enum TuneKernel {
   kTuneBvpPairs = 0,   // bvp_pairs_precision_kernel block size
   kTuneDiscretize,     // discretize_kernel block size
-  kTuneFreeEdges,      // free_edges_staged_kernel block size
+  kTuneFreeEdges,      // free_edges_queue_kernel block size
   kTuneCompactRn,      // three-kernel compaction grid: rn superset pass
   kTuneCompactEdges,   // three-kernel compaction grid: edge lists
   kNumTune
