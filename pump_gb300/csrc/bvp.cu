@@ -216,29 +216,17 @@ __device__ __forceinline__ void edge_waypoints_ff(float tau, const float *x0, co
 // item(th, &tau, &numDisc, &x0, &x1, &o): thread th's edge.
 template <int Cap, class Item>
 __device__ __forceinline__ void finish_path_queue(const PathQueue<Cap> &queue, Item item) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  int task = 0;
-  auto run = [&](auto kind) {
+  queue.drain([&](auto kind, int th, int i, int a) {
     constexpr int Kind = decltype(kind)::value;
-    const int n = queue.n[Kind] < Cap ? queue.n[Kind] : Cap;
-    for (int q0 = 0; q0 < n; q0 += 32, ++task) {
-      if (task % warps != warp || q0 + lane >= n) continue;
-      const unsigned ent = queue.e[Kind][q0 + lane];
-      const int th = (int)(ent >> 20), i = (int)((ent >> 2) & 0x3ffffu), a = (int)(ent & 3u);
-      float tau;
-      int numDisc;
-      const float *x0, *x1;
-      float *o;
-      item(th, &tau, &numDisc, &x0, &x1, &o);
-      const float dt = tau / numDisc;
-      o[i * kDim + a + (Kind == kPathXY || Kind == kPathZ ? 0 : 3)] = path_state64<Kind>(
-          dt * i, tau, __ldg(x0 + a), __ldg(x0 + a + 3), __ldg(x1 + a), __ldg(x1 + a + 3));
-    }
-  };
-  run(std::integral_constant<int, kPathXY>{});
-  run(std::integral_constant<int, kPathVXY>{});
-  run(std::integral_constant<int, kPathZ>{});
-  run(std::integral_constant<int, kPathVZ>{});
+    float tau;
+    int numDisc;
+    const float *x0, *x1;
+    float *o;
+    item(th, &tau, &numDisc, &x0, &x1, &o);
+    const float dt = tau / numDisc;
+    o[i * kDim + a + (Kind == kPathXY || Kind == kPathZ ? 0 : 3)] = path_state64<Kind>(
+        dt * i, tau, __ldg(x0 + a), __ldg(x0 + a + 3), __ldg(x1 + a), __ldg(x1 + a + 3));
+  });
 }
 
 template <int Mode, int T>
@@ -520,7 +508,12 @@ __global__ void path_states_kernel(const float *__restrict__ xs, const int *__re
 // p * rows_cap (rows at or past rows_cap are not written); a row's segment
 // is the last one of the path whose first row is at or before it (segments
 // with no samples share their first row with the next).  The precision mode
-// evaluates the cubic in binary32, as its edge waypoints do.
+// evaluates the cubic in binary32, as its edge waypoints do.  The bit-exact
+// arithmetic leaves its uncertified states to the block's queue, which its
+// warps empty a kind each, side by side: a launch is a few rows per thread and
+// bound by latency, and a warp that evaluated its own such states one after
+// the other held it (8 paths through pump_path_cp 68.2 us, 63.1 so; the query at
+// N = 1000 with its 8 candidate batches 1.022 and 0.989 ms).
 constexpr int kRowThreads = 128;
 
 template <int Mode>
@@ -532,6 +525,11 @@ __global__ void __launch_bounds__(kRowThreads) candidate_rows_kernel(
     unsigned int *done, int preload) {
   extern __shared__ int s_seg[];  // per segment: first row, toff; with preload, time and cost
   __shared__ int s_len;
+  constexpr bool Parity = Mode == PUMP_BVP_PARITY;
+  // the block's uncertified states of a pass, with their rows' times and segments
+  __shared__ PathQueue<Parity ? kRowThreads : 1> s_queue;
+  __shared__ float s_time[Parity ? kRowThreads : 1];
+  __shared__ int s_lo[Parity ? kRowThreads : 1];
   const int p = blockIdx.x;
   const int n = node_cnt[p], b = seg_base[p], ns = n > 1 ? n - 1 : 0;
   int *srow = s_seg;
@@ -573,24 +571,55 @@ __global__ void __launch_bounds__(kRowThreads) candidate_rows_kernel(
   __syncthreads();
   if (ns == 0) return;
   const int L = s_len < rows_cap ? s_len : rows_cap;
-  for (int r = blockIdx.y * kRowThreads + threadIdx.x; r < L; r += gridDim.y * kRowThreads) {
-    int lo = 0, hi = ns - 1;  // segments b + lo .. b + hi
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (srow[mid] <= r) lo = mid; else hi = mid - 1;
+  for (int r0 = blockIdx.y * kRowThreads; r0 < L; r0 += gridDim.y * kRowThreads) {  // block-uniform
+    const int r = r0 + threadIdx.x;
+    if (Parity) {
+      s_queue.clear();
+      __syncthreads();
     }
-    const int s = b + lo, k = r - srow[lo];
-    float a[kDim], c[kDim], x[kDim];
+    if (r < L) {
+      int lo = 0, hi = ns - 1;  // segments b + lo .. b + hi
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (srow[mid] <= r) lo = mid; else hi = mid - 1;
+      }
+      const int s = b + lo, k = r - srow[lo];
+      float a[kDim], c[kDim], x[kDim];
 #pragma unroll
-    for (int d = 0; d < kDim; ++d) {
-      a[d] = x0[s * kDim + d];
-      c[d] = x1[s * kDim + d];
+      for (int d = 0; d < kDim; ++d) {
+        a[d] = x0[s * kDim + d];
+        c[d] = x1[s * kDim + d];
+      }
+      const float t = dt * k + stoff[lo], tau = stime[lo];
+      unsigned bad = 0u;
+      if (Parity) {
+        bad = path_point_try(t, tau, a, c, path_ff_edge(tau, a, c), x);
+        if (bad) s_time[threadIdx.x] = t, s_lo[threadIdx.x] = lo;
+      } else {
+        path_point_f32(t, tau, a, c, x);
+      }
+      float *o = states + ((long long)p * rows_cap + r) * kDim;
+#pragma unroll
+      for (int d = 0; d < kDim; ++d) {
+        const int q = d < 3 ? d : d - 3;
+        // (a queued state is written from the queue)
+        if (!((bad >> d) & 1u)) o[d] = x[d];
+        else if (!s_queue.push(threadIdx.x, 0, d))
+          o[d] = path_state_now(d, t, tau, a[q], a[q + 3], c[q], c[q + 3]);
+      }
     }
-    if (Mode == PUMP_BVP_PARITY) path_point_fast(dt * k + stoff[lo], stime[lo], a, c, x);
-    else path_point_f32(dt * k + stoff[lo], stime[lo], a, c, x);
-    const long long t = (long long)p * rows_cap + r;
-#pragma unroll
-    for (int d = 0; d < kDim; ++d) states[t * kDim + d] = x[d];
+    if (Parity) {
+      __syncthreads();
+      s_queue.drain([&](auto kind, int th, int, int axis) {
+        constexpr int Kind = decltype(kind)::value;
+        const int lo = s_lo[th];
+        const float *e0 = x0 + (b + lo) * kDim + axis, *e1 = x1 + (b + lo) * kDim + axis;
+        states[((long long)p * rows_cap + r0 + th) * kDim + axis +
+               (Kind == kPathXY || Kind == kPathZ ? 0 : 3)] =
+            path_state64<Kind>(s_time[th], stime[lo], __ldg(e0), __ldg(e0 + 3), __ldg(e1), __ldg(e1 + 3));
+      });
+      __syncthreads();  // the queue is reused
+    }
   }
 }
 

@@ -222,7 +222,7 @@ __device__ __forceinline__ void path_point_fast(float t, float tau, const float 
   }
 }
 
-// The waypoint kernels' queue of states left for binary64, shared by a block:
+// The waypoint and dense-path kernels' queue of states left for binary64, shared by a block:
 // (thread, waypoint, axis) entries in one list per kind, so that a warp then
 // evaluates 32 of one kind at once (binary64 instructions occupy this GPU's
 // binary64 pipe for the same time for one lane as for 32; one state in about
@@ -243,6 +243,26 @@ struct PathQueue {
     if (at >= Cap) return false;
     e[kind][at] = ((unsigned)th << 20) | ((unsigned)i << 2) | (unsigned)axis;
     return true;
+  }
+  // state(kind, th, i, axis) for every entry, 32 of a kind per warp; call after
+  // a barrier
+  template <class State>
+  __device__ __forceinline__ void drain(State state) const {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    int task = 0;
+    auto run = [&](auto kind) {
+      constexpr int Kind = decltype(kind)::value;
+      const int cnt = n[Kind] < Cap ? n[Kind] : Cap;
+      for (int q0 = 0; q0 < cnt; q0 += 32, ++task) {
+        if (task % warps != warp || q0 + lane >= cnt) continue;
+        const unsigned ent = e[Kind][q0 + lane];
+        state(kind, (int)(ent >> 20), (int)((ent >> 2) & 0x3ffffu), (int)(ent & 3u));
+      }
+    };
+    run(std::integral_constant<int, kPathXY>{});
+    run(std::integral_constant<int, kPathVXY>{});
+    run(std::integral_constant<int, kPathZ>{});
+    run(std::integral_constant<int, kPathVZ>{});
   }
 };
 

@@ -233,3 +233,33 @@ def test_path_cp_first_path_many_calls(gpu, pumplib, oracle):
             ln.ctypes.data, None))
         c64, _, _ = oracle.path_cp(nodes[:cnts[0]], pm, np.float32(0.2), obs)
         assert np.float32(cp[0]) == np.float32(c64), call
+
+
+@pytest.mark.parametrize("zero", [(), (1,), (0, 1), (2,)])
+def test_path_cp_rows_left_for_binary64(gpu, pumplib, oracle, zero):
+    """Dense paths of more rows than a block takes at once, with coordinates
+    that are 0 throughout: every such state is left for binary64, up to twice
+    as many of a kind in a block as its queue holds."""
+    torch, ctx = gpu
+    tm, pm = oracle.particle_tables(P=2048, T=400)
+    rng = np.random.default_rng(12)
+    nodes = np.zeros((41, 6), np.float32)
+    nodes[:, :3] = np.linspace(0.0, 4.0, 41)[:, None] + rng.uniform(-0.02, 0.02, (41, 3))
+    nodes[:, 3:] = rng.uniform(0.2, 0.4, (41, 3))
+    for d in zero:
+        nodes[:, d] = nodes[:, d + 3] = 0.0
+    side = rng.uniform(0.07, 0.2, (20, 3)) * np.array([1.0, -1.0, 1.0])
+    c = nodes[rng.integers(1, 40, 20), :3] + side
+    obs = np.zeros((20, 12), np.float32)
+    obs[:, :3], obs[:, 6:9] = c - 0.03, c + 0.03
+    obs[:, 3:6], obs[:, 9:] = -3.1, 3.1
+    d_tm, d_obs = dev(torch, tm), dev(torch, obs)
+    offs, cnts = np.zeros(1, np.int32), np.full(1, 41, np.int32)
+    cp, cost, ln = np.zeros(1, np.float32), np.zeros(1, np.float32), np.zeros(1, np.int32)
+    pumplib.check(pumplib.load().pump_path_cp(
+        ctx.handle, nodes.ctypes.data, offs.ctypes.data, cnts.ctypes.data, 1, pumplib.PUMP_BVP_PARITY,
+        ptr(d_tm), 2048, 400, 1.0, ptr(d_obs), obs.shape[0], cp.ctypes.data, cost.ctypes.data,
+        ln.ctypes.data, None))
+    c64, cost64, len64 = oracle.path_cp(nodes, pm, np.float32(1.0), obs)
+    assert 128 < ln[0] <= 400 and ln[0] == len64 and 0.0 < c64 < 1.0
+    assert np.float32(cp[0]) == np.float32(c64) and np.float32(cost[0]) == np.float32(cost64)
