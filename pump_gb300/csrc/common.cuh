@@ -95,15 +95,17 @@ __device__ __forceinline__ void warp_store(float *__restrict__ dst, const float 
   }
 }
 
-// Least and greatest value of a warp (a NaN is passed over).
+// Least and greatest value of a warp (a NaN is passed over).  Volatile: every
+// lane of the warp takes part, and an asm that is not may be moved to where its
+// value is used, a place that only some of the lanes reach.
 __device__ __forceinline__ float warp_min_f32(float x) {
   float y;
-  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
   return y;
 }
 __device__ __forceinline__ float warp_max_f32(float x) {
   float y;
-  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
   return y;
 }
 
