@@ -14,16 +14,17 @@
 // the table is bit-identical on any IEEE machine that does not contract
 // multiply-adds.
 //
-// HSMC.  One block per new path, threads over particles.  The half-spaces of
-// a waypoint are the same for every particle of the path, so each test is a
-// block-uniform branch on b >= 1000 followed by a 3-term dot product against
-// the particle's offset row; offsets are read time-major so a warp reads 32
-// consecutive particles (384 contiguous bytes).  Validity is kept as a bit
-// per particle (__ballot_sync), and the hit count of calculateCP_HSMC is the
-// block's popcount sum, so the CP needs no second pass over a byte array.
+// HSMC.  One warp per new path, its lanes over quads of particles.  The
+// half-spaces of a waypoint are the same for every particle of the path, so the
+// warp tests up to five of them at once on each quad that it loads; offsets are
+// read time-major, 128 consecutive particles a step.  Validity is kept as a bit
+// per particle, in registers, and the hit count of calculateCP_HSMC is the
+// warp's popcount sum, so the CP needs no second pass.
 //
-// Monte Carlo CP.  Thread per (particle, path) over many paths per launch;
-// obstacles staged in shared memory; the same segment test as freeEdges.
+// Monte Carlo CP.  A block takes 32 or 128 particles of one path, its 16 warps
+// consecutive runs of the path's segments; obstacles staged in shared memory,
+// those that no particle of a warp comes near dropped per segment; the same
+// segment test as freeEdges.
 #include <math.h>
 
 #include <type_traits>
@@ -187,10 +188,17 @@ __global__ void position_variance_kernel(int T, double *__restrict__ var) {
 // ------------------------------------------------------------------ HSMC
 // One warp per new path.  Lane l owns particles 128 c + 4 l + j (j < 4), one
 // bit each, so the offsets of a c-step are 128 consecutive particles, three
-// 16-byte loads a lane (12-byte records of 32 particles, three 4-byte loads:
-// 311 us for 12,000 paths x 1024 particles with about 38 active half-spaces a
-// path; 155 us so, with up to five half-spaces of a waypoint tested on each
-// loaded particle and the comparison's product folded into its bound).  Such
+// 16-byte loads a lane.  (12-byte records of 32 particles, three 4-byte loads
+// each: 311 us for 12,000 paths x 1024 particles with about 38 active half-spaces
+// a path; 154 us so, with up to five half-spaces of a waypoint tested on each
+// loaded particle and the comparison's product folded into its bound.)  A table
+// whose rows are not whole 16-byte quads (Pmc not a multiple of four) is read 32
+// consecutive records at a time, and a lane's particles are 128 c + 32 j + l.
+// The loop over groups of 1024 particles is rolled (the group's bits selected by
+// its number): six instantiations of the test, twenty-four with it unrolled at
+// 4096 particles, do not stay in the instruction cache (100,000 paths x 4096
+// particles, 100 boxes: 4.8 ms with 4-byte loads, 8.5 ms with quads and that
+// loop unrolled, 2.9 ms so; 12,000 paths x 1024 particles the same).  Such large
 // wavefronts are bound by instruction issue.  The warp first finds the edge's W x H
 // half-space slots that are active (the reference skips a half-space when
 // b >= 1000, PUMP.cu:642); with none active the new mask is the parent's and
@@ -233,10 +241,11 @@ inline unsigned hsmc_blocks(long long n) {
   const long long want = (n + kHsmcWarps - 1) / kHsmcWarps;
   return (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks);
 }
-// Half-spaces of one waypoint tested on each loaded quad of particles (12,000
-// paths, about 38 active half-spaces each: 225 us with 2, 194 with 3 or 4, 167
-// with 5, the reference's limit; the quads' loop is not unrolled: 224 us with
-// two quads in flight, whose code is twice as long).
+// Half-spaces of one waypoint tested on each loaded quad of particles, 5 being
+// the reference's limit (12,000 paths, about 38 active half-spaces each, event
+// times of the step that chose it: 230 us with 2, 194 with 3 or 4, 167 with 5; the
+// quads' loop is not unrolled: 224 us with two quads in flight, whose code is
+// twice as long).
 constexpr int kHsmcGroup = 5;
 constexpr int kHsmcFilterObs = 128;
 
@@ -274,6 +283,20 @@ __device__ __forceinline__ bool hsmc_lhs_bound(float b, float om, float *bound) 
   return __uint_as_float(u) * om < b && !(__uint_as_float(u + 1u) * om < b);
 }
 
+// Bit b of lane l <-> bit l of lane b: halves of the 32 x 32 matrix exchanged,
+// then halves of those.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x) {
+  const int lane = threadIdx.x & 31;
+  uint32_t m = 0x0000ffffu;  // the bits whose number does not have s
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
+    x = (lane & s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y & m) << s);
+    m ^= m << (s >> 1);
+  }
+  return x;
+}
+
 // New path w (the whole warp).  valid_in[prev] is read, valid_out[w] /
 // cp_out[w] written (the two may alias one path store with valid_out =
 // store + base, as in the reference).  With hs_count (stored half-spaces per
@@ -302,16 +325,17 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
     }
     W = (int)n;
   }
-  // the epilogue's inputs, on their way while the path is propagated
-  float epi_time = 0.0f, epi_topt = 0.0f, epi_cost = 0.0f, epi_copt = 0.0f;
-  int epi_node = 0;
-  if (Epi && lane == 0) {
+  // the epilogue's inputs, one per lane, on their way while the path is
+  // propagated
+  uint32_t epi = 0u;
+  if (Epi && lane < 5) {
     const HsmcEpilogue &e = p.epi;
-    epi_time = e.path_time[prev];
-    epi_topt = __ldg(&e.topt[edge]);
-    epi_cost = e.path_cost[prev];
-    epi_copt = __ldg(&e.copt[edge]);
-    epi_node = e.wf_node[w];
+    const void *src = lane == 0   ? (const void *)&e.path_time[prev]
+                      : lane == 1 ? (const void *)&e.topt[edge]
+                      : lane == 2 ? (const void *)&e.path_cost[prev]
+                      : lane == 3 ? (const void *)&e.copt[edge]
+                                  : (const void *)&e.wf_node[w];
+    epi = *reinterpret_cast<const uint32_t *>(src);
   }
   const int maxHS = p.maxHS, P = p.P;
   const int words = (P + 31) >> 5;
@@ -422,22 +446,30 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
   }
   int overflow = 0;
   if (__any_sync(0xffffffffu, act != 0u)) {
+    // 16-byte loads need whole quads of particles in a table row; other tables
+    // are read 32 consecutive 12-byte records at a time, and the lane's four
+    // particles are 32 apart instead of consecutive (launch-uniform)
+    const bool vec = (p.Pmc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.offsets_t) & 15) == 0;
     // unpack: bit 4 c + j of bits[q] = particle 1024 q + 128 c + 4 lane + j,
-    // from word 32 q + 4 c + lane / 8 of the mask
+    // from word 32 q + 4 c + lane / 8 of the mask (without vec: particle 1024 q
+    // + 128 c + 32 j + lane, from word 32 q + 4 c + j)
     uint32_t bits[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       bits[q] = 0u;
+      if (q * 1024 >= P) break;
+      if (vec) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (q * 1024 + c * 128 >= P) break;
-        const uint32_t wk = __shfl_sync(0xffffffffu, mine[q], 4 * c + (lane >> 3));
-        bits[q] |= ((wk >> (4 * (lane & 7))) & 0xFu) << (4 * c);
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t wk = __shfl_sync(0xffffffffu, mine[q], 4 * c + (lane >> 3));
+          bits[q] |= ((wk >> (4 * (lane & 7))) & 0xFu) << (4 * c);
+        }
+      } else {
+        bits[q] = warp_transpose_bits(mine[q]);
       }
     }
     const float dtLocal = p.topts[edge] / (W - 1);
     const float t0 = p.times[prev];
-    const bool vec = (p.Pmc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.offsets_t) & 15) == 0;
     // slot sidx: its half-space and its bound on the offset's projection
     auto half_space = [&](int sidx, float (&h)[4]) {
       if (Boxes) {
@@ -456,35 +488,44 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
     // particle: dead unless fl(LHS * offset_mult) < b.  Bounded: h[n][3] is the
     // largest LHS that passes (hsmc_lhs_bound), which saves the product.  The
     // tests of a particle already dead are computed and discarded, so the loads
-    // do not wait on the bits.
+    // do not wait on the bits.  A single half-space leaves registers to load the
+    // next quad before this one is tested (200 paths x 4096 particles, 10 boxes:
+    // 40 us without, 34 so; with two half-spaces the same and slower for larger
+    // wavefronts).
     auto test = [&](const float *row, auto count, auto bounded, const float (&h)[kHsmcGroup][4]) {
       constexpr int N = decltype(count)::value;
       constexpr bool Bounded = decltype(bounded)::value;
+      constexpr bool Ahead = Bounded && N == 1;
+      // the quad at 128 c of group q (past the last particle: the row's end,
+      // whose bits are dropped)
+      auto load = [&](int at, float (&o)[4][3]) {
+        if (vec) {
+          const int p0 = at + 4 * lane < p.Pmc ? at + 4 * lane : p.Pmc - 4;
+          const float4 *r4 = reinterpret_cast<const float4 *>(row + p0 * 3);
+          const float4 x = __ldg(r4), y = __ldg(r4 + 1), z = __ldg(r4 + 2);
+          o[0][0] = x.x; o[0][1] = x.y; o[0][2] = x.z;
+          o[1][0] = x.w; o[1][1] = y.x; o[1][2] = y.y;
+          o[2][0] = y.z; o[2][1] = y.w; o[2][2] = z.x;
+          o[3][0] = z.y; o[3][1] = z.z; o[3][2] = z.w;
+        } else {
 #pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int pp = at + 32 * j + lane < p.Pmc ? at + 32 * j + lane : p.Pmc - 1;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[j][d] = __ldg(&row[pp * 3 + d]);
+          }
+        }
+      };
+#pragma unroll 1
       for (int q = 0; q < Q; ++q) {
         if (q * 1024 >= P) break;
-        uint32_t bq = bits[q];
+        uint32_t bq = bits[0];
+#pragma unroll
+        for (int k = 1; k < Q; ++k)
+          if (q == k) bq = bits[k];
         if (bq == 0u) continue;  // this lane's particles of the group are all dead
-#pragma unroll 1
-        for (int c = 0; c < 8; ++c) {
-          const int p0 = q * 1024 + c * 128 + 4 * lane;
-          if (p0 >= P) continue;
-          float o[4][3];
-          if (vec) {
-            const float4 *r4 = reinterpret_cast<const float4 *>(row + (long long)p0 * 3);
-            const float4 x = __ldg(r4), y = __ldg(r4 + 1), z = __ldg(r4 + 2);
-            o[0][0] = x.x; o[0][1] = x.y; o[0][2] = x.z;
-            o[1][0] = x.w; o[1][1] = y.x; o[1][2] = y.y;
-            o[2][0] = y.z; o[2][1] = y.w; o[2][2] = z.x;
-            o[3][0] = z.y; o[3][1] = z.z; o[3][2] = z.w;
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int pp = p0 + j < p.Pmc ? p0 + j : p.Pmc - 1;
-#pragma unroll
-              for (int d = 0; d < 3; ++d) o[j][d] = __ldg(&row[(long long)pp * 3 + d]);
-            }
-          }
+        const int end = P - q * 1024 < 1024 ? P - q * 1024 : 1024;
+        auto judge = [&](int c, const float (&o)[4][3]) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             bool pass = true;
@@ -496,13 +537,34 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
             }
             if (!pass) bq &= ~(1u << (4 * c + j));
           }
+        };
+        float o[4][3];
+        if (Ahead && vec) {
+          float next[4][3];
+          load(q * 1024, o);
+#pragma unroll 1
+          for (int c = 0; c * 128 < end; ++c) {
+            load(q * 1024 + (c + 1) * 128, next);
+            judge(c, o);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int d = 0; d < 3; ++d) o[j][d] = next[j][d];
+          }
+        } else {
+#pragma unroll 1
+          for (int c = 0; c * 128 < end; ++c) {
+            load(q * 1024 + c * 128, o);
+            judge(c, o);
+          }
         }
-        bits[q] = bq;
+#pragma unroll
+        for (int k = 0; k < Q; ++k)
+          if (q == k) bits[k] = bq;
       }
     };
     for (int c = 0; c * 32 < slots; ++c) {
-      const uint32_t act_word = __shfl_sync(0xffffffffu, act, c);
-      uint32_t m = act_word;
+      uint32_t m = __shfl_sync(0xffffffffu, act, c);
       // lane l: the bound of slot 32 c + l
       float lhs_bound = 0.0f;
       bool exact = false;
@@ -538,41 +600,42 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
         }
         if (!bounded) {
           // (rare: the bounds of the group's others are dropped again)
-          uint32_t back = 0u;
-          int at = sidx & 31;
-          for (int n = 0; n < group; ++n) {
-            float one[kHsmcGroup][4];
-            half_space(c * 32 + at, one[0]);
-            test(row, std::integral_constant<int, 1>{}, std::false_type{}, one);
-            back = act_word & ~((2u << at) - 1u);
-            at = back ? __ffs(back) - 1 : 0;
+          uint32_t back = __shfl_sync(0xffffffffu, act, c) & ~m & ~((1u << (sidx & 31)) - 1u);
+          for (; back; back &= back - 1u) {
+            half_space(c * 32 + __ffs(back) - 1, h[0]);
+            test(row, std::integral_constant<int, 1>{}, std::false_type{}, h);
           }
         } else if (group == 1) {
           test(row, std::integral_constant<int, 1>{}, std::true_type{}, h);
         } else if (group == 2) {
           test(row, std::integral_constant<int, 2>{}, std::true_type{}, h);
         } else if (group == 3) {
-          test(row, std::integral_constant<int, kHsmcGroup < 3 ? 1 : 3>{}, std::true_type{}, h);
+          test(row, std::integral_constant<int, 3>{}, std::true_type{}, h);
         } else if (group == 4) {
-          test(row, std::integral_constant<int, kHsmcGroup < 4 ? 1 : 4>{}, std::true_type{}, h);
+          test(row, std::integral_constant<int, 4>{}, std::true_type{}, h);
         } else {
-          test(row, std::integral_constant<int, kHsmcGroup < 5 ? 1 : 5>{}, std::true_type{}, h);
+          test(row, std::integral_constant<int, 5>{}, std::true_type{}, h);
         }
       }
     }
-    // repack: an octet's nibbles form word 4 c + lane / 8; lane j keeps word j
+    // repack: an octet's nibbles form word 4 c + lane / 8 (without vec, the
+    // lanes' bits b word b); lane j keeps word j
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
+      if (q * 1024 >= P) break;
       uint32_t keep = 0u;
+      if (vec) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (q * 1024 + c * 128 >= P) break;
-        uint32_t v = ((bits[q] >> (4 * c)) & 0xFu) << (4 * (lane & 7));
-        v |= __shfl_xor_sync(0xffffffffu, v, 1);
-        v |= __shfl_xor_sync(0xffffffffu, v, 2);
-        v |= __shfl_xor_sync(0xffffffffu, v, 4);
-        v = __shfl_sync(0xffffffffu, v, 8 * (lane & 3));
-        if ((lane >> 2) == c) keep = v;
+        for (int c = 0; c < 8; ++c) {
+          uint32_t v = ((bits[q] >> (4 * c)) & 0xFu) << (4 * (lane & 7));
+          v |= __shfl_xor_sync(0xffffffffu, v, 1);
+          v |= __shfl_xor_sync(0xffffffffu, v, 2);
+          v |= __shfl_xor_sync(0xffffffffu, v, 4);
+          v = __shfl_sync(0xffffffffu, v, 8 * (lane & 3));
+          if ((lane >> 2) == c) keep = v;
+        }
+      } else {
+        keep = warp_transpose_bits(bits[q]);
       }
       mine[q] = keep;
     }
@@ -589,18 +652,25 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
     }
   }
   valid_count = __reduce_add_sync(0xffffffffu, valid_count);
+  const float cp = ((float)(P - valid_count)) / P;
   if (lane == 0) {
-    const float cp = ((float)(P - valid_count)) / P;
     p.cp_out[w] = cp;
     if (overflow && p.error) atomicExch(p.error, (int)PUMP_ERR_CAPACITY);
-    if (Epi) {
-      // PUMP.cu:164-185: time, cost and the CP cut-off of new path w
+  }
+  if (Epi) {
+    // PUMP.cu:164-185: time, cost and the CP cut-off of new path w
+    const float time = __uint_as_float(__shfl_sync(0xffffffffu, epi, 0));
+    const float topt = __uint_as_float(__shfl_sync(0xffffffffu, epi, 1));
+    const float cost = __uint_as_float(__shfl_sync(0xffffffffu, epi, 2));
+    const float copt = __uint_as_float(__shfl_sync(0xffffffffu, epi, 3));
+    const int node = (int)__shfl_sync(0xffffffffu, epi, 4);
+    if (lane == 0) {
       const HsmcEpilogue &e = p.epi;
-      e.new_time[w] = epi_time + epi_topt;
-      e.new_cost[w] = epi_cost + epi_copt;
+      e.new_time[w] = time + topt;
+      e.new_cost[w] = cost + copt;
       const bool alive = !(cp > e.cp_cutoff);
       e.alive[w] = alive ? 1 : 0;
-      if (alive) e.new_next[w] = atomicExch(&e.new_head[epi_node], w);
+      if (alive) e.new_next[w] = atomicExch(&e.new_head[node], w);
     }
   }
 }
@@ -608,8 +678,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
 // The chunk's paths base .. base + cnt - 1 by the block's warps, each taking
 // the next path from the block's counter when it is free.  (Taking the next
 // path ahead, to load its edge and parent during the one before, lets a warp
-// with a long path hold back another: 221 instead of 197 us for 12,000 such
-// paths.)
+// with a long path hold back another: 12 % more for 12,000 such paths.)
 template <bool Boxes, int Q, bool Epi>
 __device__ __forceinline__ void hsmc_chunk_paths(const HsmcParams &p, int base, int cnt, int *s_next,
                                                  const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
@@ -671,6 +740,15 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_kernel(const HsmcParams 
 // when its next chunk belongs to another query.  The shared memory holds the
 // layout of the group's largest box count, waypoint count and half-space
 // count.
+// Out of line: the loop kernel's own state is saved once per chunk, not spilled
+// around the tests (N = 32000, 4096 particles: the whole query 266 ms inlined,
+// 247 so).
+template <int Q>
+__device__ __noinline__ void hsmc_loop_paths(const HsmcParams &p, int base, int cnt, int *s_next,
+                                             const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
+  hsmc_chunk_paths<true, Q, true>(p, base, cnt, s_next, s_obs, hs, hcnt, klist);
+}
+
 template <int Q>
 __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGroup *g) {
   extern __shared__ float4 s_dyn4[];
@@ -725,7 +803,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
     }
     if (threadIdx.x == 0) s_next = 0;
     __syncthreads();
-    const HsmcParams p = s_p;
+    const HsmcParams &p = s_p;
     // this query's layout of the shared memory
     const int hs_stride = hsmc_hs_stride(p.W, p.maxHS), cnt_stride = hsmc_cnt_stride(p.W);
     float4 *s_hs = reinterpret_cast<float4 *>(s_obs + hsmc_boxes_obs_floats(p.numObs));
@@ -735,7 +813,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
     const int chunk = hsmc_chunk(n, share);
     const int base = (ch - s_first[q]) * chunk;
     const int cnt = n - base < chunk ? n - base : chunk;
-    hsmc_chunk_paths<true, Q, true>(p, base, cnt, &s_next, s_obs, s_hs + warp * hs_stride,
+    hsmc_loop_paths<Q>(p, base, cnt, &s_next, s_obs, s_hs + warp * hs_stride,
                               s_cnt + warp * cnt_stride, s_klist + warp * kHsmcFilterObs);
   }
 }

@@ -753,6 +753,16 @@ def test_hsmc_particle_quads(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap100
         assert int(host(d_err)[0]) == 0
 
 
+@pytest.mark.parametrize("om", [0.3, 0.0])
+@pytest.mark.parametrize("P,Pmc,n_new", [(4096, 4096, 60), (3073, 4096, 300), (2049, 2052, 700), (1024, 2048, 300),
+                                         (3000, 3001, 100), (2100, 2101, 100), (31, 33, 200), (4, 4, 40)])
+def test_hsmc_particle_rows(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap1000):
+    """Table rows of whole quads at one, two and four words a lane, ended inside
+    a group of 1024 particles and at its edge, and ragged rows, whose particles
+    lie 32 apart in a lane (their bits transposed)."""
+    test_hsmc_particle_quads(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap1000)
+
+
 def test_hsmc_device_checks(gpu, pumplib, oracle, roadmap1000):
     """HSMC's device-side checks: an edge index outside [0, E) and a parent
     outside [0, base) skip their paths and record PUMP_ERR_BAD_INPUT; a time
