@@ -224,22 +224,30 @@ constexpr int kHsmcThreads = 128;
 constexpr int kHsmcWarps = kHsmcThreads / 32;
 // blocks of a launch that loops over a device-side path count
 constexpr int kHsmcPersistBlocks = kNumSMs * 8;
-// Paths per block chunk of a wavefront of n paths on `blocks` resident blocks:
-// a block's warps take the chunk's paths one at a time from a shared-memory
-// counter, so a warp whose paths are cheap (no active half-space: the parent's
-// masks copied) takes more of them while another tests particles.  One path
-// per warp while that fits the blocks (a small wavefront spreads over every
-// warp); then one chunk per block, up to 16 paths (no second, nearly empty
-// round: 12,000 paths in chunks of 8 were 1.23 rounds of 1,216 blocks); then
-// rounds of 16 or more.
-__host__ __device__ inline int hsmc_chunk(long long n, long long blocks) {
-  const long long rounds = n / (16 * blocks) > 1 ? n / (16 * blocks) : 1;
-  const long long c = (n + blocks * rounds - 1) / (blocks * rounds);
-  return c > kHsmcWarps ? (int)c : kHsmcWarps;
+// A wavefront's paths are dealt to the blocks: a block's warps take its paths one
+// at a time from a shared-memory counter, so a warp whose paths are cheap (no
+// active half-space: the parent's masks copied) takes more of them while another
+// tests particles.  One path per warp while that fits the resident blocks (a
+// small wavefront spreads over every warp).  Then block k of b takes the paths k,
+// k + b, k + 2 b, ...: every block has the same number, whatever n is, and waits
+// for its slowest warp once.  (Chunks of 8 consecutive paths took 12,000 paths 1.23
+// rounds of the 1,216 blocks; chunks of 16 or 17 taken in turn left one warp of four
+// idle for a round in five.)  From 16 paths a block on, if the host knows n, there
+// are more blocks than resident ones, of kHsmcRun consecutive paths each, because
+// some SMs run them faster (100,000 paths x 1024 particles near 200 boxes: 770 us
+// in such blocks, 870 dealt to 1,216, 950 in chunks of 17).
+constexpr int kHsmcRun = 8;
+constexpr int kHsmcDealt = 16;
+// Queries that share a launch take chunks of at most 16 paths, four a warp, so
+// that the larger ones' spread over all of its blocks.
+__host__ __device__ inline int hsmc_chunks(long long n, long long blocks, bool alone) {
+  const long long single = (n + kHsmcWarps - 1) / kHsmcWarps;
+  if (single <= blocks) return (int)single;
+  return (int)(alone || n <= kHsmcDealt * blocks ? blocks : (n + kHsmcDealt - 1) / kHsmcDealt);
 }
-inline unsigned hsmc_blocks(long long n) {
-  const long long want = (n + kHsmcWarps - 1) / kHsmcWarps;
-  return (unsigned)(want < kHsmcPersistBlocks ? want : kHsmcPersistBlocks);
+inline unsigned hsmc_blocks(long long n, bool device_count) {
+  if (!device_count && n > (long long)kHsmcDealt * kHsmcPersistBlocks) return (unsigned)((n + kHsmcRun - 1) / kHsmcRun);
+  return (unsigned)hsmc_chunks(n, kHsmcPersistBlocks, true);
 }
 // Half-spaces of one waypoint tested on each loaded quad of particles, 5 being
 // the reference's limit (12,000 paths, about 38 active half-spaces each, event
@@ -675,19 +683,19 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
   }
 }
 
-// The chunk's paths base .. base + cnt - 1 by the block's warps, each taking
-// the next path from the block's counter when it is free.  (Taking the next
+// The chunk's paths, every step-th one below n from the block's counter on, by
+// its warps, each taking the next one when it is free.  (Taking the next
 // path ahead, to load its edge and parent during the one before, lets a warp
 // with a long path hold back another: 12 % more for 12,000 such paths.)
 template <bool Boxes, int Q, bool Epi>
-__device__ __forceinline__ void hsmc_chunk_paths(const HsmcParams &p, int base, int cnt, int *s_next,
+__device__ __forceinline__ void hsmc_chunk_paths(const HsmcParams &p, unsigned step, int n, unsigned *s_next,
                                                  const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
   while (true) {
-    int t = 0;
-    if ((threadIdx.x & 31) == 0) t = atomicAdd(s_next, 1);
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= cnt) break;  // warp-uniform
-    hsmc_path<Boxes, Q, Epi>(p, base + t, p.wf_edge[base + t], p.wf_prev[base + t], s_obs, hs, hcnt, klist);
+    unsigned w = 0u;
+    if ((threadIdx.x & 31) == 0) w = atomicAdd(s_next, step);
+    w = __shfl_sync(0xffffffffu, w, 0);
+    if (w >= (unsigned)n) break;  // warp-uniform
+    hsmc_path<Boxes, Q, Epi>(p, (int)w, p.wf_edge[w], p.wf_prev[w], s_obs, hs, hcnt, klist);
     __syncwarp();  // the warp's half-space slots are rewritten by its next path
   }
 }
@@ -698,9 +706,16 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
   const int warp = threadIdx.x >> 5;
   int n = p.num_new;
   if (p.num_new_dev) n = (p.skip_dev && *p.skip_dev) ? 0 : (int)*p.num_new_dev;
+  // more blocks than resident ones: runs of consecutive paths
+  const bool runs = gridDim.x > (unsigned)kHsmcPersistBlocks;
+  unsigned step = 1u;
+  if (!runs) step = (unsigned)hsmc_chunks(n, gridDim.x, true);
   // a block with no path leaves before staging anything (block-uniform)
-  const int chunk = hsmc_chunk(n, gridDim.x);
-  if ((long long)blockIdx.x * chunk >= n) return;
+  if (!runs && blockIdx.x >= step) return;
+  const unsigned first = blockIdx.x * (runs ? (unsigned)kHsmcRun : 1u);
+  if (runs) n = (unsigned)n - first < (unsigned)kHsmcRun ? n : (int)(first + kHsmcRun);
+  __shared__ unsigned s_next;
+  if (threadIdx.x == 0) s_next = first;
   float *s_obs = reinterpret_cast<float *>(s_dyn4);
   float4 *hs = nullptr;
   uint8_t *hcnt = nullptr;
@@ -715,16 +730,8 @@ __device__ __forceinline__ void hsmc_run(const HsmcParams &p) {
     int *s_klist = reinterpret_cast<int *>(s_cnt + kHsmcWarps * cnt_stride);
     klist = s_klist + warp * kHsmcFilterObs;
   }
-  __shared__ int s_next;
-  const long long nchunks = ((long long)n + chunk - 1) / chunk;
-  for (long long ch = blockIdx.x; ch < nchunks; ch += gridDim.x) {  // block-uniform
-    __syncthreads();  // every warp is done with the previous chunk's counter
-    if (threadIdx.x == 0) s_next = 0;
-    __syncthreads();
-    const long long base = ch * chunk;
-    const int cnt = (int)((long long)n - base < chunk ? (long long)n - base : chunk);
-    hsmc_chunk_paths<Boxes, Q, Epi>(p, (int)base, cnt, &s_next, s_obs, hs, hcnt, klist);
-  }
+  __syncthreads();
+  hsmc_chunk_paths<Boxes, Q, Epi>(p, step, n, &s_next, s_obs, hs, hcnt, klist);
 }
 
 // Q = 32-bit particle words per lane: P <= 1024 Q.
@@ -744,9 +751,9 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_kernel(const HsmcParams 
 // around the tests (N = 32000, 4096 particles: the whole query 266 ms inlined,
 // 247 so).
 template <int Q>
-__device__ __noinline__ void hsmc_loop_paths(const HsmcParams &p, int base, int cnt, int *s_next,
+__device__ __noinline__ void hsmc_loop_paths(const HsmcParams &p, unsigned step, int n, unsigned *s_next,
                                              const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
-  hsmc_chunk_paths<true, Q, true>(p, base, cnt, s_next, s_obs, hs, hcnt, klist);
+  hsmc_chunk_paths<true, Q, true>(p, step, n, s_next, s_obs, hs, hcnt, klist);
 }
 
 template <int Q>
@@ -754,7 +761,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
   extern __shared__ float4 s_dyn4[];
   __shared__ int s_first[kLoopGroupMax + 1];  // first chunk of each query
   __shared__ HsmcParams s_p;
-  __shared__ int s_next;
+  __shared__ unsigned s_next;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nq = g->nq;
   const int share = (int)gridDim.x > nq ? (int)gridDim.x / nq : 1;  // blocks per query
@@ -765,8 +772,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
       if (*reinterpret_cast<const volatile int *>(&a->L.active)) {
         const HsmcParams &hp = a->hp;
         const int n = (hp.skip_dev && *hp.skip_dev) ? 0 : (int)*hp.num_new_dev;
-        const int chunk = hsmc_chunk(n, share);
-        c = (n + chunk - 1) / chunk;
+        c = hsmc_chunks(n, share, nq == 1);
       }
     }
     // inclusive scan over the queries (nq <= 32 lanes)
@@ -801,7 +807,7 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
       stage_obstacles(s_p.obs, s_p.numObs, s_obs);  // ends with a barrier
       cur = q;
     }
-    if (threadIdx.x == 0) s_next = 0;
+    if (threadIdx.x == 0) s_next = (unsigned)(ch - s_first[q]);
     __syncthreads();
     const HsmcParams &p = s_p;
     // this query's layout of the shared memory
@@ -810,11 +816,8 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGr
     uint8_t *s_cnt = reinterpret_cast<uint8_t *>(s_hs + kHsmcWarps * hs_stride);
     int *s_klist = reinterpret_cast<int *>(s_cnt + kHsmcWarps * cnt_stride);
     const int n = (p.skip_dev && *p.skip_dev) ? 0 : (int)*p.num_new_dev;
-    const int chunk = hsmc_chunk(n, share);
-    const int base = (ch - s_first[q]) * chunk;
-    const int cnt = n - base < chunk ? n - base : chunk;
-    hsmc_loop_paths<Q>(p, base, cnt, &s_next, s_obs, s_hs + warp * hs_stride,
-                              s_cnt + warp * cnt_stride, s_klist + warp * kHsmcFilterObs);
+    hsmc_loop_paths<Q>(p, (unsigned)hsmc_chunks(n, share, nq == 1), n, &s_next, s_obs, s_hs + warp * hs_stride,
+                       s_cnt + warp * cnt_stride, s_klist + warp * kHsmcFilterObs);
   }
 }
 
@@ -1100,7 +1103,7 @@ pump_status_t hsmc_staged_async(int num_new, int W, const int *d_edge, const int
   hp.num_new_dev = d_num_new;
   hp.skip_dev = d_skip;
   // (with a device-side count, num_new bounds it)
-  const unsigned blocks = hsmc_blocks(num_new);
+  const unsigned blocks = hsmc_blocks(num_new, d_num_new != nullptr);
   void *args[] = {(void *)&hp};
   PUMP_CUDA_TRY(cudaLaunchKernel(hsmc_kernel_for<false, false>(P), dim3(blocks), dim3(kHsmcThreads), args,
                                  0, stream));
@@ -1177,7 +1180,7 @@ pump_status_t hsmc_boxes_async(int num_new, int W, const int *d_edge, const int 
   const void *kern = epi ? hsmc_kernel_for<true, true>(P) : hsmc_kernel_for<true, false>(P);
   PUMP_TRY(smem_attr(kern, smem));
   // (with a device-side count, num_new bounds it)
-  const unsigned blocks = hsmc_blocks(num_new);
+  const unsigned blocks = hsmc_blocks(num_new, d_num_new != nullptr);
   void *args[] = {(void *)&hp};
   PUMP_CUDA_TRY(cudaLaunchKernel(kern, dim3(blocks), dim3(kHsmcThreads), args, smem, stream));
   return launch_status("hsmc_kernel (boxes)");

@@ -763,6 +763,14 @@ def test_hsmc_particle_rows(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap1000
     test_hsmc_particle_quads(P, Pmc, n_new, om, gpu, pumplib, oracle, roadmap1000)
 
 
+@pytest.mark.parametrize("n_new", [4863, 4865, 19456, 19459])
+def test_hsmc_wavefront_sizes(n_new, gpu, pumplib, oracle, roadmap1000):
+    """Wavefronts at the edges of the dealing rules: one path per warp of the
+    resident blocks and one more, sixteen paths a block, and past them runs of
+    eight consecutive paths, the last of three."""
+    test_hsmc_particle_quads(33, 64, n_new, 0.3, gpu, pumplib, oracle, roadmap1000)
+
+
 def test_hsmc_device_checks(gpu, pumplib, oracle, roadmap1000):
     """HSMC's device-side checks: an edge index outside [0, E) and a parent
     outside [0, base) skip their paths and record PUMP_ERR_BAD_INPUT; a time
