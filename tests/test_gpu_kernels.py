@@ -771,6 +771,51 @@ def test_hsmc_wavefront_sizes(n_new, gpu, pumplib, oracle, roadmap1000):
     test_hsmc_particle_quads(33, 64, n_new, 0.3, gpu, pumplib, oracle, roadmap1000)
 
 
+@pytest.mark.parametrize("boxes,spread", [(200, 1.0), (128, 0.0), (129, 0.0), (161, 0.02)])
+def test_hsmc_many_boxes(boxes, spread, gpu, pumplib, oracle, roadmap1000):
+    """More boxes than a warp's list of an edge's boxes holds: spread over the
+    map (few within an edge's reach) or all about one place (a full list, one
+    box past it, and more), where the edges there take every box."""
+    torch, _ = gpu
+    L = pumplib.load()
+    r = roadmap1000
+    rng = np.random.default_rng(boxes)
+    obs = np.zeros((boxes, 12), np.float32)
+    c = 0.5 + (rng.uniform(0, 1, (boxes, 3)) - 0.5) * spread
+    h = rng.uniform(0.01, 0.05, (boxes, 3))
+    obs[:, :3], obs[:, 6:9] = c - h, c + h
+    obs[:, 3:6], obs[:, 9:] = -3.1, 3.1
+    maxHS, T, base, n_new, P, om = 5, 400, 20, 600, 128, np.float32(0.3)
+    maxd2 = np.float32(0.1 * 0.3 * 0.3)
+    fe = np.ones(r["src"].size, np.uint8)
+    a, b, count = oracle.cache_halfspaces(r["disc"], fe, obs, maxHS, maxd2)
+    tm, _ = oracle.particle_tables(0x1234, P, T, pmajor=False)
+    edges = rng.choice(r["src"].size, n_new).astype(np.int32)
+    if spread < 1.0:  # half of the edges come near the boxes
+        near = np.nonzero((np.asarray(count).reshape(r["src"].size, -1) > 0).any(1))[0]
+        edges[: n_new // 2] = rng.choice(near, n_new // 2)
+    prev = rng.integers(0, base, n_new).astype(np.int32)
+    times = np.zeros(base + n_new, np.float32)
+    times[:base] = rng.uniform(0, 6, base).astype(np.float32)
+    vb = np.zeros((base + n_new, P), np.uint8)
+    vb[:base] = rng.random((base, P)) < 0.9
+    want, cp_o = vb.copy(), np.zeros(base + n_new, np.float32)
+    oracle.lib().orc_hsmc_propagate(n_new, 9, edges, prev, base, a, b, times, r["te"], 0.05, maxHS,
+                                    tm.reshape(-1), om, P, want, P, cp_o)
+    d = [dev(torch, x) for x in (edges, prev, obs, r["disc"], times, r["te"], tm)]
+    d_valid = dev(torch, np.packbits(vb, axis=1, bitorder="little").view(np.uint32))
+    d_cp, d_err = empty(torch, base + n_new, torch.float32), dev(torch, np.zeros(1, np.int32))
+    pumplib.check(L.pump_hsmc_propagate_boxes(
+        n_new, 9, ptr(d[0]), ptr(d[1]), r["src"].size, base, ptr(d[2]), boxes, ptr(d[3]), float(maxd2), maxHS,
+        ptr(d[4]), ptr(d[5]), 0.05, ptr(d[6]), P, T, float(om), ptr(d_valid), P, ptr(d_cp), ptr(d_err),
+        stream(torch)))
+    torch.cuda.synchronize()
+    got = bits_to_bytes(host(d_valid).reshape(base + n_new, P // 32), P)
+    assert np.array_equal(got[base:], want[base:])
+    assert same_bits(host(d_cp)[base:base + n_new], cp_o[base:]) and int(host(d_err)[0]) == 0
+    assert 0 < want[base:].mean() < vb[:base].mean()
+
+
 def test_hsmc_device_checks(gpu, pumplib, oracle, roadmap1000):
     """HSMC's device-side checks: an edge index outside [0, E) and a parent
     outside [0, base) skip their paths and record PUMP_ERR_BAD_INPUT; a time
