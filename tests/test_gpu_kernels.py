@@ -340,6 +340,73 @@ def test_waypoints_left_for_binary64(numDisc, gpu, pumplib, oracle):
     assert same_bits(host(out), want.reshape(-1)) and same_bits(host(out2), want.reshape(-1))
 
 
+@pytest.mark.parametrize("numDisc", [1, 2, 8, 33])
+def test_waypoints_coordinates_at_rest(numDisc, gpu, pumplib, oracle):
+    """Coordinates whose states need no evaluation (at rest, at zero or not) next
+    to ones that only look like it: -0 ends, huge, infinite and NaN positions at
+    rest, a velocity at one end.  Bit for bit with the reference's expression."""
+    torch, _ = gpu
+    L = pumplib.load()
+    rng = np.random.default_rng(31)
+    N = 48
+    s = np.concatenate([rng.uniform(0, 1, (N, 3)), rng.uniform(-1, 1, (N, 3))], 1).astype(np.float32)
+    s[4:12, [2, 5]] = 0.0
+    s[12:16, [0, 3]] = 0.0
+    s[12:16, [1, 4]] = 0.25, 0.0
+    s[16, [2, 5]], s[17, [2, 5]] = (-0.0, 0.0), (0.0, -0.0)
+    s[18:20, 0:3], s[18:20, 3:6] = -0.0, -0.0
+    s[20:22, 0], s[20:22, 1], s[20:22, 2], s[20:22, 3:6] = 3e38, np.inf, np.nan, 0.0
+    s[22:24, 0], s[22:24, 1], s[22:24, 3:6] = 2.0 ** 60, 2.0 ** 61, 0.0
+    s[24:26] = s[24]
+    s[24:26, 3:6] = 0.0
+    src = np.repeat(np.arange(N), N).astype(np.int32)
+    dst = np.tile(np.arange(N), N).astype(np.int32)
+    E, W = N * N, numDisc + 1
+    tau = np.array([0.5, 0.371, 1.9, 3.0], np.float32)[np.arange(E) % 4]
+    want = np.zeros((E, W, 6), np.float32)
+    x = np.zeros(6, np.float32)
+    for e in range(E):
+        dt = np.float32(tau[e] / np.float32(numDisc))
+        want[e, 0], want[e, numDisc] = s[src[e]], s[dst[e]]
+        for i in range(1, numDisc):
+            oracle.lib().orc_path_point(np.float32(dt * np.float32(i)), tau[e], s[src[e]], s[dst[e]], x)
+            want[e, i] = x
+    d = [dev(torch, a) for a in (s, src, dst, tau)]
+    out = empty(torch, E * W * 6, torch.float32)
+    pumplib.check(L.pump_discretize_edges(ptr(d[0]), ptr(d[1]), ptr(d[2]), ptr(d[3]), E, numDisc, 0, ptr(out),
+                                          stream(torch)))
+    torch.cuda.synchronize()
+    got, want = host(out), want.reshape(-1)
+    nan = np.isnan(want)
+    assert np.array_equal(np.isnan(got), nan) and same_bits(got[~nan], want[~nan])
+
+
+def test_waypoints_in_a_plane_time(gpu, pumplib):
+    """Edges with coordinates at rest take no longer than general ones."""
+    torch, _ = gpu
+    L = pumplib.load()
+    rng = np.random.default_rng(37)
+    N, E, numDisc = 1000, 100_000, 8
+    flat = np.concatenate([rng.uniform(0, 1, (N, 3)), rng.uniform(-1, 1, (N, 3))], 1).astype(np.float32)
+    line = flat.copy()
+    line[:, [1, 2, 4, 5]] = 0.0
+    src, dst = dev(torch, rng.integers(0, N, E).astype(np.int32)), dev(torch, rng.integers(0, N, E).astype(np.int32))
+    tau = dev(torch, rng.uniform(0.2, 1.2, E).astype(np.float32))
+    out = empty(torch, E * (numDisc + 1) * 6, torch.float32)
+    best = {}
+    for name, s in (("general", dev(torch, flat)), ("line", dev(torch, line))):
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            pumplib.check(L.pump_discretize_edges(ptr(s), ptr(src), ptr(dst), ptr(tau), E, numDisc, 0, ptr(out),
+                                                  stream(torch)))
+            b.record()
+            torch.cuda.synchronize()
+            best[name] = min(best.get(name, 1e9), a.elapsed_time(b))
+    # (sixteen times as long when such states were evaluated in binary64)
+    assert best["line"] <= 3.0 * best["general"], best
+
+
 def test_roadmap_edges_one_read(gpu, pumplib, roadmap1000):
     """rn and the edges from one read of the pair costs equal pump_select_kth +
     pump_build_edges (the oracle's sort and scan) bit for bit."""
