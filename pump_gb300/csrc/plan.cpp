@@ -212,6 +212,20 @@ struct SharedRoadmap {
 };
 
 
+// Steps of the smoothing's alpha bisection evaluated ahead per batch (2^D - 1
+// candidate paths, 30 / D batches).  A deeper batch saves round trips, but most of
+// its paths are never visited, so it pays while their Monte Carlo CPs (128
+// particles of a path a block) are at most two rounds of the resident blocks: 31
+// paths x 4864 particles.  Whole queries at N = 1000, us, depths 3, 4 and 5: 2048
+// particles 738, 730, 672; 4800 783, 728, 735; 6000 685, 656, 675; 8192 702, 726,
+// 771; 12,000 722, 760, 848; 100,000 1305 and 2197 (3 and 5).
+// pump_plan_batch's workers share the GPU and take 3; programs that call pump_plan
+// from several threads gain too, up to four of them (N = 1000, 2048 particles, us a
+// query, depths 3 / 5: two threads 648 / 599, four 440 / 418, eight 351 / 355).
+int smooth_depth(int num_mc, bool batch_worker) {
+  return batch_worker || num_mc > 7168 ? 3 : (num_mc > 4864 ? 4 : 5);
+}
+
 class Planner {
  public:
   // lazy: check each node's out-edges when the search first reaches it (the
@@ -1305,12 +1319,9 @@ pump_status_t Planner::search_and_smooth() {
     // paths, costs and MC CPs of all of them), then the reference's decisions
     // are replayed in order over the results: the same sequence of alphas,
     // best-path updates and early exit as PUMP.cu:492-541.  Most of a deep
-    // batch's work is for alphas the bisection never visits, but a query alone
-    // on the GPU leaves it nearly idle: D = 5 (31 paths, 6 batches of up to 30
-    // steps) took 1063 us where D = 3 (10 batches) took 1187, D = 4 1135 and
-    // D = 6 1107 for a whole query at N = 1000.  Batch workers share the GPU
-    // and keep D = 3.
-    const int D = lazy_ ? 3 : 5, K = (1 << D) - 1;
+    // batch's work is for alphas the bisection never visits; it is free while
+    // the GPU has room for it (smooth_depth).
+    const int D = smooth_depth(pb_.num_mc, lazy_), K = (1 << D) - 1;
     int it = 0;
     bool stop = false;
     while (it < 30 && !stop) {

@@ -317,3 +317,49 @@ def test_plan_path_state_readback(gpu, pumplib, goldens):
     valid = np.unpackbits(pvalid.view(np.uint8).reshape(n, -1), axis=1, bitorder="little")[:, :P]
     cp = (P - valid.sum(1)).astype(np.float32) / np.float32(P)
     assert np.all(cp <= np.float32(pb.cp_target) * np.float32(pb.cp_factor))
+
+
+def smoothing_problem(L, N, num_mc, mode, noise):
+    from pump_gb300 import workloads
+    obs = workloads.random_boxes(10, 0)
+    pb = L.Problem()
+    L.load().pump_problem_defaults(C.byref(pb))
+    pb.N, pb.num_disc, pb.num_mc, pb.bvp_mode = N, 8, num_mc, mode
+    pb.num_obstacles, pb.obstacles = obs.shape[0], obs.ctypes.data
+    for k in range(6):
+        pb.init[k], pb.goal[k] = workloads.INIT[k], workloads.GOAL[k]
+        pb.lo[k], pb.hi[k] = workloads.LO[k], workloads.HI[k]
+    pb.offset_mult, pb.cp_target, pb.cp_factor = noise, 0.01, 2.0
+    return pb, obs
+
+
+@pytest.mark.parametrize("num_mc", [4864, 4865, 7168, 7169])
+def test_plan_smoothing_depths(num_mc, gpu, pumplib, oracle):
+    """Particle counts at the edges of the smoothing's three batch depths: the
+    whole query is the oracle's."""
+    torch, ctx = gpu
+    from pump_gb300 import workloads
+    pb, obs = smoothing_problem(pumplib, 300, num_mc, pumplib.PUMP_BVP_PARITY, 0.1)
+    st, res, path, _ = run_plan(pumplib, ctx, pb)
+    assert st == pumplib.PUMP_OK
+    r = oracle.plan(300, obs, workloads.INIT, workloads.GOAL, workloads.LO, workloads.HI, np.float32(0.1),
+                    0.01, 2.0, Pmc=num_mc)
+    assert res.num_paths == r["numPaths"] and res.success == r["success"] == 1
+    assert np.array_equal(path.view(np.uint32), r["path"].view(np.uint32))
+
+
+def test_plan_smoothing_time_many_particles(gpu, pumplib):
+    """Alphas that the bisection never visits are not evaluated where their
+    Monte Carlo CPs fill the GPU: 100,000 particles take less than twice the
+    query's time with 2048 (2.3 times with 31 alphas a batch, 1.4 with 7)."""
+    import time
+    torch, ctx = gpu
+    best = {}
+    for num_mc in (2048, 100_000):
+        pb, _obs = smoothing_problem(pumplib, 1000, num_mc, pumplib.PUMP_BVP_PRECISION, 1e-3)
+        for _ in range(12):
+            t = time.perf_counter()
+            st = run_plan(pumplib, ctx, pb)[0]
+            best[num_mc] = min(best.get(num_mc, 1e9), time.perf_counter() - t)
+            assert st == pumplib.PUMP_OK
+    assert best[100_000] < 2.0 * best[2048], best
