@@ -12,7 +12,7 @@
 // themselves: one in float-float (cost_ff_value: about 180), the other from it
 // and the difference, each certified to round as the reference's; what is
 // not certified falls back to float-float for the second cost, then to the
-// reference's own expression (Exact::cost).  Of a random pair's 11 finite
+// reference's own expression (Exact::costs).  Of a random pair's 11 finite
 // differences (states as the benchmark's), 6 are settled by the derivative, 3
 // by the difference, and 2 need the costs.
 //
@@ -229,8 +229,7 @@ __device__ __forceinline__ void bisect_warp(const Src &src, BisectQueue &queue, 
         if (!(ok_a && ok_b)) {
           float x0[kDim], x1[kDim];
           src.load(first + it.item, x0, x1);
-          if (!ok_a) ca = Exact::cost(x0, x1, ta);
-          if (!ok_b) cb = Exact::cost(x0, x1, tb);
+          Exact::costs(x0, x1, ta, tb, !ok_a, !ok_b, &ca, &cb);
         }
         const float d = (ca - cb) / dtau;
         sign = d > 0 ? 1 : (d < 0 ? -1 : 0);

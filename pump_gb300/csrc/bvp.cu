@@ -135,14 +135,16 @@ struct ParityCost {
   static __device__ __noinline__ float eval(const States s, float tau) {
     return cost_eval(make_coef(s.x0, s.x1), tau);
   }
-  static __device__ __forceinline__ float cost(const float *x0, const float *x1, float tau) {
+  static __device__ __forceinline__ void costs(const float *x0, const float *x1, float ta, float tb,
+                                               bool want_a, bool want_b, float *ca, float *cb) {
     States s;
 #pragma unroll
     for (int d = 0; d < kDim; ++d) {
       s.x0[d] = x0[d];
       s.x1[d] = x1[d];
     }
-    return eval(s, tau);
+    if (want_a) *ca = eval(s, ta);
+    if (want_b) *cb = eval(s, tb);
   }
 };
 

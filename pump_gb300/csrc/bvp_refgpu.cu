@@ -77,7 +77,9 @@ struct RefGpuCost {
   struct States {
     float a[kDim], b[kDim];
   };
-  static __device__ __noinline__ float eval(const States st, float tau) {
+  // the bounded evaluation: NaN where it leaves the value open
+  static __device__ __noinline__ float bounded(const States st, float tau) {
+    if (!(tau >= 1e-4f && tau <= 1e4f)) return NAN;
     const PairFF f = make_pair_ff(st.a, st.b);
     const float a29 = __fmul_rn(f.a29, f.b29 + f.c29 * tau);
     const float a30 = __fmul_rn(f.a30, f.b30 + f.c30 * tau);
@@ -99,17 +101,40 @@ struct RefGpuCost {
                       ((((float)d4) * tau + f.abs_d3) * tau + f.abs_d2) * tau * tau;
     const double B = (double)mag * 0x1p-45 / t3 + fabs(v) * 0x1p-50;
     const float lo = (float)(v - B), hi = (float)(v + B);
-    if (tau >= 1e-4f && tau <= 1e4f && lo == hi && fabsf(lo) > 1e-30f && fabsf(lo) < 1e30f) return lo;
-    return cost_dev(tau, st.a, st.b, coord_pow(st.a, st.b));
+    return lo == hi && fabsf(lo) > 1e-30f && fabsf(lo) < 1e30f ? lo : NAN;
   }
-  static __device__ __forceinline__ float cost(const float *x0, const float *x1, float tau) {
+  // the expression at ta and tb; the coordinates' powers, 12 of its 15, are shared
+  struct Costs {
+    float ca, cb;
+  };
+  static __device__ __noinline__ Costs powers(const States st, float ta, float tb, bool want_a, bool want_b) {
+    const CoordPow p = coord_pow(st.a, st.b);
+    Costs r{0.0f, 0.0f};
+    if (want_a) r.ca = cost_dev(ta, st.a, st.b, p);
+    if (want_b) r.cb = cost_dev(tb, st.a, st.b, p);
+    return r;
+  }
+  static __device__ __forceinline__ void costs(const float *x0, const float *x1, float ta, float tb,
+                                               bool want_a, bool want_b, float *ca, float *cb) {
     States st;
 #pragma unroll
     for (int d = 0; d < kDim; ++d) {
       st.a[d] = x0[d];
       st.b[d] = x1[d];
     }
-    return eval(st, tau);
+    if (want_a) {
+      const float v = bounded(st, ta);
+      if (v == v) *ca = v, want_a = false;
+    }
+    if (want_b) {
+      const float v = bounded(st, tb);
+      if (v == v) *cb = v, want_b = false;
+    }
+    if (want_a || want_b) {
+      const Costs r = powers(st, ta, tb, want_a, want_b);
+      if (want_a) *ca = r.ca;
+      if (want_b) *cb = r.cb;
+    }
   }
 };
 

@@ -112,6 +112,32 @@ def test_bvp_pairs_parity_certified_steps(kind, tmax, gpu, pumplib, oracle):
     assert np.array_equal(np.isnan(c), nan) and same_bits(t, rt) and same_bits(c[~nan], rc[~nan])
 
 
+def bvp_pairs_time(torch, pumplib, s, mode, runs=6):
+    """Least time of pump_bvp_pairs over the states, in ms."""
+    n = s.shape[0] * (s.shape[0] - 1)
+    d, c, t = dev(torch, s), empty(torch, n, torch.float32), empty(torch, n, torch.float32)
+    best = 1e9
+    for _ in range(runs):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        pumplib.check(pumplib.load().pump_bvp_pairs(ptr(d), s.shape[0], 5.0, mode, ptr(c), ptr(t), stream(torch)))
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_bvp_pairs_refgpu_equal_states_time(gpu, pumplib):
+    """Equal states: bisections down to times that only the reference's
+    expression covers, whose powers of the coordinates both sides of a finite
+    difference share (15.4 ms when they did not, 10.1 so)."""
+    torch, _ = gpu
+    rng = np.random.default_rng(11)
+    s = np.concatenate([rng.uniform(0, 1, (1000, 3)), rng.uniform(-1, 1, (1000, 3))], 1)
+    s = s[rng.integers(0, 40, 1000)].astype(np.float32)
+    assert bvp_pairs_time(torch, pumplib, s, pumplib.PUMP_BVP_PARITY_GPU) < 13.0
+
+
 def test_bvp_batch_parity(gpu, pumplib, oracle):
     torch, _ = gpu
     L = pumplib.load()
