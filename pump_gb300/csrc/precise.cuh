@@ -356,18 +356,21 @@ __device__ __forceinline__ float sqrt_f32(float x) {
 }
 
 // The optimal time and cost, correctly rounded binary32 values (t, c) with
-// the rest of the time in dt (t + dt: about 2^-44 relative).
+// the rest of the time in dt (t + dt: about 2^-44 relative).  (Pairs left to
+// precise_general: from one binary64 Newton step, and where tmax is within
+// binary32's noise of the root, either of the two.)
 //
 // In almost every pair Q has one positive root, which is then the cost's only
 // minimum (c' = Q / t^4).  With tc = sqrt(A2 / (6 A4)), the inflection point of
 // Q, that is certain when A1 >= 0 (one sign change); when A1 < 0 and Q' has no
 // zero on t > 0 (|A1| >= 2/3 A2 tc: Q increases); and when Q < 0 up to tc (A4
 // tc^4 + 2 |A1| tc < 3 A0), since Q is convex beyond (the last two tested with
-// 1e-3 margins).  The root comes from two closed-form steps (the biquadratic
+// margins of 5e-4 and 1e-3).  The root comes from two closed-form steps (the biquadratic
 // without the linear term, then with that term frozen at its root) and three
 // Halley steps in binary32: of 2 M random pairs, all are within 1e-4 before
 // the third step, which leaves its cube.  Any positive root that the steps
-// converge to is the root.
+// converge to is the root; that it lies beyond tmax
+// is confirmed by Q(tmax) < 0.
 //
 // Then one Newton step with the residual Q(x) in float-float gives dx, and the
 // cost at the root is c(x) + c'(x) dx / 2 (c' vanishes at the root; third
@@ -410,7 +413,7 @@ __device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const Sampl
     x = x - step;
   }
   bool ok = unique && fabsf(step) <= 2e-3f * x && x >= 1e-6f && x <= 1e6f;
-  const bool beyond = x > tmax * 1.00001f;  // the cost still falls at tmax
+  const bool beyond = x > tmax * 1.00001f;  // the cost still falls at tmax (Q < 0 there, tested below)
   x = fminf(x, tmax);
   // Q(x), the Newton step and its error
   const FF x2 = two_prod(x, x);
@@ -429,7 +432,7 @@ __device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const Sampl
   if (x >= tmax) dx = beyond ? 0.0f : fminf(dx, 0.0f);
   const float bt = beyond ? 0.0f
                           : fabsf(rq) * fmaf(fabsf(dx), fmaf(mq * r, 0x1p-18f, fabsf(dx) * ddq), mq * 0x1p-40f);
-  ok = ok && fabsf(dx) <= 0x1p-18f * x && (beyond || dq > 0.0f);
+  ok = ok && fabsf(dx) <= 0x1p-18f * x && (beyond ? qv < -(mq * 0x1p-40f) : dq > 0.0f);
   // c(x) = A3 + A4 x + r (A2 + r (A1 + r A0)), 1/x in float-float
   const FF rr = {r, r * fmaf(-x, r, 1.0f)};
   FF v = ff_add_raw(ff_mul_raw(ff_mulf_raw(pc.dd, 12.0f), rr), ff_mulf_raw(pc.ds, -12.0f));

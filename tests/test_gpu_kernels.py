@@ -1178,6 +1178,71 @@ def test_bvp_pairs_precision_certified_and_general(kind, tmax, gpu, pumplib, ora
     assert ulps(t, t64).max() <= 2
 
 
+def precision_rounding(torch, pumplib, oracle, s, tmax):
+    """Pairs of the states s whose time or cost is not the binary32 rounding of
+    the binary64 minimiser's, pairs too close to a rounding boundary to tell
+    (2^-38 of the terms' magnitudes, four times what the kernel's certificates
+    take) and all pairs."""
+    tmax = float(np.float32(tmax))  # what the call's binary32 argument holds
+    c, t = run_bvp_pairs(torch, pumplib, s, mode=pumplib.PUMP_BVP_PRECISION, tmax=tmax)
+    i, j = np.nonzero(~np.eye(s.shape[0], dtype=bool))
+    t64, c64 = oracle.bvp_binary64(s[i], s[j], tmax)
+    A0, A1, A2, A3, A4 = oracle.cost_coeffs64(s[i], s[j])
+    x0, x1 = s[i].astype(np.float64), s[j].astype(np.float64)
+    a1 = 12 * np.abs((x1[:, :3] - x0[:, :3]) * (x0[:, 3:] + x1[:, 3:])).sum(1)
+    dq = np.abs((4 * A4 * t64**2 - 2 * A2) * t64 - 2 * A1)
+    mq = ((A4 * t64**2 + A2) * t64 + 2 * a1) * t64 + 3 * A0
+    mc = ((A0 / t64 + a1) / t64 + A2) / t64 + np.abs(A3) + A4 * t64
+    at_end = t64 == tmax
+    near_t = np.where(at_end, 0.0, 2.0 ** -38 * mq / np.maximum(dq, 1e-300))
+    near_c = 2.0 ** -38 * mc + np.where(at_end, 0.0, 2.0 ** -38 * mq / t64**4 * near_t)
+
+    def wrong(got, want, room):
+        lo, hi = (want - room).astype(np.float32), (want + room).astype(np.float32)
+        return (got != lo) & (got != hi), lo != hi
+    wt, ot = wrong(t, t64, near_t)
+    wc, oc = wrong(c, c64, near_c)
+    # two minima of the same cost: either time
+    other = oracle.cost64(t.astype(np.float64), (A0, A1, A2, A3, A4))
+    wt &= ~(np.abs(other - c64) <= near_c) | (np.abs(t - t64) < 1e-3 * t64)
+    # with several stationary points, whether the last one lies before tmax is
+    # read off binary32 signs, so within their noise either stands for the other
+    wt &= (np.abs(t64 - tmax) > 2.0 ** -20 * tmax) | (np.abs(t - t64) > 2.0 ** -20 * t64)
+    return int((wt | wc).sum()), int((ot | oc).sum()), t.size
+
+
+@pytest.mark.parametrize("kind", ["plain", "near", "x10", "x1e-3", "rest", "fast"])
+def test_bvp_pairs_precision_rounding(kind, gpu, pumplib, oracle):
+    """The precision mode's times and costs are the binary32 roundings of the
+    binary64 minimiser's wherever those are clear of a rounding boundary, over
+    the ways to the optimum (certified, several stationary points, at tmax),
+    and for tmax close to a pair's optimum on either side."""
+    torch, _ = gpu
+    rng = np.random.default_rng(41)
+    s = np.concatenate([rng.uniform(0, 1, (160, 3)), rng.uniform(-1, 1, (160, 3))], 1)
+    if kind == "near":
+        s = s[0] + (s - s[0]) * 1e-2
+    if kind == "x10":
+        s = s * 10
+    if kind == "x1e-3":
+        s = s * 1e-3
+    if kind == "rest":
+        s[:, 3:] = 0
+    if kind == "fast":
+        s[:, 3:] *= 3
+    s = s.astype(np.float32)
+    for tmax in (5.0, 0.4):
+        bad, open_, n = precision_rounding(torch, pumplib, oracle, s, tmax)
+        assert bad == 0 and open_ < 0.01 * n, (tmax, bad, open_, n)
+    few = s[:12]
+    root = oracle.bvp_binary64(few[:-1], few[1:], 50.0)[0]
+    for d in (0.0, 1e-7, 1e-6, 5e-6, 9e-6, 1.1e-5, 2e-5, 1e-4):
+        for r in root[:6]:
+            for sign in (1.0, -1.0):
+                bad, _, _ = precision_rounding(torch, pumplib, oracle, few, r * (1.0 + sign * d))
+                assert bad == 0, (r, sign * d)
+
+
 def test_mc_cp_binary32_vs_binary64(gpu, pumplib, oracle):
     """The binary32 Monte Carlo CP (collision tests as the reference's, in
     binary32) against the same estimate with every test in binary64: hit
