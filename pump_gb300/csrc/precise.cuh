@@ -361,16 +361,23 @@ __device__ __forceinline__ float sqrt_f32(float x) {
 // binary32's noise of the root, either of the two.)
 //
 // In almost every pair Q has one positive root, which is then the cost's only
-// minimum (c' = Q / t^4).  With tc = sqrt(A2 / (6 A4)), the inflection point of
-// Q, that is certain when A1 >= 0 (one sign change); when A1 < 0 and Q' has no
-// zero on t > 0 (|A1| >= 2/3 A2 tc: Q increases); and when Q < 0 up to tc (A4
-// tc^4 + 2 |A1| tc < 3 A0), since Q is convex beyond (the last two tested with
-// margins of 5e-4 and 1e-3).  The root comes from two closed-form steps (the biquadratic
-// without the linear term, then with that term frozen at its root) and three
-// Halley steps in binary32: of 2 M random pairs, all are within 1e-4 before
-// the third step, which leaves its cube.  Any positive root that the steps
-// converge to is the root; that it lies beyond tmax
-// is confirmed by Q(tmax) < 0.
+// minimum (c' = Q / t^4).  That is certain
+//   - when A1 >= 0 (one sign change);
+//   - when A1^2 < 8/3 A0 A2: if Q has a local maximum at some r > 0 (Q' = 0
+//     there, 4 A4 r^3 = 2 A2 r + 2 A1), its value is -A2 r^2 / 2 - 3/2 A1 r - 3 A0
+//     <= 9/8 A1^2 / A2 - 3 A0 < 0, so Q < 0 until it crosses once, past its local
+//     minimum; without one Q only increases;
+//   - when Q' has no zero on t > 0: |A1| >= 2/3 A2 tc with tc = sqrt(A2 / (6 A4)),
+//     the inflection point of Q
+// (margins of 1.5e-3 and 5e-4 in the last two, and an absolute one where the squares
+// leave binary32's normal range).  The root comes from two closed-form steps (the
+// biquadratic without the linear term, then with that term frozen at its root) and
+// three Halley steps in binary32, up to three more while a step is large.  Any
+// positive root that the steps converge to is the root; that it lies beyond tmax
+// is confirmed by Q(tmax) < 0.  (With Q < 0 up to tc bounded by leaving the t^2 term
+// out, and three steps for all, one pair in six went the general way where
+// velocities are several times what a segment's length allows: N = 4000, velocities
+// up to 3 over a unit cube, 0.815 ms, 0.391 so, 0.765 with every pair in binary64.)
 //
 // Then one Newton step with the residual Q(x) in float-float gives dx, and the
 // cost at the root is c(x) + c'(x) dx / 2 (c' vanishes at the root; third
@@ -394,15 +401,13 @@ __device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const Sampl
   constexpr float kA4 = (float)kA4d, kA4l = (float)(kA4d - (double)kA4), kR4 = (float)(1.0 / kA4d);
   // Q / A4 = t^4 - a t^2 - b t - c
   const float a = pc.A2s.h * (4.0f * kR4), b = pc.ds.h * (-24.0f * kR4), c = pc.dd.h * (36.0f * kR4);
-  const float tc = sqrt_f32(a * (1.0f / 6.0f));
-  const float tc2 = tc * tc;
-  const bool unique = b >= 0.0f || -b >= 1.334f * a * tc || tc * fmaf(tc2, tc, -b) < 0.999f * c;
+  const bool unique = b >= 0.0f || b * b < fmaf(3.55f * a, c, -1e-36f) ||
+                      -b >= 1.334f * a * sqrt_f32(a * (1.0f / 6.0f));
   const float aa = a * a;
   const float t0 = sqrt_f32(0.5f * (a + sqrt_f32(fmaf(4.0f, c, aa))));
   const float t1 = 0.5f * (a + sqrt_f32(fmaxf(fmaf(4.0f, fmaf(b, t0, c), aa), c)));
   float x = sqrt_f32(t1), step = 0.0f;
-#pragma unroll
-  for (int it = 0; it < 3; ++it) {
+  auto halley = [&] {
     const float x2 = x * x;
     const float q = fmaf(fmaf(x2 - a, x, -b), x, -c);
     const float dq = fmaf(fmaf(4.0f, x2, -2.0f * a), x, -b);
@@ -411,7 +416,10 @@ __device__ __forceinline__ PreciseMin precise_min(const SampleF &sa, const Sampl
     // Halley: s / (1 - s q'' / (2 q')), the quotient by its own estimate
     step = s * rcp_f32(fmaf(-s * r, fmaf(6.0f, x2, -a), 1.0f));
     x = x - step;
-  }
+  };
+#pragma unroll
+  for (int it = 0; it < 3; ++it) halley();
+  for (int it = 0; it < 3 && unique && fabsf(step) > 2e-3f * x; ++it) halley();
   bool ok = unique && fabsf(step) <= 2e-3f * x && x >= 1e-6f && x <= 1e6f;
   const bool beyond = x > tmax * 1.00001f;  // the cost still falls at tmax (Q < 0 there, tested below)
   x = fminf(x, tmax);

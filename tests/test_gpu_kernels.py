@@ -1243,6 +1243,20 @@ def test_bvp_pairs_precision_rounding(kind, gpu, pumplib, oracle):
                 assert bad == 0, (r, sign * d)
 
 
+def test_bvp_pairs_precision_fast_states_time(gpu, pumplib):
+    """States whose velocities are several times what a segment's length allows
+    have their optimum certified like others, but for one pair in eighty (a
+    sixth of them took the general way, and every warp with them: 3.5 times as
+    long as slow states, 1.7 so)."""
+    torch, _ = gpu
+    rng = np.random.default_rng(43)
+    slow = np.concatenate([rng.uniform(0, 1, (3000, 3)), rng.uniform(-1, 1, (3000, 3))], 1).astype(np.float32)
+    fast = slow.copy()
+    fast[:, 3:] *= 3
+    t = [bvp_pairs_time(torch, pumplib, s, pumplib.PUMP_BVP_PRECISION) for s in (slow, fast)]
+    assert t[1] < 2.5 * t[0], t
+
+
 def test_mc_cp_binary32_vs_binary64(gpu, pumplib, oracle):
     """The binary32 Monte Carlo CP (collision tests as the reference's, in
     binary32) against the same estimate with every test in binary64: hit
