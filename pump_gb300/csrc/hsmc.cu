@@ -1044,9 +1044,11 @@ pump_status_t mc_cp_hits_async(const float *d_paths, const int *d_offset, const 
     }
     return PUMP_OK;
   };
-  // particles per lane: four once that still leaves every SM two blocks
+  // particles per lane: four once one per lane is two rounds of its resident
+  // blocks (two an SM) and four still leave every SM a block: 8 paths x 4096
+  // particles, 1 and 10 boxes, 23 and 24 us with one, 17 and 19 with four.
   const long long blocks = (long long)n_paths * grid_for(Pmc, 32);
-  if (blocks >= 8LL * kNumSMs) return go(std::integral_constant<int, 4>{});
+  if (blocks >= 4LL * kNumSMs) return go(std::integral_constant<int, 4>{});
   return go(std::integral_constant<int, 1>{});
 }
 
