@@ -295,15 +295,16 @@ __global__ void __launch_bounds__(kRefThreads, Grad ? 3 : 4) refine_kernel(pump_
     if (Grad) {
       if (__any_sync(0xffffffffu, any)) {
 #pragma unroll
-        for (int m = 0; m < 12; ++m) acc[m] = warp_sum(acc[m]) * lam;
-        tb_acc = warp_sum(tb_acc) * lam;
-        Tb_acc = warp_sum(Tb_acc) * lam;
+        for (int m = 0; m < 12; ++m) acc[m] = warp_sum(acc[m]);
+        tb_acc = warp_sum(tb_acc);
+        Tb_acc = warp_sum(Tb_acc);
       }
+      // (a weight that is not finite shows in the gradient whatever is near)
       if (lane == 0) {
 #pragma unroll
-        for (int m = 0; m < 12; ++m) s_g[i * 12 + m] += acc[m];
-        s_taubar[i] = tb_acc;
-        s_Tbar[i] = Tb_acc;
+        for (int m = 0; m < 12; ++m) s_g[i * 12 + m] += acc[m] * lam;
+        s_taubar[i] = tb_acc * lam;
+        s_Tbar[i] = Tb_acc * lam;
       }
     }
   }

@@ -126,6 +126,27 @@ def test_pairs_over_lanes(gpu, pumplib, oracle, W, boxes, om):
         assert np.linalg.norm(case.path(k, g) - g64) <= REL_G * np.linalg.norm(g64) + cond[3]
 
 
+@pytest.mark.parametrize("boxes", [0, 40])
+@pytest.mark.parametrize("weight", [np.nan, np.inf])
+def test_weight_that_is_not_finite(gpu, pumplib, oracle, weight, boxes):
+    """A bound weight that is not finite shows in every intermediate node's
+    gradient, also on paths that no box is near (the bound's derivative is zero
+    there, times the weight not a number); other paths are unaffected."""
+    torch, _ = gpu
+    case = Case(torch, pumplib, oracle, 4, 5, 2e-3)
+    case.args.num_obstacles = boxes
+    g0, _ = bwd(torch, pumplib, case)
+    lam = case.lam.copy()
+    lam[[0, 2]] = weight
+    case.keep[3].copy_(torch.from_numpy(lam))
+    g, J = bwd(torch, pumplib, case)
+    assert np.isnan(J[[0, 2]]).all() or boxes
+    for k in (0, 2):
+        assert not np.isfinite(case.path(k, g.reshape(-1, 6))[1:-1]).any()
+    for k in (1, 3):
+        assert np.array_equal(case.path(k, g.reshape(-1, 6)), case.path(k, g0.reshape(-1, 6)))
+
+
 def test_clamped_segments(gpu, pumplib, oracle):
     torch, _ = gpu
     case = Case(torch, pumplib, oracle, 16, 7, 0.3, tmax=0.3, n_range=(5, 8))
