@@ -572,6 +572,50 @@ def test_roadmap_one_call(case, mode, gpu, pumplib):
         assert same_bits(np.atleast_1d(a), np.atleast_1d(b)), (case, mode, name)
 
 
+@pytest.mark.parametrize("share,room", [(1e-4, 1.0), (0.05, 0.5), (0.3, 1.0), (0.3, 0.1), (0.6, 1.0), (0.6, 0.999)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_roadmap_shares_of_the_pairs(share, room, mode, gpu, pumplib):
+    """Roadmaps of few and of most pairs (a block's masks hold several windows
+    of listed pairs), with rows that have no edge (first, inner and last), and
+    with room for a part of the edges only: the edges that fit and their row
+    starts, the whole count, and the capacity error."""
+    torch, ctx = gpu
+    L = pumplib.load()
+    rng = np.random.default_rng(7)
+    N = 910
+    s = np.concatenate([rng.uniform(0, 1, (N, 3)), rng.uniform(-1, 1, (N, 3))], 1)
+    s[[0, 1, 400, N - 2, N - 1], :3] += np.arange(1, 6)[:, None] * 40.0
+    s = s.astype(np.float32)
+    n = N * (N - 1)
+    k = int(np.float32(n) * np.float32(share))
+    c, t = run_bvp_pairs(torch, pumplib, s, mode)
+    rn = np.sort(c)[k]
+    at = np.nonzero(c < rn)[0]
+    i = (at // (N - 1)).astype(np.int32)
+    j = (at % (N - 1)).astype(np.int32)
+    j = j + (j >= i)
+    cap = int(k * room)
+    d_s = dev(torch, s)
+    d_c, d_t = empty(torch, n, torch.float32), empty(torch, n, torch.float32)
+    d_src, d_dst = (torch.full((k + 1,), -7, dtype=torch.int32, device="cuda") for _ in range(2))
+    d_ce, d_te = empty(torch, k, torch.float32), empty(torch, k, torch.float32)
+    d_go = empty(torch, N + 1, torch.int32)
+    got_rn, E = C.c_float(0), C.c_longlong(0)
+    st = L.pump_roadmap(ctx.handle, ptr(d_s), N, 5.0, mode, k, cap, ptr(d_c), ptr(d_t), ptr(d_src), ptr(d_dst),
+                        ptr(d_ce), ptr(d_te), ptr(d_go), C.byref(got_rn), C.byref(E), None, stream(torch))
+    torch.cuda.synchronize()
+    fits = at.size <= cap
+    assert st == (pumplib.PUMP_OK if fits else pumplib.PUMP_ERR_CAPACITY)
+    assert np.float32(got_rn.value) == rn
+    m = min(at.size, cap)
+    if fits:
+        assert E.value == at.size
+    assert np.array_equal(host(d_src, m), i[:m]) and np.array_equal(host(d_dst, m), j[:m])
+    assert same_bits(host(d_ce, m), c[at[:m]]) and same_bits(host(d_te, m), t[at[:m]])
+    assert (host(d_src)[m:] == -7).all()
+    assert np.array_equal(host(d_go, N + 1), np.searchsorted(i[:m], np.arange(N + 1), side="left"))
+
+
 def test_roadmap_one_call_parity_oracle(gpu, pumplib, roadmap1000):
     """In the parity arithmetic pump_roadmap's rn and edges are the oracle's."""
     torch, ctx = gpu
