@@ -810,24 +810,24 @@ def mode_record(lib, L, ctx, torch, w, mode, args, flush, batch, steps=None, war
 # Binary64 flops per ordered pair of the 2pBVP kernels (a fused multiply-add
 # counts two): ncu's counts of the add, multiply and fused instructions' lanes
 # (smsp__sass_thread_inst_executed_op_d*_pred_on.sum) of one launch, per pair,
-# at N = 4000 (precision: 48,624 + 16,291 + 2 x 81,870 over 15,996,000 pairs)
-# and N = 1000 (parity 18,763 + 25,880 + 2 x 3,235, parity_gpu 24,765 + 7,915
-# + 2 x 38,040 over 999,000).  All three evaluate in float-float on the binary32
+# at N = 4000 (precision: 7,878 + 2,709 + 2 x 13,960 over 15,996,000 pairs)
+# and N = 1000 (parity 18,763 + 25,880 + 2 x 3,235, parity_gpu 24,615 + 7,765
+# + 2 x 38,190 over 999,000).  All three evaluate in float-float on the binary32
 # pipe; binary64 is left for the values whose certificate fails.
-BVP_FP64_FLOPS_PER_PAIR = {"precision": 228655 / 15996000,
+BVP_FP64_FLOPS_PER_PAIR = {"precision": 38507 / 15996000,
                            "parity": 51113 / 999000,
                            "parity_gpu": 108760 / 999000}
 # ncu smsp__inst_executed.sum of one parity pair-kernel launch at N = 1000
 # (999,000 pairs), per pair; the same for the reference-GPU arithmetic's
 # pair kernel
 BVP_PARITY_WARP_INST_PER_PAIR = 135950305 / 999000
-BVP_REFGPU_WARP_INST_PER_PAIR = 123397391 / 999000
+BVP_REFGPU_WARP_INST_PER_PAIR = 122850043 / 999000
 # The precision kernel is bound by instruction issue, not by one pipe: warp
 # instructions executed per pair on this workload (ncu smsp__inst_executed.sum
 # over one launch of the N = 4000 workload's pair kernel, the one marking the
 # rn superset, / its pairs), and DRAM bytes per launch
 # (dram__bytes_read.sum + dram__bytes_write.sum of the same launch).
-BVP_PRECISION_WARP_INST_PER_PAIR = 251946845 / 15996000
+BVP_PRECISION_WARP_INST_PER_PAIR = 249250717 / 15996000
 # ncu smsp__inst_executed.sum on indoor4000: the edge check (pair-queue
 # kernel) at block size 256, the autotuner's choice there, per edge; the
 # waypoint kernel (thread per edge, block size 128), per waypoint

@@ -20,9 +20,10 @@
 // bisection has its own length.  Stage A takes 32 pairs, one per lane, and runs
 // the steps the derivative and then the difference settle, which are nearly as
 // many for one pair as for another; the pairs' coefficients and brackets then
-// go to a queue in shared memory.  Stage B runs the remaining steps: a lane whose pair is done
-// stores it and takes the queue's next, once kBisectRefill lanes wait for one.
-// Every pair walks the same sequence of finite differences as toptBisection.
+// go to a queue in shared memory.  Stage B runs the remaining steps: a lane whose
+// pair is done stores it and takes the queue's next, once kBisectRefill lanes
+// wait for one.  Every pair walks the same sequence of finite differences as
+// toptBisection.
 //
 // Bound by instruction issue (no DRAM traffic but the results).
 #pragma once
@@ -135,8 +136,8 @@ struct BisectQueue {
 };
 
 // Pairs first .. first + n - 1 of src, by one warp.  Src: load(k, x0, x1) the
-// two states, tmax(k), store(k, topt, cost), kWantCost.  Exact::cost(x0, x1,
-// tau): the reference's cost expression.
+// two states, tmax(k), store(k, topt, cost), kWantCost.  Exact::costs(x0, x1,
+// ta, tb, want_a, want_b, &ca, &cb): the reference's cost expression.
 template <class Exact, int kRefillLanes, class Src>
 __device__ __forceinline__ void bisect_warp(const Src &src, BisectQueue &queue, long long first, int n) {
   const int lane = threadIdx.x & 31;

@@ -153,7 +153,7 @@ struct ParityCost {
 // instruction issue.  N = 4000 (16 M pairs): 6.11 ms with two float-float costs
 // per finite difference, 3.64 ms with the differences' signs from cost_delta
 // where it settles them, 1.87 ms in two stages with their step limits (31 KB of
-// queue a block, 80 registers, 6 blocks an SM).  N = 1000: 136 warp instructions
+// queue a block, 80 registers and 76 bytes spilled, 6 blocks an SM).  N = 1000: 136 warp instructions
 // a pair instead of 396, 20.7 of 32 lanes in use, 78 % of the issue slots.
 __global__ void __launch_bounds__(kBisectThreads, 6) bvp_pairs_parity_persistent(AllPairs src,
                                                                                  int chunk) {

@@ -102,11 +102,11 @@ __global__ void __launch_bounds__(1024) prepare_bracket_kernel(
 }
 
 // All pairs (N = 4000: 0.643 ms with the refinement and the cost in binary64,
-// 44.0 warp instructions a pair; 0.24 ms with precise_min, 15.8 of them; bound
-// by instruction issue, 87 % of the slots), one block per 128 consecutive pairs
-// of a row (row i = blockIdx.y): each pair's cost and time are stored, and each warp stores
-// the ballot of its 32 pairs whose cost's order key is below *key_hi (bit
-// l = pair l of the warp), warp tile (row, column block, warp) in pair
+// 44.0 warp instructions a pair; 0.225-0.235 ms with precise_min, 15.6 of them;
+// bound by instruction issue, 87 % of the slots), one block per 128 consecutive
+// pairs of a row (row i = blockIdx.y): each pair's cost and time are stored, and
+// each warp stores the ballot of its 32 pairs whose cost's order key is below
+// *key_hi (bit l = pair l of the warp), warp tile (row, column block, warp) in pair
 // order.  No thread waits for another.
 constexpr int kPairTile = 128;
 __global__ void __launch_bounds__(kPairTile) bvp_pairs_masked_kernel(

@@ -140,7 +140,7 @@ struct RefGpuCost {
 
 // N = 1000 (1 M pairs): 1.75-2.1 ms with two float-float costs per finite
 // difference and pow for what they do not certify (one wave, its warps held by
-// the pow evaluations), 0.21 ms now.  Four blocks an SM (128 registers, no
+// the pow evaluations), 0.21 ms now.  Four blocks an SM (116 registers, no
 // spills): 1.98 ms at N = 4000, five 2.12, six 2.61.
 __global__ void __launch_bounds__(kBisectThreads, 4) bvp_pairs_refgpu_kernel(AllPairs src, int chunk) {
   __shared__ BisectQueue s_queue[kBisectWarps];

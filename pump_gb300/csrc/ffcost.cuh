@@ -30,8 +30,8 @@ namespace {
 //   - cost_eval's sum: each of its 31 additions (s7's six included) and ~15
 //     products is rounded once (|error| <= 2^-53 of the partial sum or
 //     product; t^3 and t^4 are themselves rounded products), so its error is
-//     at most 2^-52 x 33 x (the sum of the terms' magnitudes), under
-//     0.1 u^2 of that sum (the reference's GPU kernel: 2.1 u^2, see above);
+//     at most 2^-52 x 33 x (the sum of the terms' magnitudes), about
+//     2.1 u^2 of that sum (the reference's GPU kernel: as much, see above);
 //   - sums of n terms by TwoSum, whose errors (each at most u of the running
 //     sum, itself at most the magnitudes' sum) are added in binary32: at most
 //     n (n + 1) / 2 u^2 (with the squares' own low parts, each at most u of

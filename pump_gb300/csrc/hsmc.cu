@@ -248,7 +248,8 @@ __host__ __device__ inline int hsmc_chunks(long long n, long long blocks, bool a
   return (int)(alone || n <= kHsmcDealt * blocks ? blocks : (n + kHsmcDealt - 1) / kHsmcDealt);
 }
 inline unsigned hsmc_blocks(long long n, bool device_count) {
-  if (!device_count && n > (long long)kHsmcDealt * kHsmcPersistBlocks) return (unsigned)((n + kHsmcRun - 1) / kHsmcRun);
+  if (!device_count && n > (long long)kHsmcDealt * kHsmcPersistBlocks)
+    return (unsigned)((n + kHsmcRun - 1) / kHsmcRun);
   return (unsigned)hsmc_chunks(n, kHsmcPersistBlocks, true);
 }
 // Half-spaces of one waypoint tested on each loaded quad of particles, 5 being
@@ -741,6 +742,15 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_kernel(const HsmcParams 
   hsmc_run<Boxes, Q, Epi>(p);
 }
 
+// Out of line: the loop kernel's own state is saved once per chunk, not spilled
+// around the tests (N = 32000, 4096 particles, when every box was tested:
+// the whole query 266 ms inlined, 247 so).
+template <int Q>
+__device__ __noinline__ void hsmc_loop_paths(const HsmcParams &p, unsigned step, int n, unsigned *s_next,
+                                             const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
+  hsmc_chunk_paths<true, Q, true>(p, step, n, s_next, s_obs, hs, hcnt, klist);
+}
+
 // The search loop on the device, for every query of a group: the chunks of
 // the active queries' wavefronts in query order are the blocks' work items,
 // taken in turn (grid-stride).  A block stages a query's parameters (the
@@ -748,15 +758,6 @@ __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_kernel(const HsmcParams 
 // when its next chunk belongs to another query.  The shared memory holds the
 // layout of the group's largest box count, waypoint count and half-space
 // count.
-// Out of line: the loop kernel's own state is saved once per chunk, not spilled
-// around the tests (N = 32000, 4096 particles: the whole query 266 ms inlined,
-// 247 so).
-template <int Q>
-__device__ __noinline__ void hsmc_loop_paths(const HsmcParams &p, unsigned step, int n, unsigned *s_next,
-                                             const float *s_obs, float4 *hs, uint8_t *hcnt, int *klist) {
-  hsmc_chunk_paths<true, Q, true>(p, step, n, s_next, s_obs, hs, hcnt, klist);
-}
-
 template <int Q>
 __global__ void __launch_bounds__(kHsmcThreads, 8) hsmc_loop_kernel(const LoopGroup *g) {
   extern __shared__ float4 s_dyn4[];

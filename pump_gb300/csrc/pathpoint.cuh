@@ -71,10 +71,10 @@ __device__ __noinline__ float path_state_now(int d, float t, float tau, float p0
 // 3 u^2 and by a float-float one 6 u^2, so r, r^2 and r^3 to 10, 26 and 42 u^2,
 // the edge's sums to 9 u^2 and the terms to at most 54 u^2; a sum of n terms
 // (their high parts by TwoSum, the errors and unnormalised low parts in
-// binary32) adds at most 30 u^2: at most 84 u^2 M = 2^-41.6 M.  When the interval of half-width
-// 2^-41 M around the float-float value lies inside the binary32 rounding cell
-// of its high part, that is the expression's (float) conversion; otherwise (or
-// for tau outside [2^-20, 2^20], values outside [2^-40, 2^60] and non-finite
+// binary32) adds at most 30 u^2: at most 84 u^2 M = 2^-41.6 M.  When the interval
+// of half-width 2^-41 M around the float-float value lies inside the binary32
+// rounding cell of its high part, that is the expression's (float) conversion;
+// otherwise (or for tau outside [2^-20, 2^20], values outside [2^-40, 2^60] and non-finite
 // values) path_state64 gives it.  The per-edge terms (path_ff_edge) are shared
 // by the edge's waypoints.
 //
@@ -239,8 +239,8 @@ __device__ __forceinline__ void path_point_fast(float t, float tau, const float 
   }
 }
 
-// The waypoint and dense-path kernels' queue of states left for binary64, shared by a block:
-// (thread, waypoint, axis) entries in one list per kind, so that a warp then
+// The waypoint and dense-path kernels' queue of states left for binary64, shared
+// by a block: (thread, waypoint, axis) entries in one list per kind, so that a warp then
 // evaluates 32 of one kind at once (binary64 instructions occupy this GPU's
 // binary64 pipe for the same time for one lane as for 32; one state in about
 // 200 is left, and evaluating each lane's own as they came took most of the
