@@ -212,7 +212,7 @@ __global__ void position_variance_kernel(int T, double *__restrict__ var) {
 // shared memory, with the same operations (halfspace_of_box), into its own
 // shared-memory slots.  It first drops the boxes that no waypoint of the
 // edge can bring within the distance gate (gate_keeps_box on the waypoints'
-// bounding box; none dropped when a waypoint is NaN or more than
+// bounding box; none dropped when a waypoint is not finite or more than
 // kHsmcFilterObs boxes are left: 10^6 paths near 200 boxes 6.8 ms where more boxes
 // than the list holds were never filtered, 1.9 so), then per waypoint takes the
 // remaining boxes 32 at a
@@ -367,19 +367,21 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
     const int mi = lane < W ? lane : 0;
 #pragma unroll
     for (int d = 0; d < kDim; ++d) my[d] = __ldg(&ew[mi * kDim + d]);
-    // the edge's waypoints bound the boxes worth testing
+    // the edge's waypoints bound the boxes worth testing, if they are finite (an
+    // infinite one's distance to an infinite box is not a number, which passes
+    // the gate)
     float mn[3], mx[3];
-    bool nan = false;
+    bool odd = false;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       mn[d] = mx[d] = my[d];
-      nan = nan || my[d] != my[d];
+      odd = odd || !(fabsf(my[d]) < INFINITY);
     }
     for (int i = lane + 32; i < W; i += 32)
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         const float x = __ldg(&ew[i * kDim + d]);
-        nan = nan || x != x;
+        odd = odd || !(fabsf(x) < INFINITY);
         mn[d] = fminf(mn[d], x);
         mx[d] = fmaxf(mx[d], x);
       }
@@ -388,8 +390,8 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
       mn[d] = warp_min_f32(mn[d]);
       mx[d] = warp_max_f32(mx[d]);
     }
-    nan = __any_sync(0xffffffffu, nan);
-    bool filt = !nan;
+    odd = __any_sync(0xffffffffu, odd);
+    bool filt = !odd;
     int nk = 0;
     for (int o0 = 0; o0 < p.numObs && filt; o0 += 32) {
       const int o = o0 + lane;

@@ -953,6 +953,49 @@ def test_hsmc_many_boxes(boxes, spread, gpu, pumplib, oracle, roadmap1000):
     assert 0 < want[base:].mean() < vb[:base].mean()
 
 
+@pytest.mark.parametrize("boxes", [40, 128, 129, 200])
+def test_hsmc_infinite_boxes_and_waypoints(boxes, gpu, pumplib, oracle, roadmap1000):
+    """Boxes with infinite and NaN corners and edges with infinite and NaN
+    waypoints: the half-spaces derived in the kernel are the reference's, whose
+    distance between an infinite waypoint and an infinite box is not a number."""
+    torch, _ = gpu
+    from pump_gb300 import workloads
+    L = pumplib.load()
+    r = roadmap1000
+    rng = np.random.default_rng(boxes)
+    obs = workloads.large_boxes(3, boxes).copy()
+    obs[1, 2], obs[2, 7], obs[3, 6], obs[4, 0] = -np.inf, np.inf, np.inf, -np.inf
+    obs[5, 1], obs[6, 8] = np.nan, np.nan
+    E, W, maxHS, T, base, P, om = 64, 9, 6, 400, 20, 96, np.float32(0.3)
+    disc = r["disc"].reshape(-1, W, 6)[:E].copy()
+    disc[3, 1, 0], disc[5, 0, 1], disc[7, 8, 2], disc[9, 4, 1] = np.nan, np.inf, -np.inf, -np.inf
+    disc[11, 2, :3] = np.inf
+    maxd2 = np.float32(0.1 * 0.3 * 0.3)
+    a, b, _ = oracle.cache_halfspaces(disc, np.ones(E, np.uint8), obs, maxHS, maxd2)
+    tm, _ = oracle.particle_tables(0x1234, P, T, pmajor=False)
+    n_new = 4 * E
+    edges = np.tile(np.arange(E, dtype=np.int32), 4)
+    prev = rng.integers(0, base, n_new).astype(np.int32)
+    times = np.zeros(base + n_new, np.float32)
+    times[:base] = rng.uniform(0, 6, base).astype(np.float32)
+    vb = np.zeros((base + n_new, P), np.uint8)
+    vb[:base] = rng.random((base, P)) < 0.9
+    want, cp_o = vb.copy(), np.zeros(base + n_new, np.float32)
+    te = r["te"][:E].copy()
+    oracle.lib().orc_hsmc_propagate(n_new, W, edges, prev, base, a, b, times, te, 0.05, maxHS,
+                                    tm.reshape(-1), om, P, want, P, cp_o)
+    d = [dev(torch, x) for x in (edges, prev, obs, disc, times, te, tm)]
+    d_valid = dev(torch, np.packbits(vb, axis=1, bitorder="little").view(np.uint32))
+    d_cp, d_err = empty(torch, base + n_new, torch.float32), dev(torch, np.zeros(1, np.int32))
+    pumplib.check(L.pump_hsmc_propagate_boxes(
+        n_new, W, ptr(d[0]), ptr(d[1]), E, base, ptr(d[2]), boxes, ptr(d[3]), float(maxd2), maxHS, ptr(d[4]),
+        ptr(d[5]), 0.05, ptr(d[6]), P, T, float(om), ptr(d_valid), P, ptr(d_cp), ptr(d_err), stream(torch)))
+    torch.cuda.synchronize()
+    got = bits_to_bytes(host(d_valid).reshape(base + n_new, P // 32), P)
+    assert np.array_equal(got[base:], want[base:])
+    assert same_bits(host(d_cp)[base:base + n_new], cp_o[base:]) and int(host(d_err)[0]) == 0
+
+
 def test_hsmc_device_checks(gpu, pumplib, oracle, roadmap1000):
     """HSMC's device-side checks: an edge index outside [0, E) and a parent
     outside [0, base) skip their paths and record PUMP_ERR_BAD_INPUT; a time
