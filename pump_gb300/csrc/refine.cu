@@ -290,6 +290,25 @@ __global__ void __launch_bounds__(kRefThreads, Grad ? 3 : 4) refine_kernel(pump_
           Tb_acc += Tb;
         }
       }
+      // with no box the bound's derivative is zero, but a state, time or noise
+      // scale that is not finite shows in its products all the same, as it does
+      // beside a far box
+      if (Grad && nobs == 0 && my_slot == 0) {
+        any = true;
+        const float Tb = 0.0f * om * om * 0.5f * invS * dVdT, gr = 0.0f * (B.g0 * rt);
+        float tb = s * Tb;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          acc[d] += gr;
+          acc[6 + d] -= gr;
+          acc[3 + d] += 0.0f * t;
+          acc[9 + d] += 0.0f * t;
+          tb += (B.h2 * x0[3 + d] + B.h3 * x1[3 + d]) * 0.0f;
+          tb -= B.g0 * (x0[d] - x1[d]) * rt * rt * 0.0f;
+        }
+        tb_acc += tb;
+        Tb_acc += Tb;
+      }
     }
     __syncwarp();
     if (Grad) {

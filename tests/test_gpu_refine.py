@@ -147,6 +147,28 @@ def test_weight_that_is_not_finite(gpu, pumplib, oracle, weight, boxes):
         assert np.array_equal(case.path(k, g.reshape(-1, 6)), case.path(k, g0.reshape(-1, 6)))
 
 
+@pytest.mark.parametrize("at,value", [((1, 0), np.nan), ((2, 4), np.inf), ((3, 5), np.nan)])
+def test_states_that_are_not_finite_without_boxes(gpu, pumplib, oracle, at, value):
+    """Without boxes the bound's derivative is zero, but a node that is not
+    finite leaves no entry of its own and its neighbours' gradients finite (the
+    zero's products with its segments' times and states are not numbers), and
+    every other node's as it is."""
+    torch, _ = gpu
+    case = Case(torch, pumplib, oracle, 3, 9, 2e-3)
+    case.args.num_obstacles = 0
+    g0, _ = bwd(torch, pumplib, case)
+    bad = case.nodes.copy()
+    node = case.offs[1] + at[0]
+    bad[node, at[1]] = value
+    case.keep[0].copy_(torch.from_numpy(bad))
+    g, J = bwd(torch, pumplib, case)
+    assert not np.isfinite(J[1]) and np.isfinite(J[[0, 2]]).all()
+    rows = np.arange(max(node - 1, case.offs[1] + 1), node + 2)
+    assert not np.isfinite(g[rows]).any()
+    others = np.setdiff1d(np.arange(len(g)), rows)
+    assert np.array_equal(g[others], g0[others])
+
+
 def test_clamped_segments(gpu, pumplib, oracle):
     torch, _ = gpu
     case = Case(torch, pumplib, oracle, 16, 7, 0.3, tmax=0.3, n_range=(5, 8))
