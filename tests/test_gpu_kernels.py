@@ -127,17 +127,6 @@ def bvp_pairs_time(torch, pumplib, s, mode, runs=6):
     return best
 
 
-def test_bvp_pairs_refgpu_equal_states_time(gpu, pumplib):
-    """Equal states: bisections down to times that only the reference's
-    expression covers, whose powers of the coordinates both sides of a finite
-    difference share (15.4 ms when they did not, 10.1 so)."""
-    torch, _ = gpu
-    rng = np.random.default_rng(11)
-    s = np.concatenate([rng.uniform(0, 1, (1000, 3)), rng.uniform(-1, 1, (1000, 3))], 1)
-    s = s[rng.integers(0, 40, 1000)].astype(np.float32)
-    assert bvp_pairs_time(torch, pumplib, s, pumplib.PUMP_BVP_PARITY_GPU) < 13.0
-
-
 def test_bvp_batch_parity(gpu, pumplib, oracle):
     torch, _ = gpu
     L = pumplib.load()
@@ -1181,37 +1170,6 @@ def test_mc_cp_box_filter(Pmc, boxes, n_paths, gpu, pumplib, oracle):
         for k, x in enumerate(paths):
             h = oracle.mccp(x, len(x), pm, om, obs)[0] if len(x) <= T else 0
             assert int(host(hits)[k]) == h, (k, len(x))
-
-
-def test_mc_cp_time_between_rules(gpu, pumplib, oracle):
-    """Twice the particles of a call that fits the GPU once with one particle per
-    lane: four per lane, so that it still fits (1.4 times as long with one, 1.1
-    so)."""
-    from pump_gb300 import workloads
-    torch, _ = gpu
-    L = pumplib.load()
-    T, n = 80, 8
-    rng = np.random.default_rng(5)
-    a, b = rng.uniform(0, 1, (n, 1, 3)), rng.uniform(0, 1, (n, 1, 3))
-    x = np.zeros((n, T, 6), np.float32)
-    x[:, :, :3] = a + (b - a) * np.linspace(0, 1, T)[None, :, None]
-    d_x, d_o, d_l = dev(torch, x), dev(torch, np.arange(n, dtype=np.int32) * T), dev(torch, np.full(n, T, np.int32))
-    d_obs = dev(torch, workloads.random_boxes(10, 5))
-    hits, cps = empty(torch, n, torch.int32), empty(torch, n, torch.float32)
-    best = {}
-    for P in (2048, 4096):
-        tab = empty(torch, P * T * 3, torch.float32)
-        pumplib.check(L.pump_particle_tables(7, P, T, ptr(tab), None, stream(torch)))
-        for _ in range(12):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            for _ in range(40):
-                pumplib.check(L.pump_mc_cp(ptr(d_x), ptr(d_o), ptr(d_l), n, ptr(tab), P, T, 0.1, ptr(d_obs), 10,
-                                           ptr(hits), ptr(cps), 0, stream(torch)))
-            e1.record()
-            torch.cuda.synchronize()
-            best[P] = min(best.get(P, 1e9), e0.elapsed_time(e1))
-    assert best[4096] < 1.25 * best[2048], best
 
 
 @pytest.mark.parametrize("N,density", [(0, 0.5), (1, 1.0), (4095, 0.3), (4096, 1.0), (100_000, 0.01),
