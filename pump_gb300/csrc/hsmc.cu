@@ -215,11 +215,10 @@ __global__ void position_variance_kernel(int T, double *__restrict__ var) {
 // bounding box; none dropped when a waypoint is not finite or more than
 // kHsmcFilterObs boxes are left: 10^6 paths near 200 boxes 6.8 ms where more boxes
 // than the list holds were never filtered, 1.9 so), then per waypoint takes the
-// remaining boxes 32 at a
-// time, one per lane: the lanes whose box passes the gate are ranked by a
-// ballot and the first maxHS - stored of them, in index order, fill the next
-// slots, which are the slots cacheHalfspaces fills.  Only the edges a
-// wavefront propagates along get half-spaces, and no cache is written.
+// remaining boxes 32 at a time, one per lane: the lanes whose box passes the gate
+// are ranked by a ballot and the first maxHS - stored of them, in index order,
+// fill the next slots, which are the slots cacheHalfspaces fills.  Only the edges
+// a wavefront propagates along get half-spaces, and no cache is written.
 constexpr int kMaxHsmcWords = 128;   // P <= 4096 particles
 constexpr int kMaxHsSlots = 256;     // W * maxHS <= 256
 constexpr int kHsmcThreads = 128;
@@ -259,7 +258,6 @@ inline unsigned hsmc_blocks(long long n, bool device_count) {
 // twice as long).
 constexpr int kHsmcGroup = 5;
 constexpr int kHsmcFilterObs = 128;
-
 
 // Shared memory of the boxes variant: the staged boxes, then per warp its
 // half-space slots (a0, a1, a2, b), stored counts per waypoint and the list
@@ -537,7 +535,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
           if (q == k) bq = bits[k];
         if (bq == 0u) continue;  // this lane's particles of the group are all dead
         const int end = P - q * 1024 < 1024 ? P - q * 1024 : 1024;
-        auto judge = [&](int c, const float (&o)[4][3]) {
+        auto test_quad = [&](int c, const float (&o)[4][3]) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             bool pass = true;
@@ -557,7 +555,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
 #pragma unroll 1
           for (int c = 0; c * 128 < end; ++c) {
             load(q * 1024 + (c + 1) * 128, next);
-            judge(c, o);
+            test_quad(c, o);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
@@ -567,7 +565,7 @@ __device__ __forceinline__ void hsmc_path(const HsmcParams &p, int w, int edge, 
 #pragma unroll 1
           for (int c = 0; c * 128 < end; ++c) {
             load(q * 1024 + c * 128, o);
-            judge(c, o);
+            test_quad(c, o);
           }
         }
 #pragma unroll
